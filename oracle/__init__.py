@@ -40,7 +40,7 @@ def reference_tree() -> str:
 def build(ref: bool = True) -> None:
     """Compile liboracle.so and, where the reference tree exists, _ref/."""
     subprocess.run(["make", "-s", "-C", _HERE], check=True)
-    if ref and os.path.isdir(reference_tree()):
+    if ref and os.path.isdir(os.path.join(reference_tree(), "src")):
         subprocess.run(["make", "-s", "-C", _HERE, "ref", "REF=" + reference_tree()], check=True)
         subprocess.run(["make", "-s", "-C", _HERE, "examples", "REF=" + reference_tree()], check=True)
 
