@@ -1176,7 +1176,7 @@ int imr_engine_step(imr_engine *E)
     // column init of the newly admitted jobs, then one cycle of every active job
     const WorkList *L = E->d_lists;
     for (auto &g : E->init_groups) {
-        g.ck.init<<<loop_grid(E, (int)g.items.size()), g.ck.threads, g.ck.smem ? g.ck.smem : g.smem, E->s>>>(
+        g.ck.init<<<loop_grid(E, (int)g.items.size()), g.ck.threads, g.smem, E->s>>>(
             E->dj, L + g.list_base);
         ++E->launches;
         ++E->host_launches;

@@ -186,6 +186,7 @@ int make_fft_plan(int n, FftPlanDev &p)
     p.n = n;
     p.nrad = (int)rad.size();
     for (size_t i = 0; i < rad.size(); ++i) p.rad[i] = rad[i];
+    fft_group_passes(p);
     p.tw = d;
     return IMR_SUCCESS;
 }
@@ -211,95 +212,6 @@ int gaussian_weights(double sigma, float *w, int cap)
 }
 
 // ---------------------------------------------------------------- dispatch
-// Kernels specialised at compile time for the lengths below; any other
-// supported length runs the runtime-length FFT (N = 0 instantiation).
-template <int N>
-static RowKernels row_set()
-{
-    RowKernels k{};
-    if constexpr (N >= 16 && is_pow2(N)) {
-        k = RowKernels{k_row_hio_r<true, N>, k_row_hio_r<false, N>, k_row_finish_r<N>,
-                       k_fft_rows_r<-1, N>, k_fft_rows_r<+1, N>, rrow_nb(N), rrow_threads(N),
-                       rrow_smem(N), k_row_hio_p<true, N>, k_row_hio_p<false, N>,
-                       prow_smem<true, N>(), prow_smem<false, N>(), 0};
-        k.hio_fix = k_row_hio_r<false, N, true>;
-        k.p_hio_fix = k_row_hio_p<false, N, true>;
-        k.p_finish = k_row_finish_p<N>;
-        k.p_smem_fin = pfin_smem<N>();
-    } else if constexpr (N >= 8 && is_pow2(N)) {
-        k = RowKernels{k_row_hio_r<true, N>, k_row_hio_r<false, N>, k_row_finish_r<N>,
-                       k_fft_rows_r<-1, N>, k_fft_rows_r<+1, N>, rrow_nb(N), rrow_threads(N),
-                       rrow_smem(N), nullptr, nullptr, 0, 0, 0};
-        k.hio_fix = k_row_hio_r<false, N, true>;
-    } else if constexpr (is_3pow2(N)) {   // per-tile kernels + pipelined 12-value register passes
-        k = RowKernels{k_row_hio<true, N>, k_row_hio<false, N>, k_row_finish<N>, k_fft_rows<-1, N>,
-                       k_fft_rows<+1, N>, row_nb(N), row_threads(N), 0, k_row_hio_p<true, N>,
-                       k_row_hio_p<false, N>, prow_smem<true, N>(), prow_smem<false, N>(), 0};
-        k.hio_fix = k_row_hio<false, N, true>;
-        k.p_hio_fix = k_row_hio_p<false, N, true>;
-        k.p_finish = k_row_finish_p<N>;
-        k.p_smem_fin = pfin_smem<N>();
-    } else if constexpr (N < 0 && -N >= 256) {   // Bluestein lengths, 16 values per thread
-        constexpr int M = -N;
-        k = RowKernels{k_row_hio_bs16<true, M>, k_row_hio_bs16<false, M>, k_row_finish_bs16<M>,
-                       k_fft_rows_bs16<-1, M>, k_fft_rows_bs16<+1, M>, bs16_rows(M), bs16_row_threads(M),
-                       bs16_row_smem(M), nullptr, nullptr, 0, 0, M};
-        k.hio_fix = k_row_hio_bs16<false, M, true>;
-    } else if constexpr (N < 0 && -N >= 8) {   // Bluestein lengths: register chirp-z transforms
-        constexpr int M = -N;
-        k = RowKernels{k_row_hio_bs<true, M>, k_row_hio_bs<false, M>, k_row_finish_bs<M>, k_fft_rows_bs<-1, M>,
-                       k_fft_rows_bs<+1, M>, rrow_nb(M), rrow_threads(M), rrow_smem(M), nullptr, nullptr, 0, 0,
-                       M};
-        k.hio_fix = k_row_hio_bs<false, M, true>;
-    } else {
-        k = RowKernels{k_row_hio<true, N>, k_row_hio<false, N>, k_row_finish<N>, k_fft_rows<-1, N>,
-                       k_fft_rows<+1, N>, row_nb(N), row_threads(N), 0, nullptr, nullptr, 0, 0,
-                       N < 0 ? -N : 0};
-        k.hio_fix = k_row_hio<false, N, true>;
-    }
-    return k;
-}
-template <int N>
-static ColKernels col_set()
-{
-    if constexpr (N >= 128 && N <= 4096 && is_pow2(N)) {   // 16 values per thread in the pipelined pass
-        constexpr int T = pcol16_nbt(N);
-        ColKernels k{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
-                     rcol_nb(N), rcol_threads(N), rcol_smem(N), k_col_p16<N, T, false>, pcol16_smem<N, T>(),
-                     pcol_box_rows(N), 0, pcol16_threads(N, T), 0, T, 1};
-        if constexpr (N >= 256) {   // split-precision tensor-core variants
-            k.p_col_tc[0] = k_col_tc<N, T, kPrecBf16x3, 0>;
-            k.p_col_tc[1] = k_col_tc<N, T, kPrecFp16x3, 0>;
-            k.fft_tc[0][0] = k_col_tc<N, T, kPrecBf16x3, 1>;
-            k.fft_tc[0][1] = k_col_tc<N, T, kPrecBf16x3, 2>;
-            k.fft_tc[1][0] = k_col_tc<N, T, kPrecFp16x3, 1>;
-            k.fft_tc[1][1] = k_col_tc<N, T, kPrecFp16x3, 2>;
-            k.p_smem_tc = pcol_tc_smem<N, T>();
-        }
-        if constexpr (T >= 4) k.p_col_split = k_col_p16<N, T, true>;   // half tiles of >= 2 columns (16-byte TMA rows)
-        return k;
-    } else if constexpr (N >= 16 && is_pow2(N))
-        return ColKernels{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
-                          rcol_nb(N), rcol_threads(N), rcol_smem(N), k_col_p<N>, pcol_smem<N>(),
-                          pcol_box_rows(N), pcol_tma_m(N) ? 1 : 0, pcol_threads(N), 0, rcol_nb(N)};
-    else if constexpr (N >= 8 && is_pow2(N))
-        return ColKernels{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
-                          rcol_nb(N), rcol_threads(N), rcol_smem(N), nullptr, 0, 0, 0, 0, 0};
-    else if constexpr (is_3pow2(N))
-        return ColKernels{k_col<N>, k_col_init<N>, k_fft_cols<-1, N>, k_fft_cols<+1, N>, col_nb(N),
-                          col_threads(N), 0, k_col_p<N>, pcol_smem<N>(), pcol_box_rows(N),
-                          pcol_tma_m(N) ? 1 : 0, pcol_threads(N), 0, rcol_nb(N)};
-    else if constexpr (N < 0 && -N >= 256)   // Bluestein lengths, 16 values per thread
-        return ColKernels{k_col_bs16<-N, 0>, k_col_bs16<-N, 1>, k_fft_cols_bs16<-1, -N>, k_fft_cols_bs16<+1, -N>,
-                          rcol_nb(-N), bs16_col_threads(-N), bs16_col_smem(-N), nullptr, 0, 0, 0, 0, -N, 0};
-    else if constexpr (N < 0 && -N >= 8)   // Bluestein lengths: register chirp-z transforms
-        return ColKernels{k_col_bs<-N>, k_col_init_bs<-N>, k_fft_cols_bs<-1, -N>, k_fft_cols_bs<+1, -N>,
-                          rcol_nb(-N), rcol_threads(-N), rcol_smem(-N), nullptr, 0, 0, 0, 0, -N, 0};
-    else
-        return ColKernels{k_col<N>, k_col_init<N>, k_fft_cols<-1, N>, k_fft_cols<+1, N>, col_nb(N),
-                          col_threads(N), 0, nullptr, 0, 0, 0, 0, N < 0 ? -N : 0};
-}
-
 // Resident CTAs per SM of a kernel at a launch shape, asked of the occupancy
 // calculator once per (device, kernel, shape): the engine launches hundreds
 // of persistent passes per step.
@@ -400,10 +312,6 @@ bool encode_tensor_map(CUtensorMap *map, const void *base, int W, int H, int ele
     return r == CUDA_SUCCESS;
 }
 
-#define IMR_SIZES(X) X(64) X(128) X(192) X(256) X(384) X(512) X(768) X(1024) X(1536) X(2048) X(3072) X(4096)
-// Bluestein transform lengths M (power of two >= 2n - 1 for n <= 2048)
-#define IMR_BS_SIZES(X) X(-8) X(-16) X(-32) X(-64) X(-128) X(-256) X(-512) X(-1024) X(-2048) X(-4096)
-
 RowKernels row_kernels(int N)
 {
     std::vector<int> rad;
@@ -413,14 +321,19 @@ RowKernels row_kernels(int N)
         IMR_SIZES(ROWCASE)
         IMR_BS_SIZES(ROWCASE)
 #undef ROWCASE
-    default: {
-        RowKernels k = row_set<0>();
-        k.nb = (kRowVpt * kRowThreads) / N;
-        if (k.nb < 1) k.nb = 1;
-        return k;
-    }
+    default: return row_set_mx(N);
     }
 }
+
+// The grouped-pass kernels take as few rows per tile as give every SM three
+// tiles (148 x 3), but at least 512 values (two per thread); the others a fixed
+// number.
+int rows_per_tile(const RowKernels &rk, int W, int H)
+{
+    const int most = std::min(rk.nb, H);
+    return rk.mx ? std::min(most, std::max((H + 443) / 444, (511 + W) / W)) : most;
+}
+int row_tile_smem(const RowKernels &rk, int W, int rpc) { return rk.mx ? mx_row_smem(W, rpc) : rk.smem; }
 
 ColKernels col_kernels(int N)
 {
@@ -431,13 +344,7 @@ ColKernels col_kernels(int N)
         IMR_SIZES(COLCASE)
         IMR_BS_SIZES(COLCASE)
 #undef COLCASE
-    default: {
-        ColKernels k = col_set<0>();
-        k.nb = (kColVpt * kColThreads) / N;
-        if (k.nb > 8) k.nb = 8;
-        if (k.nb < 1) k.nb = 1;
-        return k;
-    }
+    default: return col_set_mx(N);
     }
 }
 
@@ -466,15 +373,15 @@ int ensure_kernel_attributes()
     for (int d : g_attr_done)
         if (d == dev) return IMR_SUCCESS;
     cudaError_t e = cudaDeviceGetAttribute(&g_optin_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    std::vector<int> sizes = {0};
+    std::vector<int> sizes = {5, 2000};   // lengths of the grouped-pass kernels of either column width
 #define PUSH(n) sizes.push_back(n);
     IMR_SIZES(PUSH)
 #undef PUSH
     std::vector<RowKernels> rks;
     std::vector<ColKernels> cks;
     for (int n : sizes) {
-        rks.push_back(n ? row_kernels(n) : row_set<0>());
-        cks.push_back(n ? col_kernels(n) : col_set<0>());
+        rks.push_back(row_kernels(n));
+        cks.push_back(col_kernels(n));
     }
 #define PUSHBS(n) rks.push_back(row_set<n>()); cks.push_back(col_set<n>());
     IMR_BS_SIZES(PUSHBS)
@@ -553,9 +460,9 @@ int fft_passes(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr
 {
     const RowKernels rk = row_kernels(W);
     const ColKernels ck = col_kernels(H);
-    const int rpc = rk.nb, cpc = ck.nb;
+    const int rpc = rk.mx ? rows_per_tile(rk, W, H) : rk.nb, cpc = ck.nb;
     const int nrt = (H + rpc - 1) / rpc, nct = (W + cpc - 1) / cpc;
-    const size_t sr = rk.smem ? (size_t)rk.smem : ((size_t)rpc * W + rk.bs_m) * 8;
+    const size_t sr = rk.smem ? (size_t)row_tile_smem(rk, W, rpc) : ((size_t)rpc * W + rk.bs_m) * 8;
     const size_t sc = ck.smem ? (size_t)ck.smem : ((size_t)H + ck.bs_m) * cpc * 8;
     if (sign < 0) {
         if (axes & 1) rk.fft_fwd<<<nrt, rk.threads, sr, s>>>(d, pr, H, rpc);
@@ -667,7 +574,7 @@ int job_prepare(unsigned W, unsigned H, const imr_params &p, JobDev &J, JobShape
     if ((rc = build_weight_table(p, S.wt, S.taps))) return rc;
     S.rk = row_kernels(J.W);
     S.ck = col_kernels(J.H);
-    J.rpc = S.rk.nb < J.H ? S.rk.nb : J.H;
+    J.rpc = rows_per_tile(S.rk, J.W, J.H);
     J.cpc = S.ck.nb < J.W ? S.ck.nb : J.W;
     S.p_rows = S.rk.p_hio != nullptr;
     S.p_cols = S.ck.p_col != nullptr && J.W % 4 == 0 && J.W >= S.ck.p_nb;
@@ -685,7 +592,7 @@ int job_prepare(unsigned W, unsigned H, const imr_params &p, JobDev &J, JobShape
     // shared memory sized for the compile-time tile (NB sequences), even when
     // the image has fewer rows / columns than NB
     if (S.rk.smem) {
-        S.smem_row = S.smem_fin = (size_t)S.rk.smem;   // norms reuse the FFT buffers
+        S.smem_row = S.smem_fin = (size_t)row_tile_smem(S.rk, J.W, J.rpc);   // norms reuse the FFT buffers
     } else if (S.rk.bs_m) {   // row + Bluestein work area (the norms reuse the work area)
         S.smem_row = S.smem_fin = ((size_t)J.W + S.rk.bs_m) * sizeof(float2);
     } else {

@@ -30,9 +30,6 @@ namespace imr {
 constexpr int kMaxTaps = 63;        // Gaussian kernel taps (half width <= 31)
 constexpr int kTapStride = 64;      // floats per cycle in the weight table
 constexpr int kRowThreads = 256;
-constexpr int kRowVpt = 8;          // complex values per thread per pass (rows, runtime length)
-constexpr int kColThreads = 256;
-constexpr int kColVpt = 8;          // complex values per thread per pass (columns, runtime length)
 constexpr int kVbTileX = 32;
 constexpr int kVbTileY = 128;
 constexpr int kVbThreads = 256;

@@ -43,6 +43,7 @@ struct RowKernels {
     // pipelined once-per-cycle pass (g', out, error sums, row blur) or null
     void (*p_finish)(const JobDev *, const WorkList *, float2 *);
     int p_smem_fin;
+    int mx;        // 1: grouped-pass kernels (kernels_mx.cuh), nb is the most rows of a tile
 };
 // Kernels and launch shape of the column passes for one column length.
 struct ColKernels {
@@ -71,7 +72,22 @@ struct ColKernels {
                                                               // tiles as half tiles (JobDev::tmXh), or null
 };
 RowKernels row_kernels(int N);
+// Rows per tile of the per-tile row kernels on a W x H image, and the dynamic
+// shared memory of such a tile.
+int rows_per_tile(const RowKernels &rk, int W, int H);
+int row_tile_smem(const RowKernels &rk, int W, int rpc);
 ColKernels col_kernels(int N);
+// Lengths with kernels specialised at compile time and Bluestein transform
+// lengths M (power of two >= 2n - 1 for n <= 2048); any other supported length
+// runs the grouped-pass kernels (row_set_mx, col_set_mx).
+#define IMR_SIZES(X) X(64) X(128) X(192) X(256) X(384) X(512) X(768) X(1024) X(1536) X(2048) X(3072) X(4096)
+#define IMR_BS_SIZES(X) X(-8) X(-16) X(-32) X(-64) X(-128) X(-256) X(-512) X(-1024) X(-2048) X(-4096)
+template <int N>
+RowKernels row_set();
+template <int N>
+ColKernels col_set();
+RowKernels row_set_mx(int n);
+ColKernels col_set_mx(int n);
 // Plain 2D transform passes (axes: 1 rows, 2 columns, 3 both).
 int fft_passes(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr, const FftPlanDev &pc,
                cudaStream_t s);

@@ -10,23 +10,34 @@
 //     v[q]  = buf[j + q*n/R] * w^(q*(j mod Ns)),   w = exp(S*2*pi*i/(Ns*R))
 //     v     = DFT_R(v)
 //     buf'[(j/Ns)*Ns*R + (j mod Ns) + q*Ns] = v[q]
-// Each pass runs in place in shared memory: every thread first loads all of
-// its butterflies' inputs into registers, the block synchronises, then every
-// thread writes its outputs.  A thread owns at most VPT complex values per pass.
-//
-// Shared-memory layout of a batch of sequences: element e of sequence b lives
-// at b*bs + e*es.  Row tiles use (bs = n, es = 1); column tiles use
-// (bs = 1, es = ncols) so that one row of the tile is contiguous.
+// Each pass of the compile-time schedule (ct_fft) runs in place in shared
+// memory: every thread first loads all of its butterflies' inputs into
+// registers, the block synchronises, then every thread writes its outputs.
+// Lengths without a compile-time kernel run the same schedule in grouped
+// passes (kernels_mx.cuh).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace imr {
 
+// One grouped pass of the schedule (kernels_mx.cuh): radices r1, r2 (r2 = 1:
+// a single radix) at sub-length Ns, L = n/(r1 r2) butterflies per sequence.
+struct FftPass {
+    int r1, r2;
+    int L, Ns;
+    int st1, st2;      // twiddle table steps: n/(Ns r1), n/(Ns r1 r2)
+    unsigned mL, mNs;  // ceil(2^32 / L), ceil(2^32 / Ns): x / d = umulhi(x, m) for x d < 2^32; 0: d = 1
+};
+constexpr int kMaxFftPasses = 8;
+constexpr int kMaxFftRadices = 14;
+
 struct FftPlanDev {
     int n;           // transform length
     int nrad;        // number of radix passes
-    int rad[14];     // radices, first pass first
+    int rad[kMaxFftRadices];   // radices, first pass first
+    int npass;                 // grouped passes
+    FftPass pass[kMaxFftPasses];
     const float2 *tw;  // exp(-2*pi*i*t/L), t < L, computed in double on the host; L = n, or bs_m
     // Bluestein (lengths with a prime factor > 7): the length-n DFT runs as a
     // convolution on the power-of-two length bs_m >= 2n - 1
@@ -249,8 +260,9 @@ __device__ __forceinline__ void dft5(float2 *v)
     float2 y0 = cadd(v[0], cadd(t1, t2));
     float2 a1 = make_float2(v[0].x + c1 * t1.x + c2 * t2.x, v[0].y + c1 * t1.y + c2 * t2.y);
     float2 a2 = make_float2(v[0].x + c2 * t1.x + c1 * t2.x, v[0].y + c2 * t1.y + c1 * t2.y);
-    float2 b1 = mul_si<S>(make_float2(s1 * d1.x + s2 * d2.x, s1 * d1.y + s2 * d2.y));
-    float2 b2 = mul_si<S>(make_float2(s2 * d1.x - s1 * d2.x, s2 * d1.y - s1 * d2.y));
+    // which product is fused is pinned: the rounding may not depend on the caller
+    float2 b1 = mul_si<S>(make_float2(__fmaf_rn(s1, d1.x, __fmul_rn(s2, d2.x)), __fmaf_rn(s1, d1.y, __fmul_rn(s2, d2.y))));
+    float2 b2 = mul_si<S>(make_float2(__fmaf_rn(s2, d1.x, -__fmul_rn(s1, d2.x)), __fmaf_rn(s2, d1.y, -__fmul_rn(s1, d2.y))));
     v[0] = y0;
     v[1] = cadd(a1, b1);
     v[4] = csub(a1, b1);
@@ -329,55 +341,6 @@ __device__ __forceinline__ void dftR(float2 *v)
     else dft8<S>(v);
 }
 
-// ---- one Stockham pass, in place in shared memory ---------------------------
-// nb sequences; butterfly u -> (sequence b, index j).  seq_fast: adjacent
-// threads take adjacent sequences (column tiles); otherwise adjacent j (rows).
-template <int R, int S, int VPT>
-__device__ __forceinline__ void stockham_pass(float2 *buf, const FftPlanDev &p, int Ns, int nb,
-                                              int bs, int es, bool seq_fast, int tid, int nthr)
-{
-    constexpr int BPT = (VPT + R - 1) / R;
-    const int n = p.n;
-    const int m = n / R;
-    const int total = nb * m;
-    const int step = n / (Ns * R);
-    float2 v[BPT][R];
-    int dst[BPT];
-#pragma unroll
-    for (int i = 0; i < BPT; ++i) {
-        const int u = tid + i * nthr;
-        dst[i] = -1;
-        if (u < total) {
-            int b, j;
-            if (seq_fast) { b = u % nb; j = u / nb; }
-            else          { j = u % m;  b = u / m; }
-            const int k = j % Ns;
-            const float2 *src = buf + b * bs + j * es;
-#pragma unroll
-            for (int q = 0; q < R; ++q) v[i][q] = src[q * m * es];
-            if (k != 0) {
-#pragma unroll
-                for (int q = 1; q < R; ++q) {
-                    float2 w = __ldg(p.tw + q * k * step);
-                    if (S > 0) w.y = -w.y;
-                    v[i][q] = cmul(v[i][q], w);
-                }
-            }
-            dftR<R, S>(v[i]);
-            dst[i] = b * bs + ((j - k) * R + k) * es;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < BPT; ++i) {
-        if (dst[i] >= 0) {
-#pragma unroll
-            for (int q = 0; q < R; ++q) buf[dst[i] + q * Ns * es] = v[i][q];
-        }
-    }
-    __syncthreads();
-}
-
 // ---- compile-time schedule -------------------------------------------------
 // Radix schedule of length N: 8s first (then 4,4 / 4 / 2 for the remaining
 // power of two), then 3s, 5s, 7s.  Must match factor_len() on the host.
@@ -399,6 +362,55 @@ __host__ __device__ constexpr RadixList radix_list(int N)
     while (m % 7 == 0) { L.r[L.n++] = 7; m /= 7; }
     if (m != 1) L.n = -1;
     return L;
+}
+
+// Group the radices of a plan into the fewest passes of one or two consecutive
+// radices whose pair has a butterfly in kernels_mx.cuh (product <= 16: 24 warps
+// per SM keep their registers), among those the one with the smallest sum of
+// squared products (even passes).
+inline bool fft_pair_grouped(int r1, int r2)
+{
+    switch (r1 * 16 + r2) {
+    case 8 * 16 + 2:
+    case 4 * 16 + 4: case 4 * 16 + 3:
+    case 2 * 16 + 7: case 2 * 16 + 5: case 2 * 16 + 3:
+    case 3 * 16 + 5: case 3 * 16 + 3: return true;
+    default: return false;
+    }
+}
+inline void fft_group_passes(FftPlanDev &p)
+{
+    int best_n[kMaxFftRadices + 1], best_s[kMaxFftRadices + 1], take[kMaxFftRadices + 1];
+    best_n[p.nrad] = best_s[p.nrad] = 0;
+    for (int i = p.nrad - 1; i >= 0; --i) {
+        best_n[i] = best_n[i + 1] + 1;
+        best_s[i] = best_s[i + 1] + p.rad[i] * p.rad[i];
+        take[i] = 1;
+        if (i + 1 < p.nrad && fft_pair_grouped(p.rad[i], p.rad[i + 1])) {
+            const int r = p.rad[i] * p.rad[i + 1], nn = best_n[i + 2] + 1, ns = best_s[i + 2] + r * r;
+            if (nn < best_n[i] || (nn == best_n[i] && ns < best_s[i])) {
+                best_n[i] = nn;
+                best_s[i] = ns;
+                take[i] = 2;
+            }
+        }
+    }
+    auto magic = [](int d) { return d == 1 ? 0u : (unsigned)(((1ull << 32) + (unsigned)d - 1) / (unsigned)d); };
+    p.npass = 0;
+    int Ns = 1;
+    for (int i = 0; i < p.nrad && p.npass < kMaxFftPasses; ++p.npass) {
+        FftPass &q = p.pass[p.npass];
+        q.r1 = p.rad[i];
+        q.r2 = take[i] == 2 ? p.rad[i + 1] : 1;
+        q.L = p.n / (q.r1 * q.r2);
+        q.Ns = Ns;
+        q.st1 = p.n / (Ns * q.r1);
+        q.st2 = p.n / (Ns * q.r1 * q.r2);
+        q.mL = magic(q.L);
+        q.mNs = magic(Ns);
+        Ns *= q.r1 * q.r2;
+        i += take[i];
+    }
 }
 
 // One Stockham pass with every size known at compile time.  NB sequences of
@@ -469,77 +481,6 @@ __device__ __forceinline__ void ct_fft(float2 *buf, int nb, const float2 *__rest
 {
     static_assert(radix_list(N).n > 0, "length must factor into 2, 3, 5, 7");
     ct_passes<N, NB, T, S, SEQ_FAST, 0, 1>(buf, nb, tw);
-}
-
-// ---- Bluestein -------------------------------------------------------------
-// X[k] = c_k * sum_j (x_j c_j) conj(c_{k-j}),  c_j = exp(S*i*pi*j^2/n)
-//      = c_k * IFFT_M( FFT_M(a) * FFT_M(b) )[k],  a_j = x_j c_j (zero padded),
-// b the kernel conj(c_j) wrapped on the M grid; FFT_M(b)/M is precomputed
-// (bspec_f for S = -1, bspec_b for S = +1).  nb sequences: data element
-// (b, j) at b*dbs + j*des, work element (b, j) at the compile-time layout of
-// ct_fft<M, NB, T, ., SEQ_FAST>.  Ends with a barrier.
-template <int M, int NB, int T, int S, bool SEQ_FAST>
-__device__ __forceinline__ void bluestein(float2 *data, int dbs, int des, float2 *work, int nb,
-                                          const FftPlanDev &p)
-{
-    const int n = p.n;
-    constexpr int WBS = SEQ_FAST ? 1 : M;
-    constexpr int WES = SEQ_FAST ? NB : 1;
-    for (int idx = threadIdx.x; idx < NB * M; idx += T) {
-        int b, j;
-        if (SEQ_FAST) { b = idx % NB; j = idx / NB; }
-        else          { j = idx % M;  b = idx / M; }
-        float2 v = make_float2(0.f, 0.f);
-        if (b < nb && j < n) {
-            float2 c = __ldg(p.chirp + j);
-            if (S > 0) c.y = -c.y;
-            v = cmul(data[b * dbs + j * des], c);
-        }
-        work[b * WBS + j * WES] = v;
-    }
-    __syncthreads();
-    ct_fft<M, NB, T, -1, SEQ_FAST>(work, nb, p.tw);
-    const float2 *spec = S < 0 ? p.bspec_f : p.bspec_b;
-    for (int idx = threadIdx.x; idx < NB * M; idx += T) {
-        int b, j;
-        if (SEQ_FAST) { b = idx % NB; j = idx / NB; }
-        else          { j = idx % M;  b = idx / M; }
-        work[b * WBS + j * WES] = cmul(work[b * WBS + j * WES], __ldg(spec + j));
-    }
-    __syncthreads();
-    ct_fft<M, NB, T, +1, SEQ_FAST>(work, nb, p.tw);
-    for (int idx = threadIdx.x; idx < NB * n; idx += T) {
-        int b, j;
-        if (SEQ_FAST) { b = idx % NB; j = idx / NB; }
-        else          { j = idx % n;  b = idx / n; }
-        if (b < nb) {
-            float2 c = __ldg(p.chirp + j);
-            if (S > 0) c.y = -c.y;
-            data[b * dbs + j * des] = cmul(work[b * WBS + j * WES], c);
-        }
-    }
-    __syncthreads();
-}
-
-// Full transform of nb sequences held in shared memory (see layout above).
-// Requires nb * n <= VPT * nthr.  Ends with a __syncthreads().
-template <int S, int VPT>
-__device__ void fft_smem(float2 *buf, const FftPlanDev &p, int nb, int bs, int es, bool seq_fast,
-                         int tid, int nthr)
-{
-    int Ns = 1;
-    for (int i = 0; i < p.nrad; ++i) {
-        const int R = p.rad[i];
-        switch (R) {
-        case 8: stockham_pass<8, S, VPT>(buf, p, Ns, nb, bs, es, seq_fast, tid, nthr); break;
-        case 4: stockham_pass<4, S, VPT>(buf, p, Ns, nb, bs, es, seq_fast, tid, nthr); break;
-        case 2: stockham_pass<2, S, VPT>(buf, p, Ns, nb, bs, es, seq_fast, tid, nthr); break;
-        case 3: stockham_pass<3, S, VPT>(buf, p, Ns, nb, bs, es, seq_fast, tid, nthr); break;
-        case 5: stockham_pass<5, S, VPT>(buf, p, Ns, nb, bs, es, seq_fast, tid, nthr); break;
-        default: stockham_pass<7, S, VPT>(buf, p, Ns, nb, bs, es, seq_fast, tid, nthr); break;
-        }
-        Ns *= R;
-    }
 }
 
 }  // namespace imr

@@ -96,6 +96,7 @@ static bool radices(int n, FftPlanDev &p, const float2 *tw)
     p.n = n;
     p.nrad = L.n;
     for (int i = 0; i < L.n; ++i) p.rad[i] = L.r[i];
+    fft_group_passes(p);
     p.tw = tw;
     return true;
 }
@@ -169,7 +170,7 @@ extern "C" int imr_shrink_wrap_noalloc(const float *d_modulus, float *d_out, uns
     J.H = (int)H;
     const RowKernels rk = row_kernels(J.W);
     const ColKernels ck = col_kernels(J.H);
-    J.rpc = rk.nb < J.H ? rk.nb : J.H;
+    J.rpc = rows_per_tile(rk, J.W, J.H);
     J.cpc = ck.nb < J.W ? ck.nb : J.W;
     const bool p_rows = rk.p_hio != nullptr;
     bool p_cols = ck.p_col != nullptr && J.W % 4 == 0 && J.W >= ck.p_nb;
@@ -263,7 +264,7 @@ extern "C" int imr_shrink_wrap_noalloc(const float *d_modulus, float *d_out, uns
     S.lists[2] = WorkList{nullptr, J.n_vb_tiles};
     size_t smem_row, smem_fin;
     if (rk.smem) {
-        smem_row = smem_fin = (size_t)rk.smem;
+        smem_row = smem_fin = (size_t)row_tile_smem(rk, J.W, J.rpc);
     } else {
         smem_row = (size_t)rk.nb * J.W * sizeof(float2);
         smem_fin = smem_row + (size_t)rk.nb * J.W * sizeof(float);

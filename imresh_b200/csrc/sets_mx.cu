@@ -1,0 +1,27 @@
+// Grouped-pass kernels of the lengths without a compile-time kernel.
+#include "kernel_sets.cuh"
+
+namespace imr {
+
+RowKernels row_set_mx(int n)
+{
+    RowKernels k{k_row_hio_mx<true, false>, k_row_hio_mx<false, false>, k_row_finish_mx<0>, k_fft_rows_mx<-1>,
+                 k_fft_rows_mx<+1>, std::max(1, kMxRowElems / n), kMxRowThreads, 0, nullptr, nullptr, 0, 0, 0};
+    k.smem = mx_row_smem(n, k.nb);
+    k.hio_fix = k_row_hio_mx<false, true>;
+    k.mx = 1;
+    return k;
+}
+template <int T>
+static ColKernels col_set_mx_t(int n)
+{
+    return ColKernels{k_col_mx<0, T>, k_col_mx<1, T>, k_fft_cols_mx<-1, T>, k_fft_cols_mx<+1, T>, kMxColW, T,
+                      mx_col_smem(n), nullptr, 0, 0, 0, 0, 0, 0};
+}
+ColKernels col_set_mx(int n)
+{
+    return mx_col_threads(n) == 256 ? col_set_mx_t<256>(n) : col_set_mx_t<512>(n);
+}
+
+
+}  // namespace imr
