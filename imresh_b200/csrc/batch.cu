@@ -292,8 +292,8 @@ static int grow(imr_engine *E, size_t n_items, size_t n_lists)
     return IMR_SUCCESS;
 }
 
-// Loop-kernel grid: enough CTAs to fill the GPU, never more than the items.
-static int loop_grid(const imr_engine *E, int items) { return std::max(1, std::min(items, E->sms * 16)); }
+// Per-tile kernels: one CTA per item (some of them take one item only).
+static int item_grid(int items) { return std::max(1, items); }
 
 static void finish_now(imr_engine *E, EJob *j, int status)
 {
@@ -487,13 +487,13 @@ static int launch_cycle(imr_engine *E, cudaStream_t s, const WorkList *L, std::v
                                     E->grid_pct)))
                 return rc;
         } else {
-            g.rk.finish<<<loop_grid(E, (int)g.items.size()), g.rk.threads, g.smem_fin, s>>>(E->dj, L + g.list_base,
+            g.rk.finish<<<item_grid((int)g.items.size()), g.rk.threads, g.smem_fin, s>>>(E->dj, L + g.list_base,
                                                                                          nullptr);
         }
         ++k;
     }
     if (n_vb) {
-        k_vblur<<<loop_grid(E, (int)n_vb), kVbThreads, 0, s>>>(E->dj, L + vb_base);
+        k_vblur<<<item_grid((int)n_vb), kVbThreads, 0, s>>>(E->dj, L + vb_base);
         ++k;
     }
     int max_hio = 0;
@@ -509,7 +509,7 @@ static int launch_cycle(imr_engine *E, cudaStream_t s, const WorkList *L, std::v
                 kf<<<scaled_grid((const void *)kf, g.rk.threads, sm, n, E->grid_pct), g.rk.threads, sm, s>>>(E->dj,
                                                                                                           Li);
             } else {
-                (i == 0 ? g.rk.hio_first : g.rk.hio)<<<loop_grid(E, n), g.rk.threads, g.smem, s>>>(E->dj, Li);
+                (i == 0 ? g.rk.hio_first : g.rk.hio)<<<item_grid(n), g.rk.threads, g.smem, s>>>(E->dj, Li);
             }
             ++k;
         }
@@ -521,7 +521,7 @@ static int launch_cycle(imr_engine *E, cudaStream_t s, const WorkList *L, std::v
                 g.ck.p_col<<<scaled_grid((const void *)g.ck.p_col, g.ck.p_threads, g.ck.p_smem, n, E->grid_pct),
                              g.ck.p_threads, g.ck.p_smem, s>>>(E->dj, Li);
             else
-                g.ck.col<<<loop_grid(E, n), g.ck.threads, g.smem, s>>>(E->dj, Li);
+                g.ck.col<<<item_grid(n), g.ck.threads, g.smem, s>>>(E->dj, Li);
             ++k;
         }
     }
@@ -1176,7 +1176,7 @@ int imr_engine_step(imr_engine *E)
     // column init of the newly admitted jobs, then one cycle of every active job
     const WorkList *L = E->d_lists;
     for (auto &g : E->init_groups) {
-        g.ck.init<<<loop_grid(E, (int)g.items.size()), g.ck.threads, g.smem, E->s>>>(
+        g.ck.init<<<item_grid((int)g.items.size()), g.ck.threads, g.smem, E->s>>>(
             E->dj, L + g.list_base);
         ++E->launches;
         ++E->host_launches;

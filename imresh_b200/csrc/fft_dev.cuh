@@ -136,7 +136,8 @@ __device__ __forceinline__ void dft8(float2 *v)
 
 // 16 points as 4 x 4: DFT4 over n1 of x[4 n1 + n2], twiddle W16^(n2 k1),
 // DFT4 over n2; output k1 + 4 k2.
-template <int S>
+// HALF: v[8..15] are zero and not read; x + 0 and x - 0 are x.
+template <int S, bool HALF = false>
 __device__ __forceinline__ void dft16(float2 *v)
 {
     const float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f;   // cos, sin(pi/8)
@@ -144,8 +145,15 @@ __device__ __forceinline__ void dft16(float2 *v)
     float2 y[4][4];
 #pragma unroll
     for (int n2 = 0; n2 < 4; ++n2) {
-        float2 a[4] = {v[n2], v[4 + n2], v[8 + n2], v[12 + n2]};
-        dft4<S>(a);
+        float2 a[4];
+        if constexpr (HALF) {
+            a[0] = cadd(v[n2], v[4 + n2]);
+            a[2] = csub(v[n2], v[4 + n2]);
+            cadd_sub_si<S>(v[n2], v[4 + n2], a[1], a[3]);
+        } else {
+            a[0] = v[n2], a[1] = v[4 + n2], a[2] = v[8 + n2], a[3] = v[12 + n2];
+            dft4<S>(a);
+        }
 #pragma unroll
         for (int k1 = 0; k1 < 4; ++k1) y[n2][k1] = a[k1];
     }

@@ -404,6 +404,32 @@ struct RegTw16 {
         }
     }
     __device__ __forceinline__ void load(const float2 *__restrict__ tw, int l) { load_pass<0, 1>(tw, l); }
+    // the powers of butterfly i in pass P (sub-length NS, radix R)
+    template <int P, int NS, int R>
+    __device__ __forceinline__ void get(int i, float2 (&p)[4]) const
+    {
+        constexpr int off = tw16_slots_upto(N, P);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) p[e] = w[off + ((N / 16) % NS == 0 ? 0 : i)][e];
+    }
+};
+
+// The same powers read from the table at each use: 20 registers fewer, for
+// kernels whose transforms otherwise spill (four table loads per butterfly,
+// mostly L1 hits).
+template <int N>
+struct LdTw16 {
+    const float2 *tw;
+    int l;
+    template <int P, int NS, int R>
+    __device__ __forceinline__ void get(int i, float2 (&p)[4]) const
+    {
+        constexpr int STEP = N / (NS * R);
+        const int t = ((l + i * (N / 16)) % NS) * STEP;   // t < N/R
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            p[e] = (R >> e) > 1 ? __ldg(tw + (((1 << e) * t) & (N - 1))) : make_float2(1.f, 0.f);
+    }
 };
 
 // u[q] *= w^q, q = 1..R-1, from the table powers p = (w, w^2, w^4, w^8)
@@ -457,8 +483,10 @@ struct RowSwz16 {
     __device__ __forceinline__ static int at(int b, int e) { return b * N + (e ^ ((e >> 4) & 15)); }
 };
 
-template <int N, class LAYOUT, int S, int P, int NS>
-__device__ __forceinline__ void reg16_passes(float2 (&v)[16], float2 *buf, int b, int l, const RegTw16<N> &tw)
+// HALF: v[8..15] are zero on entry (the zero-padded half of a Bluestein
+// transform): the first radix-16 pass skips the operations with them.
+template <int N, class LAYOUT, int S, int P, int NS, bool HALF = false, class TW>
+__device__ __forceinline__ void reg16_passes(float2 (&v)[16], float2 *buf, int b, int l, const TW &tw)
 {
     constexpr RadixList L = reg16_radix_list(N);
     if constexpr (P < L.n) {
@@ -475,10 +503,12 @@ __device__ __forceinline__ void reg16_passes(float2 (&v)[16], float2 *buf, int b
 #pragma unroll
             for (int q = 0; q < R; ++q) u[q] = v[i + q * BPT];
             if constexpr (NS > 1) {
-                constexpr int off = tw16_slots_upto(N, P);
-                twiddle_pow<R, S>(u, tw.w[off + (Q % NS == 0 ? 0 : i)]);
+                float2 p[4];
+                tw.template get<P, NS, R>(i, p);
+                twiddle_pow<R, S>(u, p);
             }
-            dftR<R, S>(u);
+            if constexpr (HALF && P == 0) dft16<S, true>(u);
+            else dftR<R, S>(u);
 #pragma unroll
             for (int q = 0; q < R; ++q) v[i + q * BPT] = u[q];
         }
@@ -494,16 +524,16 @@ __device__ __forceinline__ void reg16_passes(float2 (&v)[16], float2 *buf, int b
             __syncthreads();
 #pragma unroll
             for (int m = 0; m < 16; ++m) v[m] = buf[LAYOUT::at(b, l + m * Q)];
-            reg16_passes<N, LAYOUT, S, P + 1, NS * R>(v, buf, b, l, tw);
+            reg16_passes<N, LAYOUT, S, P + 1, NS * R, false>(v, buf, b, l, tw);
         }
     }
 }
 
-template <int N, class LAYOUT, int S>
-__device__ __forceinline__ void reg16_fft(float2 (&v)[16], float2 *buf, int b, int l, const RegTw16<N> &tw)
+template <int N, class LAYOUT, int S, bool HALF = false, class TW>
+__device__ __forceinline__ void reg16_fft(float2 (&v)[16], float2 *buf, int b, int l, const TW &tw)
 {
     static_assert(is_pow2(N) && N >= 128 && N <= 4096, "16-value FFT length: 2^k, 128..4096");
-    reg16_passes<N, LAYOUT, S, 0, 1>(v, buf, b, l, tw);
+    reg16_passes<N, LAYOUT, S, 0, 1, HALF>(v, buf, b, l, tw);
 }
 
 // ---- half of each 16-value sequence per thread (half tiles) --------------------

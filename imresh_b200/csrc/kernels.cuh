@@ -34,6 +34,16 @@ __device__ __forceinline__ WorkItem item_at(const WorkList *L, int i)
     return WorkItem{0, i};
 }
 
+// A list's header, with the first job's description requested at the same time:
+// a plan's lists (items == nullptr) always mean job 0, and the description is
+// the next thing a block reads, one memory latency (0.3 us) later.
+__device__ __forceinline__ WorkList list_and_job0(const JobDev *jobs, const WorkList *L)
+{
+    if (threadIdx.x < (sizeof(JobDev) + 127) / 128)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char *>(jobs) + 128 * threadIdx.x));
+    return *L;
+}
+
 // Kernel wrapper: the CTAs stride over the list's items, so one launch with a
 // fixed grid serves any number of items (the count lives in device memory and
 // may change between replays of a captured graph).
@@ -1338,42 +1348,60 @@ __global__ void __launch_bounds__(rcol_threads(M)) k_fft_cols_bs(float2 *data, F
 // The same chain as reg_bluestein on the 16-value register FFT: two
 // exchanges per length-M transform up to M = 4096 instead of three, and
 // twiddle powers in registers (loaded once per CTA; every job of a launch has
-// the same work length).  Rows: 4096/M rows per CTA (256 threads); column
-// tiles: rcol_nb(M) columns (512 threads for M >= 512).
-__host__ __device__ constexpr int bs16_rows(int M) { return M >= 4096 ? 1 : 4096 / M; }
+// the same work length).  n <= M/2, so a thread's values m >= 8 are the zero
+// padding: they are neither loaded, updated nor stored, the first radix-16 pass
+// skips the operations with them, and the last pass does not form them.
+//
+// Tiles are small -- one row of M = 2048 on 128 threads, two columns on 256 --
+// because what bounds these passes is how evenly a few hundred to a thousand
+// sequences fill 148 SMs: two rows per 256-thread CTA at two CTAs per SM ran
+// the 733 rows of a 1021 x 733 image as 367 CTAs in 296 places.  All of a tile's
+// operands (X, g_prev, mask, modulus) are requested before its first transform.
+__host__ __device__ constexpr int bs16_rows(int M) { return M >= 2048 ? 1 : 2048 / M; }
 __host__ __device__ constexpr int bs16_row_threads(int M) { return bs16_rows(M) * M / 16; }
-__host__ __device__ constexpr int bs16_row_smem(int M) { return bs16_rows(M) * M * 8; }
-__host__ __device__ constexpr int bs16_col_threads(int M) { return rcol_nb(M) * M / 16; }
-__host__ __device__ constexpr int bs16_col_smem(int M) { return rcol_nb(M) * M * 8; }
+// exchange buffer | g_prev of the rows
+__host__ __device__ constexpr int bs16_row_smem(int M) { return bs16_rows(M) * (M + M / 2) * 8; }
+__host__ __device__ constexpr int bs16_col_nb(int M) { return M >= 4096 ? 2 : (4096 / M > 16 ? 16 : 4096 / M); }
+__host__ __device__ constexpr int bs16_col_threads(int M) { return bs16_col_nb(M) * M / 16; }
+// exchange buffer | modulus of the columns
+__host__ __device__ constexpr int bs16_col_smem(int M) { return bs16_col_nb(M) * (M * 8 + M / 2 * 4); }
+// 16 warps per SM at 128 registers, no spills; 20 and 24 warps (96, 80 registers,
+// 180-480 bytes of spills) measured 0-10 % slower.
+__host__ __device__ constexpr int bs16_min_blocks(int threads) { return threads <= 512 ? 512 / threads : 1; }
 
+// The length-n transform of v (positions l + m*M/16, m < 8; the others are
+// ignored and left undefined); spec: the kernel spectrum of the direction S.
 template <int M, class LAYOUT, int S>
-__device__ __forceinline__ void reg16_bluestein(float2 (&v)[16], float2 *sm, int b, int l, const RegTw16<M> &tw,
-                                                const FftPlanDev &p)
+__device__ __forceinline__ void reg16_bluestein(float2 (&v)[16], float2 *sm, int b, int l, const LdTw16<M> &tw, int n,
+                                                const float2 *chirp, const float2 *spec)
 {
     constexpr int Q = M / 16;
-    const int n = p.n;
+    // opaque per transform: otherwise the chirp values and the 64 exchange
+    // addresses that the four transforms of a pass share are kept for all of
+    // them, and spilled
+    asm volatile("" : "+r"(l), "+l"(chirp), "+r"(n));
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
+    for (int m = 0; m < 8; ++m) {
         const int j = l + m * Q;
         if (j < n) {
-            float2 c = __ldg(p.chirp + j);
+            float2 c = __ldg(chirp + j);
             if (S > 0) c.y = -c.y;
             v[m] = cmul(v[m], c);
         } else {
             v[m] = make_float2(0.f, 0.f);
         }
     }
-    reg16_fft<M, LAYOUT, -1>(v, sm, b, l, tw);
-    const float2 *spec = S < 0 ? p.bspec_f : p.bspec_b;
+    reg16_fft<M, LAYOUT, -1, true>(v, sm, b, l, LdTw16<M>{tw.tw, l});
 #pragma unroll
     for (int m = 0; m < 16; ++m) v[m] = cmul(v[m], __ldg(spec + l + m * Q));
-    reg16_fft<M, LAYOUT, +1>(v, sm, b, l, tw);
-    __syncthreads();   // the last exchange's reads are done before the buffer is written again
+    asm volatile("" : "+r"(l));
+    reg16_fft<M, LAYOUT, +1>(v, sm, b, l, LdTw16<M>{tw.tw, l});
+    asm volatile("" : "+r"(l), "+l"(chirp), "+r"(n));
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
+    for (int m = 0; m < 8; ++m) {
         const int j = l + m * Q;
         if (j < n) {
-            float2 c = __ldg(p.chirp + j);
+            float2 c = __ldg(chirp + j);
             if (S > 0) c.y = -c.y;
             v[m] = cmul(v[m], c);
         }
@@ -1381,179 +1409,233 @@ __device__ __forceinline__ void reg16_bluestein(float2 (&v)[16], float2 *sm, int
 }
 
 template <bool FIRST, int M, bool FIX = false>
-__global__ void __launch_bounds__(bs16_row_threads(M), 2) k_row_hio_bs16(const JobDev *jobs, const WorkList *L)
+__global__ void __launch_bounds__(bs16_row_threads(M), bs16_min_blocks(bs16_row_threads(M)))
+k_row_hio_bs16(const JobDev *jobs, const WorkList *L)
 {
     extern __shared__ float4 smem4[];
-    float2 *sm = reinterpret_cast<float2 *>(smem4);
-    constexpr int Q = M / 16, T = bs16_row_threads(M);
+    float2 *const sm = reinterpret_cast<float2 *>(smem4);
+    constexpr int Q = M / 16, T = bs16_row_threads(M), H8 = 8;
+    const WorkList list = list_and_job0(jobs, L);
+    if ((int)blockIdx.x >= list.n) return;
     const int b = threadIdx.x / Q, l = threadIdx.x % Q;
-    const int n_items = L->n;
-    if ((int)blockIdx.x >= n_items) return;
-    RegTw16<M> rtw;
-    rtw.load(jobs[item_at(L, blockIdx.x).job].prow.tw, l);
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-        const WorkItem wi = item_at(L, it);
-        const JobDev &J = jobs[wi.job];
-        JobState *st = J.st;
-        if (st->stop) continue;
-        const int W = J.W;
-        const int y = wi.tile * J.rpc + b;
-        const bool ok = b < J.rpc && y < J.H;
-        const size_t base = (size_t)y * W;
-        float2 v[16];
+    const WorkItem wi = list.items ? list.items[blockIdx.x] : WorkItem{0, (int)blockIdx.x};
+    const JobDev &J = jobs[wi.job];
+    JobState *const st = J.st;
+    const int W = J.W, y = wi.tile * J.rpc + b;
+    const bool ok = b < J.rpc && y < J.H;
+    float2 *const sg = sm + bs16_rows(M) * M + b * (M / 2);
+    const size_t base = (size_t)y * W;
+    const float2 *const Xi = J.X + base, *const Gi = J.G + base;
+    const uint8_t *const mki = J.mask + base;
+    float2 v[16];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) {
-            const int j = l + m * Q;
-            v[m] = ok && j < W ? J.X[base + j] : make_float2(0.f, 0.f);
-        }
-        reg16_bluestein<M, RowSwz16<M>, +1>(v, sm, b, l, rtw, J.prow);
-        const float beta = J.beta;
-        const float thr = st->thr;
-        const int k = FIX ? st->cycle : 0;
-        const bool init_gprev = FIX ? k == 0 : FIRST && st->hio_cycle == 0;
-        const bool fin = FIX && k >= J.n_cycles;
-        const bool track = FIX && (J.target > 0.f || fin);
-        double tot = 0.0, cnt = 0.0;
-#pragma unroll
-        for (int m = 0; m < 16; ++m) {
-            const int j = l + m * Q;
-            if (!ok || j >= W) continue;
-            const size_t idx = base + j;
-            const float2 gp1 = v[m];
-            uint8_t msk;
-            if (FIRST) {
-                msk = J.vb[idx] < thr ? 1 : 0;
-                J.mask[idx] = msk;
-            } else {
-                msk = J.mask[idx];
-            }
-            if (FIX && track) hio_track(J.out, idx, gp1, msk, tot, cnt);
-            if (fin) continue;
-            const float2 gp = init_gprev ? gp1 : J.G[idx];
-            float2 g;
-            if ((FIX ? msk == 1 : msk != 0) || gp1.x < 0.f)
-                g = make_float2(__fsub_rn(gp.x, __fmul_rn(beta, gp1.x)), __fsub_rn(gp.y, __fmul_rn(beta, gp1.y)));
-            else
-                g = gp1;
-            J.G[idx] = g;
-            v[m] = g;
-        }
-        if (!fin) {
-            reg16_bluestein<M, RowSwz16<M>, -1>(v, sm, b, l, rtw, J.prow);
-            if (ok) {
-#pragma unroll
-                for (int m = 0; m < 16; ++m) {
-                    const int j = l + m * Q;
-                    if (j < W) J.X[base + j] = v[m];
-                }
-            }
-        }
-        if (FIX) hio_tile_done<T>(J, wi.tile, tot, cnt);
-        __syncthreads();
+    for (int m = 0; m < H8; ++m) {
+        const int j = l + m * Q;
+        v[m] = ok && j < W ? Xi[j] : make_float2(0.f, 0.f);
     }
+#pragma unroll
+    for (int m = 0; m < H8; ++m) {   // (g_prev of a first iteration, not yet written, is not used)
+        const int j = l + m * Q;
+        if (ok && j < W) cp_async8(sg + j, Gi + j);
+    }
+    uint32_t mk[2] = {0u, 0u};   // mask bytes of m = 0..3, 4..7
+    if (!FIRST) {
+#pragma unroll
+        for (int m = 0; m < H8; ++m) {
+            const int j = l + m * Q;
+            mk[m / 4] |= (uint32_t)(ok && j < W ? mki[j] : 0) << (8 * (m % 4));
+        }
+    }
+    const int stop = st->stop;
+    const float thr = FIRST ? st->thr : 0.f;
+    const int k = FIX ? st->cycle : FIRST ? st->hio_cycle : 1;
+    const bool init_gprev = k == 0;
+    const bool fin = FIX && k >= J.n_cycles;
+    const bool track = FIX && (J.target > 0.f || fin);
+    if (stop) return;
+    reg16_bluestein<M, RowSwz16<M>, +1>(v, sm, b, l, LdTw16<M>{J.prow.tw, l}, W, J.prow.chirp, J.prow.bspec_b);
+    if (FIRST) {
+        const float *const vb = J.vb + base;
+#pragma unroll
+        for (int m = 0; m < H8; ++m) {
+            const int j = l + m * Q;
+            const uint8_t bit = (ok && j < W ? vb[j] : 0.f) < thr ? 1 : 0;
+            mk[m / 4] |= (uint32_t)bit << (8 * (m % 4));
+            if (ok && j < W) J.mask[base + j] = bit;
+        }
+    }
+    cp_async_wait();   // each thread reads back what it copied
+    float2 *const G = J.G + base;
+    const float beta = J.beta;
+    double tot = 0.0, cnt = 0.0;
+#pragma unroll
+    for (int m = 0; m < H8; ++m) {
+        const int j = l + m * Q;
+        if (!ok || j >= W) continue;
+        const float2 gp1 = v[m];
+        const uint8_t msk = (uint8_t)(mk[m / 4] >> (8 * (m % 4)));
+        if (FIX && track) hio_track(J.out, base + j, gp1, msk, tot, cnt);
+        if (fin) continue;
+        const float2 gp = init_gprev ? gp1 : sg[j];
+        float2 g;
+        if ((FIX ? msk == 1 : msk != 0) || gp1.x < 0.f)
+            g = make_float2(__fsub_rn(gp.x, __fmul_rn(beta, gp1.x)), __fsub_rn(gp.y, __fmul_rn(beta, gp1.y)));
+        else
+            g = gp1;
+        G[j] = g;
+        v[m] = g;
+    }
+    if (!fin) {
+        reg16_bluestein<M, RowSwz16<M>, -1>(v, sm, b, l, LdTw16<M>{J.prow.tw, l}, W, J.prow.chirp, J.prow.bspec_f);
+        if (ok) {
+            float2 *const X = J.X + base;
+#pragma unroll
+            for (int m = 0; m < H8; ++m) {
+                const int j = l + m * Q;
+                if (j < W) X[j] = v[m];
+            }
+        }
+    }
+    if (FIX) hio_tile_done<T>(J, wi.tile, tot, cnt);
 }
 
 template <int M>
-__global__ void __launch_bounds__(bs16_row_threads(M), 2) k_row_finish_bs16(const JobDev *jobs, const WorkList *L,
-                                                                         float2 *dbg_gprime)
+__global__ void __launch_bounds__(bs16_row_threads(M), bs16_min_blocks(bs16_row_threads(M)))
+k_row_finish_bs16(const JobDev *jobs, const WorkList *L, float2 *dbg_gprime)
 {
     extern __shared__ float4 smem4[];
-    float2 *sm = reinterpret_cast<float2 *>(smem4);
-    constexpr int Q = M / 16, T = bs16_row_threads(M);
+    float2 *const sm = reinterpret_cast<float2 *>(smem4);
+    constexpr int Q = M / 16, T = bs16_row_threads(M), H8 = 8;
     __shared__ float wsm[kTapStride];
     __shared__ double red[2 * T / 32 > 2 ? 2 * T / 32 : 2];
+    const WorkList list = list_and_job0(jobs, L);
+    if ((int)blockIdx.x >= list.n) return;
     const int b = threadIdx.x / Q, l = threadIdx.x % Q;
-    const int n_items = L->n;
-    if ((int)blockIdx.x >= n_items) return;
-    RegTw16<M> rtw;
-    rtw.load(jobs[item_at(L, blockIdx.x).job].prow.tw, l);
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-        const WorkItem wi = item_at(L, it);
-        const JobDev &J = jobs[wi.job];
-        JobState *st = J.st;
-        if (st->stop) continue;
-        const int c = st->cycle;
-        if (wi.tile == 0 && threadIdx.x == 0) st->max_bits = 0u;
-        const int W = J.W;
-        const int y = wi.tile * J.rpc + b;
-        const bool ok = b < J.rpc && y < J.H;
-        const size_t base = (size_t)y * W;
-        const int K = J.ntaps[c];
-        if (threadIdx.x < kTapStride) wsm[threadIdx.x] = J.weights[(size_t)c * kTapStride + threadIdx.x];
-        float2 v[16];
+    const WorkItem wi = list.items ? list.items[blockIdx.x] : WorkItem{0, (int)blockIdx.x};
+    const JobDev &J = jobs[wi.job];
+    JobState *const st = J.st;
+    const int W = J.W, y = wi.tile * J.rpc + b;
+    const bool ok = b < J.rpc && y < J.H;
+    const size_t base = (size_t)y * W;
+    const float2 *const X = J.X + base;
+    const uint8_t *const mask = J.mask + base;
+    float2 v[16];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) {
-            const int j = l + m * Q;
-            v[m] = ok && j < W ? J.X[base + j] : make_float2(0.f, 0.f);
-        }
-        reg16_bluestein<M, RowSwz16<M>, +1>(v, sm, b, l, rtw, J.prow);   // ends with a barrier: sm is free
-        float *nrow = reinterpret_cast<float *>(sm) + b * M;
-        double tot = 0.0, cnt = 0.0;
+    for (int m = 0; m < H8; ++m) {
+        const int j = l + m * Q;
+        v[m] = ok && j < W ? X[j] : make_float2(0.f, 0.f);
+    }
+    uint8_t mk[H8];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) {
-            const int j = l + m * Q;
-            if (j >= W) continue;
-            const float nv = cnorm_ref(v[m]);
-            nrow[j] = nv;
-            if (ok) {
-                const size_t idx = base + j;
-                J.out[idx] = v[m].x;
-                if (dbg_gprime) dbg_gprime[idx] = v[m];
-                if (c > 0 && J.mask[idx]) {
-                    tot += (double)nv;
-                    cnt += 1.0;
-                }
-            }
-        }
-        block_sum2<T>(tot, cnt, red);   // includes barriers: nrow complete after it
-        if (threadIdx.x == 0) {
-            J.err_part[2 * wi.tile] = tot;
-            J.err_part[2 * wi.tile + 1] = cnt;
-        }
+    for (int m = 0; m < H8; ++m) {
+        const int j = l + m * Q;
+        mk[m] = ok && j < W ? mask[j] : 0;
+    }
+    const int stop = st->stop, c = st->cycle;
+    if (stop) return;
+    if (wi.tile == 0 && threadIdx.x == 0) st->max_bits = 0u;
+    const int K = J.ntaps[c];
+    if (threadIdx.x < kTapStride) wsm[threadIdx.x] = J.weights[(size_t)c * kTapStride + threadIdx.x];
+    reg16_bluestein<M, RowSwz16<M>, +1>(v, sm, b, l, LdTw16<M>{J.prow.tw, l}, W, J.prow.chirp, J.prow.bspec_b);
+    __syncthreads();   // the last exchange has been read: the buffer now holds the norms
+    float *const nrow = reinterpret_cast<float *>(sm) + b * M;
+    double tot = 0.0, cnt = 0.0;
+#pragma unroll
+    for (int m = 0; m < H8; ++m) {
+        const int j = l + m * Q;
+        if (j >= W) continue;
+        const float nv = cnorm_ref(v[m]);
+        nrow[j] = nv;
         if (ok) {
-#pragma unroll
-            for (int m = 0; m < 16; ++m) {
-                const int j = l + m * Q;
-                if (j < W) J.hb[base + j] = hblur_at(nrow, W, j, wsm, K);
+            J.out[base + j] = v[m].x;
+            if (dbg_gprime) dbg_gprime[base + j] = v[m];
+            if (c > 0 && mk[m]) {
+                tot += (double)nv;
+                cnt += 1.0;
             }
         }
-        __syncthreads();
+    }
+    block_sum2<T>(tot, cnt, red);   // includes barriers: nrow complete after it
+    if (threadIdx.x == 0) {
+        J.err_part[2 * wi.tile] = tot;
+        J.err_part[2 * wi.tile + 1] = cnt;
+    }
+    // the outputs' tap sums side by side (independent chains), each in the
+    // tap order of hblur_at
+    const int hw = (K - 1) / 2;
+    float sum[H8];
+#pragma unroll
+    for (int m = 0; m < H8; ++m) sum[m] = 0.f;
+    for (int t = 0; t < K; ++t) {
+        const float wk = wsm[t];
+#pragma unroll
+        for (int m = 0; m < H8; ++m) {
+            int xs = l + m * Q - hw + t;
+            xs = xs < 0 ? 0 : (xs > W - 1 ? W - 1 : xs);
+            sum[m] = __fadd_rn(sum[m], __fmul_rn(nrow[xs], wk));
+        }
+    }
+    if (ok) {
+#pragma unroll
+        for (int m = 0; m < H8; ++m) {
+            const int j = l + m * Q;
+            if (j < W) J.hb[base + j] = sum[m];
+        }
     }
 }
 
 // column kernels: mode 0 column pass (fwd, modulus, inv), 1 column init
 // (inverse of (M, 0)), 2 plain forward, 3 plain inverse
 template <int M, int MODE>
-__device__ __forceinline__ void col_bs16_tile(float2 *X, const float *Mod, int W, int H, int x0, int cpc,
-                                              const FftPlanDev &p, const RegTw16<M> &rtw, bool guard)
+__device__ __forceinline__ void col_bs16_load(float2 (&v)[16], const float2 *X, const float *Mod, int W, int H, int x0,
+                                              int b, int l)
 {
     extern __shared__ float4 smem4[];
-    float2 *sm = reinterpret_cast<float2 *>(smem4);
-    constexpr int NB = rcol_nb(M), Q = M / 16;
-    const int b = threadIdx.x % NB, l = threadIdx.x / NB;
+    constexpr int NB = bs16_col_nb(M), Q = M / 16;
+    float *const smod = reinterpret_cast<float *>(reinterpret_cast<float2 *>(smem4) + NB * M);
     const int x = x0 + b;
-    const bool ok = b < cpc && x < W;
-    float2 v[16];
+    const bool ok = x < W;
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
+    for (int m = 0; m < 8; ++m) {
         const int j = l + m * Q;
         if (MODE == 1) v[m] = make_float2(ok && j < H ? Mod[(size_t)j * W + x] : 0.f, 0.f);
         else v[m] = ok && j < H ? X[(size_t)j * W + x] : make_float2(0.f, 0.f);
     }
     if (MODE == 0) {
-        reg16_bluestein<M, ColSwz16<M, NB>, -1>(v, sm, b, l, rtw, p);
 #pragma unroll
-        for (int m = 0; m < 16; ++m) {
+        for (int m = 0; m < 8; ++m) {
             const int j = l + m * Q;
-            const float mod = ok && j < H ? Mod[(size_t)j * W + x] : 0.f;
-            const float f = modulus_factor(mod, v[m], guard);
-            v[m] = make_float2(__fmul_rn(v[m].x, f), __fmul_rn(v[m].y, f));
+            if (ok && j < H) cp_async4(smod + j * NB + b, Mod + (size_t)j * W + x);
         }
     }
-    reg16_bluestein<M, ColSwz16<M, NB>, MODE == 2 ? -1 : +1>(v, sm, b, l, rtw, p);
+}
+template <int M, int MODE>
+__device__ __forceinline__ void col_bs16_run(float2 (&v)[16], float2 *X, int W, int H, int x0, const float2 *chirp,
+                                             const float2 *sf, const float2 *sb, const LdTw16<M> &rtw, bool guard,
+                                             int b, int l)
+{
+    extern __shared__ float4 smem4[];
+    float2 *const sm = reinterpret_cast<float2 *>(smem4);
+    constexpr int NB = bs16_col_nb(M), Q = M / 16;
+    const float *const smod = reinterpret_cast<const float *>(sm + NB * M);
+    const int x = x0 + b;
+    const bool ok = x < W;
+    if (MODE == 0) {
+        reg16_bluestein<M, ColSwz16<M, NB>, -1>(v, sm, b, l, rtw, H, chirp, sf);
+        cp_async_wait();   // each thread reads back what it copied
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            const int j = l + m * Q;
+            if (j < H) {
+                const float f = modulus_factor(ok ? smod[j * NB + b] : 0.f, v[m], guard);
+                v[m] = make_float2(__fmul_rn(v[m].x, f), __fmul_rn(v[m].y, f));
+            }
+        }
+    }
+    reg16_bluestein<M, ColSwz16<M, NB>, MODE == 2 ? -1 : +1>(v, sm, b, l, rtw, H, chirp, MODE == 2 ? sf : sb);
     if (ok) {
 #pragma unroll
-        for (int m = 0; m < 16; ++m) {
+        for (int m = 0; m < 8; ++m) {
             const int j = l + m * Q;
             if (j < H) X[(size_t)j * W + x] = v[m];
         }
@@ -1561,25 +1643,31 @@ __device__ __forceinline__ void col_bs16_tile(float2 *X, const float *Mod, int W
 }
 
 template <int M, int MODE>
-__global__ void __launch_bounds__(bs16_col_threads(M)) k_col_bs16(const JobDev *jobs, const WorkList *L)
+__global__ void __launch_bounds__(bs16_col_threads(M), bs16_min_blocks(bs16_col_threads(M)))
+k_col_bs16(const JobDev *jobs, const WorkList *L)
 {
-    constexpr int NB = rcol_nb(M);
-    const int n_items = L->n;
-    if ((int)blockIdx.x >= n_items) return;
-    RegTw16<M> rtw;
-    rtw.load(jobs[item_at(L, blockIdx.x).job].pcol.tw, threadIdx.x / NB);
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-        const WorkItem wi = item_at(L, it);
-        const JobDev &J = jobs[wi.job];
-        if (MODE == 0 && J.st->stop) continue;
-        col_bs16_tile<M, MODE>(J.X, J.M, J.W, J.H, wi.tile * J.cpc, J.cpc, J.pcol, rtw,
-                               J.mode == kModeShrinkWrap);
-        __syncthreads();
-    }
+    constexpr int NB = bs16_col_nb(M);
+    const WorkList list = list_and_job0(jobs, L);
+    if ((int)blockIdx.x >= list.n) return;
+    const LdTw16<M> rtw{jobs[list.items ? list.items[blockIdx.x].job : 0].pcol.tw, (int)threadIdx.x / NB};
+    const WorkItem wi = list.items ? list.items[blockIdx.x] : WorkItem{0, (int)blockIdx.x};
+    const JobDev &J = jobs[wi.job];
+    const JobState *const st = J.st;
+    float2 *const X = J.X;
+    const float *const Mod = J.M;
+    const int W = J.W, H = J.H, x0 = wi.tile * J.cpc;
+    const float2 *const chirp = J.pcol.chirp, *const sf = J.pcol.bspec_f, *const sb = J.pcol.bspec_b;
+    const bool guard = J.mode == kModeShrinkWrap;
+    float2 v[16];
+    const int b = threadIdx.x % NB, l = threadIdx.x / NB;
+    col_bs16_load<M, MODE>(v, X, Mod, W, H, x0, b, l);
+    if (MODE == 0 && st->stop) return;
+    col_bs16_run<M, MODE>(v, X, W, H, x0, chirp, sf, sb, LdTw16<M>{J.pcol.tw, l}, guard, b, l);
 }
 
 template <int S, int M>
-__global__ void __launch_bounds__(bs16_row_threads(M), 2) k_fft_rows_bs16(float2 *data, FftPlanDev p, int H, int rpc)
+__global__ void __launch_bounds__(bs16_row_threads(M), bs16_min_blocks(bs16_row_threads(M)))
+k_fft_rows_bs16(float2 *data, FftPlanDev p, int H, int rpc)
 {
     extern __shared__ float4 smem4[];
     float2 *sm = reinterpret_cast<float2 *>(smem4);
@@ -1589,18 +1677,17 @@ __global__ void __launch_bounds__(bs16_row_threads(M), 2) k_fft_rows_bs16(float2
     const int y = blockIdx.x * rpc + b;
     const bool ok = b < rpc && y < H;
     const size_t base = (size_t)y * n;
-    RegTw16<M> rtw;
-    rtw.load(p.tw, l);
+    const LdTw16<M> rtw{p.tw, l};
     float2 v[16];
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
+    for (int m = 0; m < 8; ++m) {
         const int j = l + m * Q;
         v[m] = ok && j < n ? data[base + j] : make_float2(0.f, 0.f);
     }
-    reg16_bluestein<M, RowSwz16<M>, S>(v, sm, b, l, rtw, p);
+    reg16_bluestein<M, RowSwz16<M>, S>(v, sm, b, l, rtw, n, p.chirp, S < 0 ? p.bspec_f : p.bspec_b);
     if (ok) {
 #pragma unroll
-        for (int m = 0; m < 16; ++m) {
+        for (int m = 0; m < 8; ++m) {
             const int j = l + m * Q;
             if (j < n) data[base + j] = v[m];
         }
@@ -1608,12 +1695,15 @@ __global__ void __launch_bounds__(bs16_row_threads(M), 2) k_fft_rows_bs16(float2
 }
 
 template <int S, int M>
-__global__ void __launch_bounds__(bs16_col_threads(M)) k_fft_cols_bs16(float2 *data, FftPlanDev p, int W, int cpc)
+__global__ void __launch_bounds__(bs16_col_threads(M), bs16_min_blocks(bs16_col_threads(M)))
+k_fft_cols_bs16(float2 *data, FftPlanDev p, int W, int cpc)
 {
-    constexpr int NB = rcol_nb(M);
-    RegTw16<M> rtw;
-    rtw.load(p.tw, threadIdx.x / NB);
-    col_bs16_tile<M, S < 0 ? 2 : 3>(data, nullptr, W, p.n, blockIdx.x * cpc, cpc, p, rtw, true);
+    constexpr int NB = bs16_col_nb(M), MODE = S < 0 ? 2 : 3;
+    const int b = threadIdx.x % NB, l = threadIdx.x / NB;
+    float2 v[16];
+    col_bs16_load<M, MODE>(v, data, nullptr, W, p.n, blockIdx.x * cpc, b, l);
+    col_bs16_run<M, MODE>(v, data, W, p.n, blockIdx.x * cpc, p.chirp, p.bspec_f, p.bspec_b, LdTw16<M>{p.tw, l}, true, b,
+                          l);
 }
 
 }  // namespace imr

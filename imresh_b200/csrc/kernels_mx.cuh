@@ -55,19 +55,6 @@ __host__ __device__ constexpr int mx_col_smem(int n)
     return 2 * mx_col_pad(n) * 8 + mx_col_pad(n) * 4 + n * 8;
 }
 
-__device__ __forceinline__ void cp_async8(void *dst, const void *src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void *dst, const void *src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait()
-{
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
 // z *= w, the twiddle step.  The schedule's rounding, pinned: forward
 // re = fma(zx, wx, -(zy wy)), im = fma(zx, wy, zy wx); an inverse transform,
 // which runs here on conjugates (see mx_fft), fuses the other product of im.
@@ -201,16 +188,6 @@ __device__ __forceinline__ int mx_fft(int a, int b, int otw, const FftPlanDev &p
         b = t;
     }
     return a;
-}
-
-// A list's header, with the first job's description requested at the same time:
-// a plan's lists (items == nullptr) always mean job 0, and the description is
-// the next thing a block reads, one memory latency (0.3 us) later.
-__device__ __forceinline__ WorkList list_and_job0(const JobDev *jobs, const WorkList *L)
-{
-    if (threadIdx.x < (sizeof(JobDev) + 127) / 128)
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(reinterpret_cast<const char *>(jobs) + 128 * threadIdx.x));
-    return *L;
 }
 
 // The plan of a length as words, one per thread, to be stored to shared memory
