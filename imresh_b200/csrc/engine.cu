@@ -272,14 +272,13 @@ int scaled_grid(const void *kernel, int threads, int smem, int items, int grid_p
 }
 
 int launch_finish(const RowKernels &rk, int items, size_t smem_fin, cudaStream_t s, const JobDev *dj,
-                  const WorkList *L, float2 *dbg, int grid_pct)
+                  const WorkList *L, float2 *dbg, int grid_pct, bool dependent)
 {
-    if (rk.p_finish)
-        rk.p_finish<<<scaled_grid((const void *)rk.p_finish, rk.threads, rk.p_smem_fin, items, grid_pct), rk.threads,
-                      rk.p_smem_fin, s>>>(dj, L, dbg);
-    else
-        rk.finish<<<items, rk.threads, smem_fin, s>>>(dj, L, dbg);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e =
+        rk.p_finish ? launch_pass(dependent, rk.p_finish,
+                                  scaled_grid((const void *)rk.p_finish, rk.threads, rk.p_smem_fin, items, grid_pct),
+                                  rk.threads, rk.p_smem_fin, s, dj, L, dbg)
+                    : launch_pass(dependent, rk.finish, items, rk.threads, smem_fin, s, dj, L, dbg);
     if (e != cudaSuccess) {
         set_error("finish launch", e);
         return IMR_ERR_CUDA;
@@ -508,6 +507,7 @@ struct imr_plan {
     WorkList *Lrow = nullptr, *Lcol = nullptr, *Lvb = nullptr;   // device
     int prec = 0;   // column pass: 0 FP32, 1 BF16 hi+lo tensor cores, 2 FP16 hi+lo tensor cores
     int g_col_tc = 0;
+    bool dependent = false;   // passes launched to start while the pass before drains
 };
 
 // The pipelined column pass of the plan's precision.
@@ -521,25 +521,27 @@ static int plan_launch_cycle(imr_plan *P, cudaStream_t s)
     const JobDev &J = P->hj;
     const RowKernels &rk = P->rk;
     const ColKernels &ck = P->ck;
-    int rc = launch_finish(rk, J.n_row_tiles, P->smem_fin, s, P->dj, P->Lrow, P->dbg_gprime);
+    const JobDev *dj = P->dj;
+    const WorkList *Lrow = P->Lrow, *Lcol = P->Lcol, *Lvb = P->Lvb;
+    const bool dep = P->dependent;
+    int rc = launch_finish(rk, J.n_row_tiles, P->smem_fin, s, dj, Lrow, P->dbg_gprime, 100, dep);
     if (rc) return rc;
-    k_vblur<<<J.n_vb_tiles, kVbThreads, 0, s>>>(P->dj, P->Lvb);
-    for (int i = 0; i < J.n_hio; ++i) {
-        if (P->p_rows) {
-            if (i == 0)
-                rk.p_hio_first<<<P->g_row_first, rk.threads, rk.p_smem_first, s>>>(P->dj, P->Lrow);
-            else
-                rk.p_hio<<<P->g_row, rk.threads, rk.p_smem, s>>>(P->dj, P->Lrow);
-        } else {
-            (i == 0 ? rk.hio_first : rk.hio)<<<J.n_row_tiles, rk.threads, P->smem_row, s>>>(P->dj, P->Lrow);
-        }
-        if (P->p_cols)
-            plan_col_kernel(P)<<<P->prec ? P->g_col_tc : P->g_col, ck.p_threads,
-                                 P->prec ? ck.p_smem_tc : ck.p_smem, s>>>(P->dj, P->Lcol);
+    cudaError_t e = launch_pass(dep, k_vblur, J.n_vb_tiles, kVbThreads, 0, s, dj, Lvb);
+    for (int i = 0; i < J.n_hio && e == cudaSuccess; ++i) {
+        if (!P->p_rows)
+            e = launch_pass(dep, i == 0 ? rk.hio_first : rk.hio, J.n_row_tiles, rk.threads, P->smem_row, s, dj, Lrow);
+        else if (i == 0)
+            e = launch_pass(dep, rk.p_hio_first, P->g_row_first, rk.threads, rk.p_smem_first, s, dj, Lrow);
         else
-            ck.col<<<J.n_col_tiles, ck.threads, P->smem_col, s>>>(P->dj, P->Lcol);
+            e = launch_pass(dep, rk.p_hio, P->g_row, rk.threads, rk.p_smem, s, dj, Lrow);
+        if (e != cudaSuccess) break;
+        if (!P->p_cols)
+            e = launch_pass(dep, ck.col, J.n_col_tiles, ck.threads, P->smem_col, s, dj, Lcol);
+        else if (P->prec)
+            e = launch_pass(false, plan_col_kernel(P), P->g_col_tc, ck.p_threads, ck.p_smem_tc, s, dj, Lcol);
+        else
+            e = launch_pass(dep, plan_col_kernel(P), P->g_col, ck.p_threads, ck.p_smem, s, dj, Lcol);
     }
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("kernel launch", e);
         return IMR_ERR_CUDA;
@@ -819,6 +821,14 @@ int imr_plan_create(imr_plan **out, unsigned W, unsigned H, const imr_params *pa
             n_split = col_split(J.n_col_tiles, g_max);
         }
         P->g_col = std::min(g_max, J.n_col_tiles + n_split);
+    }
+    {
+        const int every = 1 << 30;
+        const int r_row = P->p_rows ? persistent_grid((const void *)P->rk.p_hio, P->rk.threads, P->rk.p_smem, every)
+                                    : persistent_grid((const void *)P->rk.hio, P->rk.threads, (int)P->smem_row, every);
+        const int r_col = P->p_cols ? persistent_grid((const void *)P->ck.p_col, P->ck.p_threads, P->ck.p_smem, every)
+                                    : persistent_grid((const void *)P->ck.col, P->ck.threads, (int)P->smem_col, every);
+        P->dependent = dependent_pass(J.n_row_tiles, r_row) && dependent_pass(J.n_col_tiles + n_split, r_col);
     }
     const WorkList lists[3] = {{nullptr, J.n_row_tiles, 0}, {nullptr, J.n_col_tiles, n_split},
                                {nullptr, J.n_vb_tiles, 0}};

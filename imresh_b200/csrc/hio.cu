@@ -165,6 +165,7 @@ struct imr_hio_plan {
     bool p_rows = false, p_cols = false;
     int g_row = 0, g_col = 0;
     size_t smem_row = 0, smem_col = 0;
+    bool dependent = false;   // passes launched to start while the pass before drains
     int chunk = 0;   // iterations per graph replay
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
@@ -175,15 +176,14 @@ struct imr_hio_plan {
 static int hio_launch_iteration(imr_hio_plan *P, cudaStream_t s)
 {
     const JobDev &J = P->hj;
-    if (P->p_rows)
-        P->rk.p_hio_fix<<<P->g_row, P->rk.threads, P->rk.p_smem, s>>>(P->dj, P->Lrow);
-    else
-        P->rk.hio_fix<<<J.n_row_tiles, P->rk.threads, P->smem_row, s>>>(P->dj, P->Lrow);
-    if (P->p_cols)
-        P->ck.p_col<<<P->g_col, P->ck.p_threads, P->ck.p_smem, s>>>(P->dj, P->Lcol);
-    else
-        P->ck.col<<<J.n_col_tiles, P->ck.threads, P->smem_col, s>>>(P->dj, P->Lcol);
-    cudaError_t e = cudaGetLastError();
+    const JobDev *dj = P->dj;
+    const WorkList *Lrow = P->Lrow, *Lcol = P->Lcol;
+    cudaError_t e =
+        P->p_rows ? launch_pass(P->dependent, P->rk.p_hio_fix, P->g_row, P->rk.threads, P->rk.p_smem, s, dj, Lrow)
+                  : launch_pass(P->dependent, P->rk.hio_fix, J.n_row_tiles, P->rk.threads, P->smem_row, s, dj, Lrow);
+    if (e == cudaSuccess)
+        e = P->p_cols ? launch_pass(P->dependent, P->ck.p_col, P->g_col, P->ck.p_threads, P->ck.p_smem, s, dj, Lcol)
+                      : launch_pass(P->dependent, P->ck.col, J.n_col_tiles, P->ck.threads, P->smem_col, s, dj, Lcol);
     if (e != cudaSuccess) {
         set_error("kernel launch", e);
         return IMR_ERR_CUDA;
@@ -269,6 +269,15 @@ int imr_hio_plan_create(imr_hio_plan **out, unsigned W, unsigned H, unsigned nCy
             n_split = col_split(J.n_col_tiles, g_max);
         }
         P->g_col = std::min(g_max, J.n_col_tiles + n_split);
+    }
+    {
+        const int every = 1 << 30;
+        const int r_row = P->p_rows
+                              ? persistent_grid((const void *)P->rk.p_hio_fix, P->rk.threads, P->rk.p_smem, every)
+                              : persistent_grid((const void *)P->rk.hio_fix, P->rk.threads, (int)P->smem_row, every);
+        const int r_col = P->p_cols ? persistent_grid((const void *)P->ck.p_col, P->ck.p_threads, P->ck.p_smem, every)
+                                    : persistent_grid((const void *)P->ck.col, P->ck.threads, (int)P->smem_col, every);
+        P->dependent = dependent_pass(J.n_row_tiles, r_row) && dependent_pass(J.n_col_tiles + n_split, r_col);
     }
     const WorkList lists[2] = {{nullptr, J.n_row_tiles, 0}, {nullptr, J.n_col_tiles, n_split}};
     e = cudaMemcpy(P->Lrow, lists, sizeof(lists), cudaMemcpyHostToDevice);

@@ -49,6 +49,7 @@ __device__ __forceinline__ WorkList list_and_job0(const JobDev *jobs, const Work
 // may change between replays of a captured graph).
 #define IMR_ITEM_LOOP(BODY_CALL)                                        \
     do {                                                                \
+        pdl_wait();                                                     \
         const int n_items_ = L->n;                                      \
         for (int it_ = blockIdx.x; it_ < n_items_; it_ += gridDim.x) {  \
             const WorkItem wi = item_at(L, it_);                        \
@@ -1427,6 +1428,7 @@ k_row_hio_bs16(const JobDev *jobs, const WorkList *L)
     const size_t base = (size_t)y * W;
     const float2 *const Xi = J.X + base, *const Gi = J.G + base;
     const uint8_t *const mki = J.mask + base;
+    pdl_wait();
     float2 v[16];
 #pragma unroll
     for (int m = 0; m < H8; ++m) {
@@ -1464,6 +1466,7 @@ k_row_hio_bs16(const JobDev *jobs, const WorkList *L)
             if (ok && j < W) J.mask[base + j] = bit;
         }
     }
+    pdl_trigger();
     cp_async_wait();   // each thread reads back what it copied
     float2 *const G = J.G + base;
     const float beta = J.beta;
@@ -1519,6 +1522,7 @@ k_row_finish_bs16(const JobDev *jobs, const WorkList *L, float2 *dbg_gprime)
     const size_t base = (size_t)y * W;
     const float2 *const X = J.X + base;
     const uint8_t *const mask = J.mask + base;
+    pdl_wait();
     float2 v[16];
 #pragma unroll
     for (int m = 0; m < H8; ++m) {
@@ -1537,6 +1541,7 @@ k_row_finish_bs16(const JobDev *jobs, const WorkList *L, float2 *dbg_gprime)
     const int K = J.ntaps[c];
     if (threadIdx.x < kTapStride) wsm[threadIdx.x] = J.weights[(size_t)c * kTapStride + threadIdx.x];
     reg16_bluestein<M, RowSwz16<M>, +1>(v, sm, b, l, LdTw16<M>{J.prow.tw, l}, W, J.prow.chirp, J.prow.bspec_b);
+    pdl_trigger();
     __syncthreads();   // the last exchange has been read: the buffer now holds the norms
     float *const nrow = reinterpret_cast<float *>(sm) + b * M;
     double tot = 0.0, cnt = 0.0;
@@ -1622,6 +1627,7 @@ __device__ __forceinline__ void col_bs16_run(float2 (&v)[16], float2 *X, int W, 
     const bool ok = x < W;
     if (MODE == 0) {
         reg16_bluestein<M, ColSwz16<M, NB>, -1>(v, sm, b, l, rtw, H, chirp, sf);
+        pdl_trigger();
         cp_async_wait();   // each thread reads back what it copied
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
@@ -1660,6 +1666,7 @@ k_col_bs16(const JobDev *jobs, const WorkList *L)
     const bool guard = J.mode == kModeShrinkWrap;
     float2 v[16];
     const int b = threadIdx.x % NB, l = threadIdx.x / NB;
+    pdl_wait();
     col_bs16_load<M, MODE>(v, X, Mod, W, H, x0, b, l);
     if (MODE == 0 && st->stop) return;
     col_bs16_run<M, MODE>(v, X, W, H, x0, chirp, sf, sb, LdTw16<M>{J.pcol.tw, l}, guard, b, l);
@@ -1813,11 +1820,12 @@ __global__ void __launch_bounds__(rrow_threads(N), prow_min_blocks(FIRST, FIX, N
         mbar_fence_init();
     }
     __syncthreads();
-    int item = next_live(blockIdx.x);
-    if (threadIdx.x == 0 && item < n_items) issue(item, 0);
     // every job of this launch has row length N: one twiddle set for all items
     RegTw<N> rtw;
-    if (item < n_items) rtw.load(jobs[walk.at(item).job].prow.tw, l);
+    if ((int)blockIdx.x < n_items) rtw.load(jobs[walk.at(blockIdx.x).job].prow.tw, l);
+    pdl_wait();
+    int item = next_live(blockIdx.x);
+    if (threadIdx.x == 0 && item < n_items) issue(item, 0);
     for (int k = 0; item < n_items; ++k) {
         const int s = k & 1;
         int nxt = n_items;
@@ -1864,6 +1872,7 @@ __global__ void __launch_bounds__(rrow_threads(N), prow_min_blocks(FIRST, FIX, N
 #pragma unroll
         for (int m = 0; m < V; ++m) v[m] = sX[b * N + l + m * Q];
         reg_fft_1buf<N, RowSwz<N, NB>, +1>(v, sX, b, l, rtw);
+        if (s_next[s] >= n_items) pdl_trigger();
         const bool init_gprev = FIX ? kit == 0 : first_cycle;
         const bool track = tested && ok;
         double tot = 0.0, cnt = 0.0;
@@ -1950,10 +1959,11 @@ __global__ void __launch_bounds__(rrow_threads(N)) k_row_finish_p(const JobDev *
         mbar_fence_init();
     }
     __syncthreads();
+    RegTw<N> rtw;
+    if ((int)blockIdx.x < n_items) rtw.load(jobs[walk.at(blockIdx.x).job].prow.tw, l);
+    pdl_wait();
     int item = next_live(blockIdx.x);
     if (threadIdx.x == 0 && item < n_items) issue(item, 0);
-    RegTw<N> rtw;
-    if (item < n_items) rtw.load(jobs[walk.at(item).job].prow.tw, l);
     for (int k = 0; item < n_items; ++k) {
         const int s = k & 1;
         int nxt = n_items;
@@ -1995,6 +2005,7 @@ __global__ void __launch_bounds__(rrow_threads(N)) k_row_finish_p(const JobDev *
 #pragma unroll
         for (int m = 0; m < V; ++m) v[m] = sX[b * N + l + m * Q];
         reg_fft_1buf<N, RowSwz<N, NB>, +1>(v, sX, b, l, rtw);
+        if (s_next[s] >= n_items) pdl_trigger();
         __syncthreads();   // the FFT's last reads of the X region are done: it now holds the norms
         float *nrow = reinterpret_cast<float *>(sX) + b * N;
         double tot = 0.0, cnt = 0.0;
@@ -2093,12 +2104,13 @@ __global__ void __launch_bounds__(rcol_threads(N)) k_col_p(const JobDev *jobs, c
         mbar_init(&bars[1], 1);
         mbar_fence_init();
     }
-    int item = next_live(blockIdx.x);
-    if (item < n_items) {
-        const float2 *gtw = jobs[walk.at(item).job].pcol.tw;
+    if ((int)blockIdx.x < n_items) {
+        const float2 *gtw = jobs[walk.at(blockIdx.x).job].pcol.tw;
         for (int i = threadIdx.x; i < N; i += rcol_threads(N)) stw[i] = gtw[i];
     }
     __syncthreads();
+    pdl_wait();
+    int item = next_live(blockIdx.x);
     if (threadIdx.x == 0 && item < n_items) issue(item, 0);
     for (int k = 0; item < n_items; ++k) {
         const int nxt = next_live(item + gridDim.x);
@@ -2130,6 +2142,7 @@ __global__ void __launch_bounds__(rcol_threads(N)) k_col_p(const JobDev *jobs, c
 #pragma unroll
         for (int m = 0; m < V; ++m) v[m] = sX[(l + m * Q) * NB + b];
         reg_fft_1buf<N, ColSwz<N, NB>, -1, true>(v, sX, b, l, stw);
+        if (nxt >= n_items) pdl_trigger();
 #pragma unroll
         for (int m = 0; m < V; ++m) {
             float mod;
@@ -2247,10 +2260,11 @@ k_col_p16(const JobDev *jobs, const WorkList *L)
         }
     };
 
-    int item = walk.next(blockIdx.x);
     // the column length is N for every job of this launch: one set of twiddles
     RegTw16<N> rtw;
-    if (item < n_items) rtw.load(jobs[walk.at(item).job].pcol.tw, l);
+    if ((int)blockIdx.x < n_items) rtw.load(jobs[walk.at(blockIdx.x).job].pcol.tw, l);
+    pdl_wait();
+    int item = walk.next(blockIdx.x);
     int it_next = n_items;   // thread 0: the next item to request
     if (threadIdx.x == 0) {
         for (int t = 0; t < NST; ++t) mbar_init(&bars[t], 1);
@@ -2324,6 +2338,7 @@ k_col_p16(const JobDev *jobs, const WorkList *L)
             for (int m = 0; m < V; ++m) v[m] = sX[(l + m * Q) * NB + b];
             reg16_fft<N, ColSwz16<N, NB>, -1>(v, sX, b, l, rtw);
             if (threadIdx.x == 0) request_next(k);
+            if (s_item[(k + 1) % NST] >= n_items) pdl_trigger();
 #pragma unroll
             for (int m = 0; m < V; ++m) {
                 const float f = modulus_factor(mod[m], v[m], guard);
@@ -2375,6 +2390,7 @@ k_col_p16(const JobDev *jobs, const WorkList *L)
             for (int j = 0; j < 8; ++j) v[j] = sX[(hl + (2 * j + h) * Q) * HNB + hb];
             reg16h_fft<N, ColSwz16<N, HNB>, -1>(v, sX, mid, hb, hl, h, pair, npairs, htw);
             if (threadIdx.x == 0) request_next(k);
+            if (s_item[(k + 1) % NST] >= n_items) pdl_trigger();
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float f = modulus_factor(mod[j], v[j], guard);

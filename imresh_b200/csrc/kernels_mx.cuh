@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_hio_mx(const JobDev *j
         const float beta = J.beta;
         const bool other = job != wi.job;   // (after the barrier that ended the last item)
         const int word = other ? mx_plan_word(J.prow) : 0;
+        if (job < 0) pdl_wait();
         const int oa = 0, ob = mx_row_pad(rpc * W), og = 2 * ob, ot = og + rpc * W;
         float2 xv[V];
 #pragma unroll
@@ -271,6 +272,7 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_hio_mx(const JobDev *j
         for (int h = 0; h < 2; ++h) {
             r = mx_fft<false, T>(r, oa + ob - r, ot, sp, nr, h == 0);
             if (h == 1) break;
+            if (it + (int)gridDim.x >= l.n) pdl_trigger();
             if (FIRST) {
                 const float *const vb = J.vb + base;
                 float bl[V];
@@ -344,6 +346,7 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_finish_mx(const JobDev
         const uint8_t *const mask = J.mask + base;
         const bool other = job != wi.job;
         const int word = other ? mx_plan_word(J.prow) : 0;
+        if (job < 0) pdl_wait();
         const int oa = 0, ob = mx_row_pad(rpc * W), ot = 2 * ob + rpc * W;
         float2 xv[V];
 #pragma unroll
@@ -374,6 +377,7 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_finish_mx(const JobDev
         if (stop) continue;
         if (wi.tile == 0 && threadIdx.x == 0) st->max_bits = 0u;
         const int r = mx_fft<false, T>(oa, ob, ot, sp, nr, true);
+        if (it + (int)gridDim.x >= l.n) pdl_trigger();
         float *const nrm = reinterpret_cast<float *>(sm + oa + ob - r);
         double tot = 0.0, cnt = 0.0;
 #pragma unroll
@@ -487,7 +491,8 @@ __device__ __forceinline__ void mx_col_request(const float2 *X, const float *M, 
 }
 // the tile's work once it has arrived
 template <int MODE, int T>
-__device__ __forceinline__ void mx_col_run(float2 *X, int W, int H, int x0, const FftPlanDev &p, bool guard)
+__device__ __forceinline__ void mx_col_run(float2 *X, int W, int H, int x0, const FftPlanDev &p, bool guard,
+                                           bool last)
 {
     extern __shared__ float4 smem4[];
     float2 *const sm = reinterpret_cast<float2 *>(smem4);
@@ -499,6 +504,7 @@ __device__ __forceinline__ void mx_col_run(float2 *X, int W, int H, int x0, cons
     int r = 0;
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
+        if (last && h == 1) pdl_trigger();
         r = mx_fft<true, T>(r, ob - r, ot, p, C, MODE == 1 || MODE == 3 || h == 1);
         if (MODE != 0 || h == 1) break;
         if (ok) {
@@ -539,6 +545,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_col_mx(const JobDev *jo
         const bool guard = J.mode == kModeShrinkWrap;
         const bool other = job != wi.job;
         const int word = other ? mx_plan_word(J.pcol) : 0;
+        if (job < 0) pdl_wait();
         mx_col_request<MODE, T>(X, M, W, H, x0);
         if (other)
             for (int i = threadIdx.x; i < H; i += T) cp_async8(sm + 2 * mx_col_pad(H) + i, gtw + i);
@@ -548,7 +555,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_col_mx(const JobDev *jo
         cp_async_wait();
         __syncthreads();
         if (stop) continue;
-        mx_col_run<MODE, T>(X, W, H, x0, sp, guard);
+        mx_col_run<MODE, T>(X, W, H, x0, sp, guard, it + (int)gridDim.x >= l.n);
         __syncthreads();
     }
 }
@@ -565,7 +572,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_fft_cols_mx(float2 *dat
     for (int i = threadIdx.x; i < H; i += T) cp_async8(sm + 2 * mx_col_pad(H) + i, p.tw + i);
     cp_async_wait();
     __syncthreads();
-    mx_col_run<MODE, T>(data, W, H, x0, p, true);
+    mx_col_run<MODE, T>(data, W, H, x0, p, true, false);
 }
 
 }  // namespace imr

@@ -122,6 +122,17 @@ __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.
 __device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 
+// ---- programmatic dependent launch ------------------------------------------------
+// A pass launched with the attribute may start before the pass ahead of it has
+// ended: once all of that pass's CTAs have called pdl_trigger or exited.  What
+// it does before pdl_wait may touch only what no pass writes (work lists, job
+// descriptions, tables); pdl_wait returns when the passes ahead are complete
+// and their writes visible.  A pass triggers half-way through its last item,
+// after its own pdl_wait, so no pass runs beside the one before the last.  Both
+// are no-ops in a launch without the attribute.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- per-thread asynchronous copies (no alignment beyond the element's) --------
 __device__ __forceinline__ void cp_async8(void *dst, const void *src)
 {
