@@ -1783,6 +1783,11 @@ struct LiveWalker {
     __device__ __forceinline__ WorkItem at(int it) const { return items ? items[it] : WorkItem{0, it}; }
 };
 
+// Lengths whose pipelined passes prepare before pdl_wait and trigger half-way.
+// From 2048 on the passes are too long to gain by it, and the few instructions
+// more cost the 80-register row pass a spill (2048^2: 2 % of an iteration).
+__host__ __device__ constexpr bool pdl_length(int N) { return N < 2048; }
+
 // FIX: fixed-support HIO iteration (see b_row_hio)
 template <bool FIRST, int N, bool FIX = false>
 __global__ void __launch_bounds__(rrow_threads(N), prow_min_blocks(FIRST, FIX, N)) k_row_hio_p(const JobDev *jobs, const WorkList *L)
@@ -1822,10 +1827,11 @@ __global__ void __launch_bounds__(rrow_threads(N), prow_min_blocks(FIRST, FIX, N
     __syncthreads();
     // every job of this launch has row length N: one twiddle set for all items
     RegTw<N> rtw;
-    if ((int)blockIdx.x < n_items) rtw.load(jobs[walk.at(blockIdx.x).job].prow.tw, l);
+    if (pdl_length(N) && (int)blockIdx.x < n_items) rtw.load(jobs[walk.at(blockIdx.x).job].prow.tw, l);
     pdl_wait();
     int item = next_live(blockIdx.x);
     if (threadIdx.x == 0 && item < n_items) issue(item, 0);
+    if (!pdl_length(N) && item < n_items) rtw.load(jobs[walk.at(item).job].prow.tw, l);
     for (int k = 0; item < n_items; ++k) {
         const int s = k & 1;
         int nxt = n_items;
@@ -1872,7 +1878,7 @@ __global__ void __launch_bounds__(rrow_threads(N), prow_min_blocks(FIRST, FIX, N
 #pragma unroll
         for (int m = 0; m < V; ++m) v[m] = sX[b * N + l + m * Q];
         reg_fft_1buf<N, RowSwz<N, NB>, +1>(v, sX, b, l, rtw);
-        if (s_next[s] >= n_items) pdl_trigger();
+        if (pdl_length(N) && s_next[s] >= n_items) pdl_trigger();
         const bool init_gprev = FIX ? kit == 0 : first_cycle;
         const bool track = tested && ok;
         double tot = 0.0, cnt = 0.0;
@@ -1960,10 +1966,11 @@ __global__ void __launch_bounds__(rrow_threads(N)) k_row_finish_p(const JobDev *
     }
     __syncthreads();
     RegTw<N> rtw;
-    if ((int)blockIdx.x < n_items) rtw.load(jobs[walk.at(blockIdx.x).job].prow.tw, l);
+    if (pdl_length(N) && (int)blockIdx.x < n_items) rtw.load(jobs[walk.at(blockIdx.x).job].prow.tw, l);
     pdl_wait();
     int item = next_live(blockIdx.x);
     if (threadIdx.x == 0 && item < n_items) issue(item, 0);
+    if (!pdl_length(N) && item < n_items) rtw.load(jobs[walk.at(item).job].prow.tw, l);
     for (int k = 0; item < n_items; ++k) {
         const int s = k & 1;
         int nxt = n_items;
@@ -2005,7 +2012,7 @@ __global__ void __launch_bounds__(rrow_threads(N)) k_row_finish_p(const JobDev *
 #pragma unroll
         for (int m = 0; m < V; ++m) v[m] = sX[b * N + l + m * Q];
         reg_fft_1buf<N, RowSwz<N, NB>, +1>(v, sX, b, l, rtw);
-        if (s_next[s] >= n_items) pdl_trigger();
+        if (pdl_length(N) && s_next[s] >= n_items) pdl_trigger();
         __syncthreads();   // the FFT's last reads of the X region are done: it now holds the norms
         float *nrow = reinterpret_cast<float *>(sX) + b * N;
         double tot = 0.0, cnt = 0.0;
@@ -2262,9 +2269,10 @@ k_col_p16(const JobDev *jobs, const WorkList *L)
 
     // the column length is N for every job of this launch: one set of twiddles
     RegTw16<N> rtw;
-    if ((int)blockIdx.x < n_items) rtw.load(jobs[walk.at(blockIdx.x).job].pcol.tw, l);
+    if (pdl_length(N) && (int)blockIdx.x < n_items) rtw.load(jobs[walk.at(blockIdx.x).job].pcol.tw, l);
     pdl_wait();
     int item = walk.next(blockIdx.x);
+    if (!pdl_length(N) && item < n_items) rtw.load(jobs[walk.at(item).job].pcol.tw, l);
     int it_next = n_items;   // thread 0: the next item to request
     if (threadIdx.x == 0) {
         for (int t = 0; t < NST; ++t) mbar_init(&bars[t], 1);
@@ -2338,7 +2346,7 @@ k_col_p16(const JobDev *jobs, const WorkList *L)
             for (int m = 0; m < V; ++m) v[m] = sX[(l + m * Q) * NB + b];
             reg16_fft<N, ColSwz16<N, NB>, -1>(v, sX, b, l, rtw);
             if (threadIdx.x == 0) request_next(k);
-            if (s_item[(k + 1) % NST] >= n_items) pdl_trigger();
+            if (pdl_length(N) && s_item[(k + 1) % NST] >= n_items) pdl_trigger();
 #pragma unroll
             for (int m = 0; m < V; ++m) {
                 const float f = modulus_factor(mod[m], v[m], guard);
@@ -2390,7 +2398,7 @@ k_col_p16(const JobDev *jobs, const WorkList *L)
             for (int j = 0; j < 8; ++j) v[j] = sX[(hl + (2 * j + h) * Q) * HNB + hb];
             reg16h_fft<N, ColSwz16<N, HNB>, -1>(v, sX, mid, hb, hl, h, pair, npairs, htw);
             if (threadIdx.x == 0) request_next(k);
-            if (s_item[(k + 1) % NST] >= n_items) pdl_trigger();
+            if (pdl_length(N) && s_item[(k + 1) % NST] >= n_items) pdl_trigger();
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float f = modulus_factor(mod[j], v[j], guard);
