@@ -1157,11 +1157,20 @@ int imr_gaussian_blur(float *d_data, float *d_tmp, unsigned W, unsigned H, doubl
     const int K = gaussian_weights(sigma, t.w, kMaxTaps);
     if (K > kMaxTaps) return IMR_ERR_INVALID_VALUE;
     cudaStream_t s = (cudaStream_t)stream;
-    if (axes & 1) k_hblur<<<H, kRowThreads, (size_t)W * 4, s>>>(d_data, (int)W, (int)H, t, K);
+    // both axes: rows into the scratch image, columns back from it
+    float *const rows_out = axes == 3 ? d_tmp : d_data;
+    if (axes & 1) {
+        const int chunks = hb_row_floats((int)W) / kHbOut;
+        const int nr = std::max(1, std::min(kRowThreads / chunks, (int)H / 296));
+        const int threads = std::min(kRowThreads, (nr * chunks + 31) / 32 * 32);
+        k_hblur<<<(H + nr - 1) / nr, threads, (size_t)nr * hb_row_floats((int)W) * 4, s>>>(d_data, rows_out, (int)W,
+                                                                                         (int)H, nr, t, K);
+    }
     if (axes & 2) {
         const int nt = (int)(((W + kVbTileX - 1) / kVbTileX) * ((H + kVbTileY - 1) / kVbTileY));
-        k_vblur_plain<<<nt, kVbThreads, 0, s>>>(d_data, d_tmp, (int)W, (int)H, t, K, nullptr);
-        CK(cudaMemcpyAsync(d_data, d_tmp, (size_t)W * H * 4, cudaMemcpyDeviceToDevice, s));
+        k_vblur_plain<<<nt, kVbThreads, 0, s>>>(axes == 3 ? d_tmp : d_data, axes == 3 ? d_data : d_tmp, (int)W, (int)H, t,
+                                                K, nullptr);
+        if (axes == 2) CK(cudaMemcpyAsync(d_data, d_tmp, (size_t)W * H * 4, cudaMemcpyDeviceToDevice, s));
     }
     CK(cudaGetLastError());
     return IMR_SUCCESS;
