@@ -138,15 +138,32 @@ def _ptr(x) -> int:
     raise TypeError(f"cannot take a pointer of {type(x)}")
 
 
-def _stream(s) -> int:
-    if s is None:
+_RAW_STREAM = None
+
+
+def _current_stream() -> int:
+    """torch's current stream as a cudaStream_t; 0 without torch or a GPU."""
+    global _RAW_STREAM
+    if _RAW_STREAM is None:   # (looked up once a GPU is there)
         try:
             import torch
-            if torch.cuda.is_available():
-                return torch.cuda.current_stream().cuda_stream
+            if not torch.cuda.is_available():
+                return 0
+            torch.cuda.current_stream()   # initialises CUDA
+            raw, device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+            if raw(device()) != torch.cuda.current_stream().cuda_stream:
+                raise AttributeError
+            _RAW_STREAM = lambda: raw(device())   # noqa: E731  no Stream object per call
+        except AttributeError:
+            _RAW_STREAM = lambda: torch.cuda.current_stream().cuda_stream   # noqa: E731
         except Exception:
-            pass
-        return 0
+            return 0
+    return _RAW_STREAM()
+
+
+def _stream(s) -> int:
+    if s is None:
+        return _current_stream()
     if isinstance(s, int):
         return s
     return s.cuda_stream
@@ -300,6 +317,8 @@ class CEngineInfo(C.Structure):
 
 
 def _engine_sigs(L):
+    if L.imr_engine_set_cycles_per_step.argtypes:   # set before (last)
+        return
     vp = C.c_void_p
     L.imr_engine_create.argtypes = [C.POINTER(vp), C.c_size_t, C.c_int, vp]
     L.imr_engine_submit.argtypes = [vp, vp, vp, C.c_uint, C.c_uint, C.POINTER(CParams), C.c_longlong]
@@ -463,6 +482,8 @@ MASK_F32, MASK_U8 = 0, 1
 
 
 def _hio_sigs(L):
+    if L.imr_rand_field.argtypes:   # set before (last)
+        return
     vp, u, f, i = C.c_void_p, C.c_uint, C.c_float, C.c_int
     L.imr_hybrid_input_output.argtypes = [vp, vp, u, u, u, f, f, vp]
     L.imr_hio_plan_create.argtypes = [C.POINTER(vp), u, u, u, f, f]

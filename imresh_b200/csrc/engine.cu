@@ -211,6 +211,48 @@ int gaussian_weights(double sigma, float *w, int cap)
     return K;
 }
 
+// ---------------------------------------------------------------- scratch memory
+// Device memory of the synchronous host-buffer calls (forward model, maximum,
+// error): from one pool per device that keeps up to kScratchKeep bytes between
+// calls and gives the rest back.  The default pool gives everything back at each
+// synchronisation, and mapping it again took half of a 1000 x 800 forward model
+// (0.5 of 1.0 ms).  Stream-ordered, so calls on several streams and threads may
+// overlap.
+constexpr uint64_t kScratchKeep = 256ull << 20;
+static std::mutex g_pool_mu;
+static std::map<int, cudaMemPool_t> g_pool;
+
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    cudaMemPool_t pool = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        auto it = g_pool.find(dev);
+        if (it == g_pool.end()) {
+            cudaMemPoolProps pp;
+            memset(&pp, 0, sizeof(pp));
+            pp.allocType = cudaMemAllocationTypePinned;
+            pp.handleTypes = cudaMemHandleTypeNone;
+            pp.location.type = cudaMemLocationTypeDevice;
+            pp.location.id = dev;
+            uint64_t keep = kScratchKeep;
+            e = cudaMemPoolCreate(&pool, &pp);
+            if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            if (e != cudaSuccess) {
+                if (pool) cudaMemPoolDestroy(pool);
+                return e;
+            }
+            g_pool[dev] = pool;
+        } else {
+            pool = it->second;
+        }
+    }
+    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
 // ---------------------------------------------------------------- dispatch
 // Resident CTAs per SM of a kernel at a launch shape, asked of the occupancy
 // calculator once per (device, kernel, shape): the engine launches hundreds
@@ -454,11 +496,9 @@ int build_weight_table(const imr_params &p, std::vector<float> &w, std::vector<i
 // Unnormalised 2D transform passes over a [H][W] complex array with the
 // plain FFT kernels: axes bit 1 = rows, bit 2 = columns; sign -1 runs rows
 // then columns, +1 columns then rows.
-int fft_passes(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr, const FftPlanDev &pc,
-               cudaStream_t s)
+static int fft_launch(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr, const FftPlanDev &pc,
+                      const RowKernels &rk, const ColKernels &ck, cudaStream_t s)
 {
-    const RowKernels rk = row_kernels(W);
-    const ColKernels ck = col_kernels(H);
     const int rpc = rk.mx ? rows_per_tile(rk, W, H) : rk.nb, cpc = ck.nb;
     const int nrt = (H + rpc - 1) / rpc, nct = (W + cpc - 1) / cpc;
     const size_t sr = rk.smem ? (size_t)row_tile_smem(rk, W, rpc) : ((size_t)rpc * W + rk.bs_m) * 8;
@@ -476,6 +516,11 @@ int fft_passes(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr
         return IMR_ERR_CUDA;
     }
     return IMR_SUCCESS;
+}
+int fft_passes(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr, const FftPlanDev &pc,
+               cudaStream_t s)
+{
+    return fft_launch(d, W, H, sign, axes, pr, pc, row_kernels(W), col_kernels(H), s);
 }
 
 }  // namespace imr
@@ -1070,7 +1115,7 @@ int imr_fft2d_split(void *d_data, unsigned W, unsigned H, int sign, int precisio
     cudaStream_t s = (cudaStream_t)stream;
     char *dev = nullptr;
     const size_t jb = (sizeof(JobDev) + 255) / 256 * 256;
-    CK(cudaMallocAsync((void **)&dev, jb + 256 + 256, s));
+    CK(scratch_alloc((void **)&dev, jb + 256 + 256, s));
     JobDev *dj = (JobDev *)dev;
     WorkList *dl = (WorkList *)(dev + jb);
     JobState *dst = (JobState *)(dev + jb + 256);
@@ -1137,11 +1182,30 @@ int imr_cuda_shrink_wrap(float *io, unsigned W, unsigned H, void *stream, unsign
 int imr_fft2d(void *d_data, unsigned W, unsigned H, int sign, void *stream)
 {
     if (!d_data || W == 0 || H == 0 || (sign != 1 && sign != -1)) return IMR_ERR_INVALID_VALUE;
-    int rc = ensure_kernel_attributes();
-    if (rc) return rc;
-    FftPlanDev pr, pc;
-    if ((rc = make_fft_plan((int)W, pr)) || (rc = make_fft_plan((int)H, pc))) return rc;
-    return fft_passes((float2 *)d_data, (int)W, (int)H, sign, 3, pr, pc, (cudaStream_t)stream);
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    // the plans and kernels of the thread's last size (their tables live as long
+    // as the process)
+    static thread_local struct {
+        int dev = -1;
+        unsigned W = 0, H = 0;
+        FftPlanDev pr, pc;
+        RowKernels rk;
+        ColKernels ck;
+    } last;
+    if (last.dev != dev || last.W != W || last.H != H) {
+        last.dev = -1;
+        int rc = ensure_kernel_attributes();
+        if (rc) return rc;
+        if ((rc = make_fft_plan((int)W, last.pr)) || (rc = make_fft_plan((int)H, last.pc))) return rc;
+        last.rk = row_kernels((int)W);
+        last.ck = col_kernels((int)H);
+        last.W = W;
+        last.H = H;
+        last.dev = dev;
+    }
+    return fft_launch((float2 *)d_data, (int)W, (int)H, sign, 3, last.pr, last.pc, last.rk, last.ck,
+                      (cudaStream_t)stream);
 }
 
 int imr_gaussian_blur(float *d_data, float *d_tmp, unsigned W, unsigned H, double sigma, int axes,
@@ -1182,20 +1246,25 @@ int imr_diffraction_intensity(float *h_io, unsigned W, unsigned H, void *stream)
     if (!length_supported((int)W) || !length_supported((int)H)) return IMR_ERR_UNSUPPORTED_SIZE;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t N = (size_t)W * H;
-    float2 *d = nullptr;
-    float *f = nullptr;
-    CK(cudaMallocAsync((void **)&d, N * 8, s));
-    CK(cudaMallocAsync((void **)&f, N * 4, s));
-    CK(cudaMemcpyAsync(f, h_io, N * 4, cudaMemcpyHostToDevice, s));
+    char *buf = nullptr;
+    CK(scratch_alloc((void **)&buf, N * 12, s));
+    float2 *d = (float2 *)buf;
+    float *f = (float *)(buf + N * 8);
     const int g = (int)std::min<size_t>((N + 255) / 256, 148 * 16);
-    k_real_to_complex<<<g, 256, 0, s>>>(f, d, (long)N);
-    int rc = imr_fft2d(d, W, H, -1, stream);
+    cudaError_t e = cudaMemcpyAsync(f, h_io, N * 4, cudaMemcpyHostToDevice, s);
+    int rc = IMR_SUCCESS;
+    if (e == cudaSuccess) {
+        k_real_to_complex<<<g, 256, 0, s>>>(f, d, (long)N);
+        rc = imr_fft2d(d, W, H, -1, stream);
+    }
+    if (e == cudaSuccess && rc == IMR_SUCCESS) {
+        k_complex_norm<<<g, 256, 0, s>>>(d, f, (long)N);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h_io, f, N * 4, cudaMemcpyDeviceToHost, s);
+    }
+    cudaFreeAsync(buf, s);
     if (rc) return rc;
-    k_complex_norm<<<g, 256, 0, s>>>(d, f, (long)N);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(h_io, f, N * 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaFreeAsync(d, s));
-    CK(cudaFreeAsync(f, s));
+    CK(e);
     CK(cudaStreamSynchronize(s));
     return IMR_SUCCESS;
 }
@@ -1209,7 +1278,7 @@ int imr_vector_max(const float *d, size_t n, float *h_max, void *stream)
     }
     cudaStream_t s = (cudaStream_t)stream;
     unsigned *dk = nullptr;
-    CK(cudaMallocAsync((void **)&dk, sizeof(unsigned), s));
+    CK(scratch_alloc((void **)&dk, sizeof(unsigned), s));
     CK(cudaMemsetAsync(dk, 0, sizeof(unsigned), s));
     long blocks = (long)((n + 255) / 256);
     if (blocks > 148 * 8) blocks = 148 * 8;

@@ -42,6 +42,8 @@ int bluestein_m(int n);
 int make_fft_plan(int n, FftPlanDev &p);
 int gaussian_weights(double sigma, float *w, int cap);
 int ensure_kernel_attributes();
+// Scratch of a synchronous call (free with cudaFreeAsync on the same stream).
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s);
 void resolve_params(const imr_params *in, imr_params &out);
 int build_weight_table(const imr_params &p, std::vector<float> &w, std::vector<int> &taps);
 

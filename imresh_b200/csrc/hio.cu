@@ -427,7 +427,7 @@ int imr_calculate_hio_error(const void *d_data, const void *d_mask, int mask_typ
         const long grid = std::min<long>(((long)n + 255) / 256, 148L * 4);
         char *buf = nullptr;
         const size_t pb = (size_t)grid * 2 * sizeof(double);
-        HCK(cudaMallocAsync((void **)&buf, pb + 256, s));
+        HCK(scratch_alloc((void **)&buf, pb + 256, s));
         double *part = (double *)buf;
         double *dres = (double *)(buf + pb);
         unsigned *counter = (unsigned *)(buf + pb + 2 * sizeof(double));
