@@ -294,6 +294,42 @@ int persistent_grid(const void *kernel, int threads, int smem, int items)
     return (int)(g < items ? g : items);
 }
 
+// Tiles of the small-image passes for a W x H plan, 0 where they are not used:
+// up to 1024 sequences of up to 1024 values (HIO iteration, pipelined passes ->
+// these, both launched dependently: 64^2 6.5 -> 4.7 us, 256^2 8.1 -> 6.1, 384^2 14.4 ->
+// 8.3, 512^2 11.6 -> 8.4, 1024^2 20.1 -> 16.7).  Beyond that their tiles are many
+// and the pipelined passes' copies ahead pay again (2048 columns of 512: 10.1 us
+// against 11.3; 2048 rows of 512: 8.9 against 11.0).  They replace pipelined
+// passes only: the per-tile passes of other shapes (widths that no tensor map
+// describes) order their transforms differently.
+void narrow_tiles(const RowKernels &rk, const ColKernels &ck, bool p_cols, int W, int H, int *rows, int *cols)
+{
+    *rows = rk.n_hio && H <= 1024 ? (H + rk.n_nb - 1) / rk.n_nb : 0;
+    *cols = ck.n_col && p_cols && W <= 1024 ? (W + ck.n_nb - 1) / ck.n_nb : 0;
+}
+
+// Whether the two passes of an iteration on a W x H job are launched dependently
+// (see dependent_pass; the small-image passes always may be: one short item per
+// block, placed as SMs become free).
+bool passes_dependent(const JobDev &J, const JobShape &S, const RowKernels &rk, const ColKernels &ck, bool fix, int n_split,
+                      bool row_narrow, bool col_narrow)
+{
+    const int every = 1 << 30;
+    auto row_ok = [&] {
+        const auto pk = fix ? rk.p_hio_fix : rk.p_hio;
+        const auto k = fix ? rk.hio_fix : rk.hio;
+        return dependent_pass(J.n_row_tiles, pk ? persistent_grid((const void *)pk, rk.threads, rk.p_smem, every)
+                                                : persistent_grid((const void *)k, rk.threads, (int)S.smem_row, every));
+    };
+    auto col_ok = [&] {
+        return S.p_cols ? dependent_pass(J.n_col_tiles + n_split,
+                                         persistent_grid((const void *)ck.p_col, ck.p_threads, ck.p_smem, every))
+                        : dependent_pass(J.n_col_tiles,
+                                         persistent_grid((const void *)ck.col, ck.threads, (int)S.smem_col, every));
+    };
+    return (row_narrow || row_ok()) && (col_narrow || col_ok());
+}
+
 // A persistent column pass runs one tile per CTA at a time.  When the tiles
 // fill at most half of the resident CTAs (256^2: 16 tiles, 512^2: 32, on 148
 // SMs) every tile runs as two half tiles on two CTAs (bit-identical results):
@@ -442,6 +478,10 @@ int ensure_kernel_attributes()
         if (e == cudaSuccess && r.p_hio) e = allow_smem(r.p_hio);
         if (e == cudaSuccess && r.p_hio_first) e = allow_smem(r.p_hio_first);
         if (e == cudaSuccess) e = allow_smem(r.hio_fix);
+        if (e == cudaSuccess && r.n_hio) e = allow_smem(r.n_hio);
+        if (e == cudaSuccess && r.n_hio) e = allow_smem(r.n_hio_first);
+        if (e == cudaSuccess && r.n_hio) e = allow_smem(r.n_hio_fix);
+        if (e == cudaSuccess && c.n_col) e = allow_smem(c.n_col);
         if (e == cudaSuccess && r.p_hio_fix) e = allow_smem(r.p_hio_fix);
         if (e == cudaSuccess && r.p_finish) e = allow_smem(r.p_finish);
         if (e == cudaSuccess && c.p_col) e = allow_smem(c.p_col);
@@ -550,6 +590,8 @@ struct imr_plan {
     bool p_rows = false, p_cols = false;   // pipelined passes in use
     int g_row_first = 0, g_row = 0, g_col = 0;
     WorkList *Lrow = nullptr, *Lcol = nullptr, *Lvb = nullptr;   // device
+    int n_row_narrow = 0, n_col_narrow = 0;       // tiles of the small-image passes (0: not used)
+    WorkList *Lrow_n = nullptr, *Lcol_n = nullptr;
     int prec = 0;   // column pass: 0 FP32, 1 BF16 hi+lo tensor cores, 2 FP16 hi+lo tensor cores
     int g_col_tc = 0;
     bool dependent = false;   // passes launched to start while the pass before drains
@@ -561,31 +603,47 @@ static void (*plan_col_kernel(const imr_plan *P))(const JobDev *, const WorkList
     return P->prec ? P->ck.p_col_tc[P->prec - 1] : P->ck.p_col;
 }
 
+// The plan's row and column pass of one HIO iteration.
+static cudaError_t plan_launch_row(imr_plan *P, bool first, cudaStream_t s)
+{
+    const RowKernels &rk = P->rk;
+    const JobDev *dj = P->dj;
+    const WorkList *L = P->Lrow;
+    if (P->n_row_narrow)
+        return launch_pass(P->dependent, first ? rk.n_hio_first : rk.n_hio, P->n_row_narrow, rk.n_threads, rk.n_smem, s,
+                           dj, (const WorkList *)P->Lrow_n);
+    if (!P->p_rows)
+        return launch_pass(P->dependent, first ? rk.hio_first : rk.hio, P->hj.n_row_tiles, rk.threads, P->smem_row, s, dj,
+                           L);
+    return first ? launch_pass(P->dependent, rk.p_hio_first, P->g_row_first, rk.threads, rk.p_smem_first, s, dj, L)
+                 : launch_pass(P->dependent, rk.p_hio, P->g_row, rk.threads, rk.p_smem, s, dj, L);
+}
+static cudaError_t plan_launch_col(imr_plan *P, cudaStream_t s)
+{
+    const ColKernels &ck = P->ck;
+    const JobDev *dj = P->dj;
+    const WorkList *L = P->Lcol;
+    if (P->prec) return launch_pass(false, plan_col_kernel(P), P->g_col_tc, ck.p_threads, ck.p_smem_tc, s, dj, L);
+    if (P->n_col_narrow)
+        return launch_pass(P->dependent, ck.n_col, P->n_col_narrow, ck.n_threads, ck.n_smem, s, dj,
+                           (const WorkList *)P->Lcol_n);
+    if (!P->p_cols) return launch_pass(P->dependent, ck.col, P->hj.n_col_tiles, ck.threads, P->smem_col, s, dj, L);
+    return launch_pass(P->dependent, plan_col_kernel(P), P->g_col, ck.p_threads, ck.p_smem, s, dj, L);
+}
+
 static int plan_launch_cycle(imr_plan *P, cudaStream_t s)
 {
     const JobDev &J = P->hj;
     const RowKernels &rk = P->rk;
-    const ColKernels &ck = P->ck;
     const JobDev *dj = P->dj;
-    const WorkList *Lrow = P->Lrow, *Lcol = P->Lcol, *Lvb = P->Lvb;
+    const WorkList *Lrow = P->Lrow, *Lvb = P->Lvb;
     const bool dep = P->dependent;
     int rc = launch_finish(rk, J.n_row_tiles, P->smem_fin, s, dj, Lrow, P->dbg_gprime, 100, dep);
     if (rc) return rc;
     cudaError_t e = launch_pass(dep, k_vblur, J.n_vb_tiles, kVbThreads, 0, s, dj, Lvb);
     for (int i = 0; i < J.n_hio && e == cudaSuccess; ++i) {
-        if (!P->p_rows)
-            e = launch_pass(dep, i == 0 ? rk.hio_first : rk.hio, J.n_row_tiles, rk.threads, P->smem_row, s, dj, Lrow);
-        else if (i == 0)
-            e = launch_pass(dep, rk.p_hio_first, P->g_row_first, rk.threads, rk.p_smem_first, s, dj, Lrow);
-        else
-            e = launch_pass(dep, rk.p_hio, P->g_row, rk.threads, rk.p_smem, s, dj, Lrow);
-        if (e != cudaSuccess) break;
-        if (!P->p_cols)
-            e = launch_pass(dep, ck.col, J.n_col_tiles, ck.threads, P->smem_col, s, dj, Lcol);
-        else if (P->prec)
-            e = launch_pass(false, plan_col_kernel(P), P->g_col_tc, ck.p_threads, ck.p_smem_tc, s, dj, Lcol);
-        else
-            e = launch_pass(dep, plan_col_kernel(P), P->g_col, ck.p_threads, ck.p_smem, s, dj, Lcol);
+        e = plan_launch_row(P, i == 0, s);
+        if (e == cudaSuccess) e = plan_launch_col(P, s);
     }
     if (e != cudaSuccess) {
         set_error("kernel launch", e);
@@ -665,7 +723,8 @@ int job_prepare(unsigned W, unsigned H, const imr_params &p, JobDev &J, JobShape
     S.oMask = off; off += al(N);
     S.oW = off; off += al(S.wt.size() * 4);
     S.oT = off; off += al(S.taps.size() * 4);
-    S.oEP = off; off += al((size_t)2 * J.n_row_tiles * 8);
+    const int n_ep = std::max(J.n_row_tiles, S.rk.n_nb ? (J.H + S.rk.n_nb - 1) / S.rk.n_nb : 0);
+    S.oEP = off; off += al((size_t)2 * n_ep * 8);
     S.oErr = off; off += al((size_t)(J.n_cycles + 1) * 4);
     S.bytes = off;
     return IMR_SUCCESS;
@@ -829,7 +888,7 @@ int imr_plan_create(imr_plan **out, unsigned W, unsigned H, const imr_params *pa
         return rc;
     }
     const size_t extra = (sizeof(JobState) + 255) / 256 * 256 + (sizeof(JobDev) + 255) / 256 * 256 +
-                         (3 * sizeof(WorkList) + 255) / 256 * 256;
+                         (5 * sizeof(WorkList) + 255) / 256 * 256;
     cudaError_t e = cudaMalloc(&P->arena, S.bytes + extra);
     if (e != cudaSuccess) {
         set_error("cudaMalloc plan arena", e);
@@ -843,6 +902,8 @@ int imr_plan_create(imr_plan **out, unsigned W, unsigned H, const imr_params *pa
     P->Lrow = (WorkList *)((char *)P->dj + (sizeof(JobDev) + 255) / 256 * 256);
     P->Lcol = P->Lrow + 1;
     P->Lvb = P->Lrow + 2;
+    P->Lrow_n = P->Lrow + 3;
+    P->Lcol_n = P->Lrow + 4;
     job_bind(J, S, a, st);
     P->st = J.st;
     P->rk = S.rk;
@@ -867,16 +928,10 @@ int imr_plan_create(imr_plan **out, unsigned W, unsigned H, const imr_params *pa
         }
         P->g_col = std::min(g_max, J.n_col_tiles + n_split);
     }
-    {
-        const int every = 1 << 30;
-        const int r_row = P->p_rows ? persistent_grid((const void *)P->rk.p_hio, P->rk.threads, P->rk.p_smem, every)
-                                    : persistent_grid((const void *)P->rk.hio, P->rk.threads, (int)P->smem_row, every);
-        const int r_col = P->p_cols ? persistent_grid((const void *)P->ck.p_col, P->ck.p_threads, P->ck.p_smem, every)
-                                    : persistent_grid((const void *)P->ck.col, P->ck.threads, (int)P->smem_col, every);
-        P->dependent = dependent_pass(J.n_row_tiles, r_row) && dependent_pass(J.n_col_tiles + n_split, r_col);
-    }
-    const WorkList lists[3] = {{nullptr, J.n_row_tiles, 0}, {nullptr, J.n_col_tiles, n_split},
-                               {nullptr, J.n_vb_tiles, 0}};
+    narrow_tiles(P->rk, P->ck, P->p_cols, P->W, P->H, &P->n_row_narrow, &P->n_col_narrow);
+    P->dependent = passes_dependent(J, S, P->rk, P->ck, false, n_split, P->n_row_narrow > 0, P->n_col_narrow > 0);
+    const WorkList lists[5] = {{nullptr, J.n_row_tiles, 0}, {nullptr, J.n_col_tiles, n_split}, {nullptr, J.n_vb_tiles, 0},
+                               {nullptr, P->n_row_narrow, 0}, {nullptr, P->n_col_narrow, 0}};
     e = cudaMemcpy(P->Lrow, lists, sizeof(lists), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = job_upload(J, S, a, P->dj, 0) ? cudaErrorUnknown : cudaSuccess;
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -896,7 +951,7 @@ int imr_plan_create(imr_plan **out, unsigned W, unsigned H, const imr_params *pa
 int imr_plan_launches(imr_plan *P, long *launches)
 {
     if (!P || !launches) return IMR_ERR_INVALID_VALUE;
-    *launches = (P->hj.Mt ? 2 : 1) + (long)P->hj.n_cycles * (2 + 2L * P->hj.n_hio) + 2;
+    *launches = (P->hj.Mt && (!P->n_col_narrow || P->prec) ? 2 : 1) + (long)P->hj.n_cycles * (2 + 2L * P->hj.n_hio) + 2;
     return IMR_SUCCESS;
 }
 
@@ -907,7 +962,8 @@ int imr_plan_execute(imr_plan *P, const float *d_modulus, float *d_out, void *st
     const JobDev &J = P->hj;
     const size_t N = (size_t)P->W * P->H;
     CK(cudaMemcpyAsync((void *)J.M, d_modulus, N * 4, cudaMemcpyDeviceToDevice, s));
-    if (int rc = job_modulus_tiles(J, s)) return rc;
+    if (!P->n_col_narrow || P->prec)   // the passes that read the modulus in tiles
+        if (int rc = job_modulus_tiles(J, s)) return rc;
     CK(cudaMemsetAsync(P->st, 0, sizeof(JobState), s));
     P->ck.init<<<J.n_col_tiles, P->ck.threads, P->smem_col, s>>>(P->dj, P->Lcol);
     CK(cudaGetLastError());
@@ -927,7 +983,8 @@ int imr_plan_execute_host(imr_plan *P, const float *h_modulus, float *h_out, voi
     const JobDev &J = P->hj;
     const size_t N = (size_t)P->W * P->H;
     CK(cudaMemcpyAsync((void *)J.M, h_modulus, N * 4, cudaMemcpyHostToDevice, s));
-    if (int rc = job_modulus_tiles(J, s)) return rc;
+    if (!P->n_col_narrow || P->prec)   // the passes that read the modulus in tiles
+        if (int rc = job_modulus_tiles(J, s)) return rc;
     CK(cudaMemsetAsync(P->st, 0, sizeof(JobState), s));
     P->ck.init<<<J.n_col_tiles, P->ck.threads, P->smem_col, s>>>(P->dj, P->Lcol);
     CK(cudaGetLastError());
@@ -993,20 +1050,13 @@ static cudaError_t profile_replay(imr_plan *P, int iters, bool split, cudaStream
         int k = 0;
         cudaEventRecordWithFlags(ev[k++], cs, cudaEventRecordExternal);
         for (int i = 0; i < iters; ++i) {
-            if (P->p_rows)
-                P->rk.p_hio<<<P->g_row, P->rk.threads, P->rk.p_smem, cs>>>(P->dj, P->Lrow);
-            else
-                P->rk.hio<<<J.n_row_tiles, P->rk.threads, P->smem_row, cs>>>(P->dj, P->Lrow);
+            if (e == cudaSuccess) e = plan_launch_row(P, false, cs);
             if (split) cudaEventRecordWithFlags(ev[k++], cs, cudaEventRecordExternal);
-            if (P->p_cols)
-                plan_col_kernel(P)<<<P->prec ? P->g_col_tc : P->g_col, P->ck.p_threads,
-                                     P->prec ? P->ck.p_smem_tc : P->ck.p_smem, cs>>>(P->dj, P->Lcol);
-            else
-                P->ck.col<<<J.n_col_tiles, P->ck.threads, P->smem_col, cs>>>(P->dj, P->Lcol);
+            if (e == cudaSuccess) e = plan_launch_col(P, cs);
             if (split || i == iters - 1) cudaEventRecordWithFlags(ev[k++], cs, cudaEventRecordExternal);
         }
         const cudaError_t e2 = cudaStreamEndCapture(cs, &gr);
-        e = e2 != cudaSuccess ? e2 : cudaGraphInstantiate(&gx, gr, 0);
+        if (e == cudaSuccess) e = e2 != cudaSuccess ? e2 : cudaGraphInstantiate(&gx, gr, 0);
     }
     if (e == cudaSuccess) e = cudaMemsetAsync(P->st, 0, sizeof(JobState), s);
     if (e == cudaSuccess) e = cudaGraphLaunch(gx, s);   // warm-up

@@ -70,6 +70,11 @@ struct RowKernels {
     void (*p_finish)(const JobDev *, const WorkList *, float2 *);
     int p_smem_fin;
     int mx;        // 1: grouped-pass kernels (kernels_mx.cuh), nb is the most rows of a tile
+    // passes of small images (n_nb rows per one-item block), or null
+    void (*n_hio_first)(const JobDev *, const WorkList *);
+    void (*n_hio)(const JobDev *, const WorkList *);
+    void (*n_hio_fix)(const JobDev *, const WorkList *);
+    int n_nb, n_threads, n_smem;
 };
 // Kernels and launch shape of the column passes for one column length.
 struct ColKernels {
@@ -96,6 +101,8 @@ struct ColKernels {
     int p_smem_tc;   // their dynamic shared memory
     void (*p_col_split)(const JobDev *, const WorkList *);   // p_col running WorkList::n_split
                                                               // tiles as half tiles (JobDev::tmXh), or null
+    void (*n_col)(const JobDev *, const WorkList *);   // pass of small images (n_nb columns per one-item block), or null
+    int n_nb, n_threads, n_smem;
 };
 RowKernels row_kernels(int N);
 // Rows per tile of the per-tile row kernels on a W x H image, and the dynamic
@@ -117,6 +124,7 @@ ColKernels col_set_mx(int n);
 // Plain 2D transform passes (axes: 1 rows, 2 columns, 3 both).
 int fft_passes(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr, const FftPlanDev &pc,
                cudaStream_t s);
+void narrow_tiles(const RowKernels &rk, const ColKernels &ck, bool p_cols, int W, int H, int *rows, int *cols);
 // Persistent grid size for a pipelined kernel (CTAs per SM x SMs, <= items).
 int persistent_grid(const void *kernel, int threads, int smem, int items);
 // Launch the once-per-cycle row pass over `items` row tiles: the pipelined
@@ -158,6 +166,8 @@ struct JobShape {
     std::vector<float> wt;
     std::vector<int> taps;
 };
+bool passes_dependent(const JobDev &J, const JobShape &S, const RowKernels &rk, const ColKernels &ck, bool fix, int n_split,
+                      bool row_narrow, bool col_narrow);
 int job_prepare(unsigned W, unsigned H, const imr_params &p, JobDev &J, JobShape &S);
 void job_bind(JobDev &J, JobShape &S, char *arena, JobState *st);
 int job_upload(const JobDev &J, const JobShape &S, char *arena, JobDev *dj, cudaStream_t s);

@@ -160,6 +160,8 @@ struct imr_hio_plan {
     JobState *st = nullptr;
     void *arena = nullptr;
     WorkList *Lrow = nullptr, *Lcol = nullptr;
+    int n_row_narrow = 0, n_col_narrow = 0;   // tiles of the small-image passes (0: not used)
+    WorkList *Lrow_n = nullptr, *Lcol_n = nullptr;
     RowKernels rk{};
     ColKernels ck{};
     bool p_rows = false, p_cols = false;
@@ -177,13 +179,17 @@ static int hio_launch_iteration(imr_hio_plan *P, cudaStream_t s)
 {
     const JobDev &J = P->hj;
     const JobDev *dj = P->dj;
-    const WorkList *Lrow = P->Lrow, *Lcol = P->Lcol;
-    cudaError_t e =
-        P->p_rows ? launch_pass(P->dependent, P->rk.p_hio_fix, P->g_row, P->rk.threads, P->rk.p_smem, s, dj, Lrow)
-                  : launch_pass(P->dependent, P->rk.hio_fix, J.n_row_tiles, P->rk.threads, P->smem_row, s, dj, Lrow);
+    const WorkList *Lrow = P->n_row_narrow ? P->Lrow_n : P->Lrow, *Lcol = P->n_col_narrow ? P->Lcol_n : P->Lcol;
+    const RowKernels &rk = P->rk;
+    const ColKernels &ck = P->ck;
+    const bool dep = P->dependent;
+    cudaError_t e = P->n_row_narrow ? launch_pass(dep, rk.n_hio_fix, P->n_row_narrow, rk.n_threads, rk.n_smem, s, dj, Lrow)
+                    : P->p_rows     ? launch_pass(dep, rk.p_hio_fix, P->g_row, rk.threads, rk.p_smem, s, dj, Lrow)
+                                    : launch_pass(dep, rk.hio_fix, J.n_row_tiles, rk.threads, P->smem_row, s, dj, Lrow);
     if (e == cudaSuccess)
-        e = P->p_cols ? launch_pass(P->dependent, P->ck.p_col, P->g_col, P->ck.p_threads, P->ck.p_smem, s, dj, Lcol)
-                      : launch_pass(P->dependent, P->ck.col, J.n_col_tiles, P->ck.threads, P->smem_col, s, dj, Lcol);
+        e = P->n_col_narrow ? launch_pass(dep, ck.n_col, P->n_col_narrow, ck.n_threads, ck.n_smem, s, dj, Lcol)
+            : P->p_cols     ? launch_pass(dep, ck.p_col, P->g_col, ck.p_threads, ck.p_smem, s, dj, Lcol)
+                            : launch_pass(dep, ck.col, J.n_col_tiles, ck.threads, P->smem_col, s, dj, Lcol);
     if (e != cudaSuccess) {
         set_error("kernel launch", e);
         return IMR_ERR_CUDA;
@@ -250,6 +256,8 @@ int imr_hio_plan_create(imr_hio_plan **out, unsigned W, unsigned H, unsigned nCy
     P->dj = (JobDev *)(a + S.bytes + sst);
     P->Lrow = (WorkList *)(a + S.bytes + sst + sdj);
     P->Lcol = P->Lrow + 1;
+    P->Lrow_n = P->Lrow + 2;
+    P->Lcol_n = P->Lrow + 3;
     job_bind(J, S, a, st);
     P->st = st;
     P->rk = S.rk;
@@ -270,16 +278,10 @@ int imr_hio_plan_create(imr_hio_plan **out, unsigned W, unsigned H, unsigned nCy
         }
         P->g_col = std::min(g_max, J.n_col_tiles + n_split);
     }
-    {
-        const int every = 1 << 30;
-        const int r_row = P->p_rows
-                              ? persistent_grid((const void *)P->rk.p_hio_fix, P->rk.threads, P->rk.p_smem, every)
-                              : persistent_grid((const void *)P->rk.hio_fix, P->rk.threads, (int)P->smem_row, every);
-        const int r_col = P->p_cols ? persistent_grid((const void *)P->ck.p_col, P->ck.p_threads, P->ck.p_smem, every)
-                                    : persistent_grid((const void *)P->ck.col, P->ck.threads, (int)P->smem_col, every);
-        P->dependent = dependent_pass(J.n_row_tiles, r_row) && dependent_pass(J.n_col_tiles + n_split, r_col);
-    }
-    const WorkList lists[2] = {{nullptr, J.n_row_tiles, 0}, {nullptr, J.n_col_tiles, n_split}};
+    narrow_tiles(P->rk, P->ck, P->p_cols, P->W, P->H, &P->n_row_narrow, &P->n_col_narrow);
+    P->dependent = passes_dependent(J, S, P->rk, P->ck, true, n_split, P->n_row_narrow > 0, P->n_col_narrow > 0);
+    const WorkList lists[4] = {{nullptr, J.n_row_tiles, 0}, {nullptr, J.n_col_tiles, n_split},
+                               {nullptr, P->n_row_narrow, 0}, {nullptr, P->n_col_narrow, 0}};
     e = cudaMemcpy(P->Lrow, lists, sizeof(lists), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = job_upload(J, S, a, P->dj, 0) ? cudaErrorUnknown : cudaSuccess;
     if (e == cudaSuccess) e = cudaHostAlloc((void **)&P->h_stop, 2 * sizeof(int), cudaHostAllocDefault);
@@ -319,7 +321,7 @@ static int hio_run(imr_hio_plan *P, unsigned seed, cudaStream_t s)
     const JobDev &J = P->hj;
     const long N = (long)P->W * P->H;
     HCK(cudaMemsetAsync(P->st, 0, sizeof(JobState), s));
-    int rc = job_modulus_tiles(J, s);
+    int rc = P->n_col_narrow ? IMR_SUCCESS : job_modulus_tiles(J, s);
     if (rc) return rc;
     if ((rc = launch_rand_field(J.X, N, seed, s))) return rc;
     if ((rc = fft_passes(J.X, P->W, P->H, -1, 3, J.prow, J.pcol, s))) return rc;

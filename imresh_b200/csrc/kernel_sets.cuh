@@ -10,6 +10,29 @@
 namespace imr {
 
 template <int N>
+static void add_narrow(RowKernels &k)
+{
+    if constexpr (narrow_length(N)) {
+        k.n_hio_first = k_row_hio_n<true, N>;
+        k.n_hio = k_row_hio_n<false, N>;
+        k.n_hio_fix = k_row_hio_n<false, N, true>;
+        k.n_nb = row_n_rows(N);
+        k.n_threads = row_n_threads(N);
+        k.n_smem = row_n_smem(N);
+    }
+}
+template <int N>
+static void add_narrow(ColKernels &k)
+{
+    if constexpr (narrow_length(N)) {
+        k.n_col = k_col_n<N>;
+        k.n_nb = kColN;
+        k.n_threads = col_n_threads(N);
+        k.n_smem = col_n_smem(N);
+    }
+}
+
+template <int N>
 RowKernels row_set()
 {
     RowKernels k{};
@@ -22,6 +45,7 @@ RowKernels row_set()
         k.p_hio_fix = k_row_hio_p<false, N, true>;
         k.p_finish = k_row_finish_p<N>;
         k.p_smem_fin = pfin_smem<N>();
+        add_narrow<N>(k);
     } else if constexpr (N >= 8 && is_pow2(N)) {
         k = RowKernels{k_row_hio_r<true, N>, k_row_hio_r<false, N>, k_row_finish_r<N>,
                        k_fft_rows_r<-1, N>, k_fft_rows_r<+1, N>, rrow_nb(N), rrow_threads(N),
@@ -35,6 +59,7 @@ RowKernels row_set()
         k.p_hio_fix = k_row_hio_p<false, N, true>;
         k.p_finish = k_row_finish_p<N>;
         k.p_smem_fin = pfin_smem<N>();
+        add_narrow<N>(k);
     } else if constexpr (N < 0 && -N >= 256) {   // Bluestein lengths, 16 values per thread
         constexpr int M = -N;
         k = RowKernels{k_row_hio_bs16<true, M>, k_row_hio_bs16<false, M>, k_row_finish_bs16<M>,
@@ -69,20 +94,25 @@ ColKernels col_set()
             k.fft_tc[1][1] = k_col_tc<N, T, kPrecFp16x3, 2>;
             k.p_smem_tc = pcol_tc_smem<N, T>();
         }
+        add_narrow<N>(k);
         if constexpr (T >= 4) k.p_col_split = k_col_p16<N, T, true>;   // half tiles of >= 2 columns (16-byte TMA rows)
         return k;
-    } else if constexpr (N >= 16 && is_pow2(N))
-        return ColKernels{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
-                          rcol_nb(N), rcol_threads(N), rcol_smem(N), k_col_p<N>, pcol_smem<N>(),
-                          pcol_box_rows(N), pcol_tma_m(N) ? 1 : 0, pcol_threads(N), 0, rcol_nb(N)};
-    else if constexpr (N >= 8 && is_pow2(N))
+    } else if constexpr (N >= 16 && is_pow2(N)) {
+        ColKernels k{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
+                     rcol_nb(N), rcol_threads(N), rcol_smem(N), k_col_p<N>, pcol_smem<N>(),
+                     pcol_box_rows(N), pcol_tma_m(N) ? 1 : 0, pcol_threads(N), 0, rcol_nb(N)};
+        add_narrow<N>(k);
+        return k;
+    } else if constexpr (N >= 8 && is_pow2(N))
         return ColKernels{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
                           rcol_nb(N), rcol_threads(N), rcol_smem(N), nullptr, 0, 0, 0, 0, 0};
-    else if constexpr (is_3pow2(N))
-        return ColKernels{k_col<N>, k_col_init<N>, k_fft_cols<-1, N>, k_fft_cols<+1, N>, col_nb(N),
-                          col_threads(N), 0, k_col_p<N>, pcol_smem<N>(), pcol_box_rows(N),
-                          pcol_tma_m(N) ? 1 : 0, pcol_threads(N), 0, rcol_nb(N)};
-    else if constexpr (N < 0 && -N >= 256)   // Bluestein lengths, 16 values per thread
+    else if constexpr (is_3pow2(N)) {
+        ColKernels k{k_col<N>, k_col_init<N>, k_fft_cols<-1, N>, k_fft_cols<+1, N>, col_nb(N),
+                     col_threads(N), 0, k_col_p<N>, pcol_smem<N>(), pcol_box_rows(N),
+                     pcol_tma_m(N) ? 1 : 0, pcol_threads(N), 0, rcol_nb(N)};
+        add_narrow<N>(k);
+        return k;
+    } else if constexpr (N < 0 && -N >= 256)   // Bluestein lengths, 16 values per thread
         return ColKernels{k_col_bs16<-N, 0>, k_col_bs16<-N, 1>, k_fft_cols_bs16<-1, -N>, k_fft_cols_bs16<+1, -N>,
                           bs16_col_nb(-N), bs16_col_threads(-N), bs16_col_smem(-N), nullptr, 0, 0, 0, 0, -N, 0};
     else if constexpr (N < 0 && -N >= 8)   // Bluestein lengths: register chirp-z transforms

@@ -147,7 +147,7 @@ __device__ __forceinline__ void block_sum2(double &a, double &b, double *scratch
 // in a fixed order), applies the stop tests E_k < target (cpp:251-254) and
 // k == nCycles (cpp:255-256), and moves the job to iteration k + 1.
 template <int T>
-__device__ __forceinline__ void hio_tile_done(const JobDev &J, int tile, double tot, double cnt)
+__device__ __forceinline__ void hio_tile_done(const JobDev &J, int tile, double tot, double cnt, int n_tiles)
 {
     __shared__ double red[2 * (T / 32 > 1 ? T / 32 : 1)];
     __shared__ int s_last;
@@ -157,7 +157,7 @@ __device__ __forceinline__ void hio_tile_done(const JobDev &J, int tile, double 
         J.err_part[2 * tile] = tot;
         J.err_part[2 * tile + 1] = cnt;
         __threadfence();
-        s_last = atomicAdd(&st->counter, 1u) == (unsigned)J.n_row_tiles - 1u;
+        s_last = atomicAdd(&st->counter, 1u) == (unsigned)n_tiles - 1u;
     }
     __syncthreads();
     if (!s_last) return;
@@ -165,7 +165,7 @@ __device__ __forceinline__ void hio_tile_done(const JobDev &J, int tile, double 
     tot = 0.0;
     cnt = 0.0;
     const volatile double *ep = J.err_part;
-    for (int t = threadIdx.x; t < J.n_row_tiles; t += T) {
+    for (int t = threadIdx.x; t < n_tiles; t += T) {
         tot += ep[2 * t];
         cnt += ep[2 * t + 1];
     }
@@ -462,7 +462,7 @@ __device__ __forceinline__ void b_row_hio(const JobDev *jobs, const WorkItem wi)
         fft_rows<N, -1>(sm, nr, J.prow);
         for (int i = threadIdx.x; i < n; i += T) J.X[base + i] = sm[i];
     }
-    if (FIX) hio_tile_done<T>(J, wi.tile, tot, cnt);
+    if (FIX) hio_tile_done<T>(J, wi.tile, tot, cnt, J.n_row_tiles);
 }
 template <bool FIRST, int N, bool FIX = false>
 __global__ void __launch_bounds__(row_threads(N)) k_row_hio(const JobDev *jobs, const WorkList *L)
@@ -1038,7 +1038,7 @@ __device__ __forceinline__ void b_row_hio_r(const JobDev *jobs, const WorkItem w
             for (int m = 0; m < 8; ++m) J.X[base + l + m * Q] = v[m];
         }
     }
-    if (FIX) hio_tile_done<rrow_threads(N)>(J, wi.tile, tot, cnt);
+    if (FIX) hio_tile_done<rrow_threads(N)>(J, wi.tile, tot, cnt, J.n_row_tiles);
 }
 template <bool FIRST, int N, bool FIX = false>
 __global__ void __launch_bounds__(rrow_threads(N)) k_row_hio_r(const JobDev *jobs, const WorkList *L)
@@ -1250,7 +1250,7 @@ __device__ __forceinline__ void b_row_hio_bs(const JobDev *jobs, const WorkItem 
             }
         }
     }
-    if (FIX) hio_tile_done<rrow_threads(M)>(J, wi.tile, tot, cnt);
+    if (FIX) hio_tile_done<rrow_threads(M)>(J, wi.tile, tot, cnt, J.n_row_tiles);
 }
 template <bool FIRST, int M, bool FIX = false>
 __global__ void __launch_bounds__(rrow_threads(M)) k_row_hio_bs(const JobDev *jobs, const WorkList *L)
@@ -1608,7 +1608,7 @@ k_row_hio_bs16(const JobDev *jobs, const WorkList *L)
             }
         }
     }
-    if (FIX) hio_tile_done<T>(J, wi.tile, tot, cnt);
+    if (FIX) hio_tile_done<T>(J, wi.tile, tot, cnt, J.n_row_tiles);
 }
 
 template <int M>
@@ -2021,7 +2021,7 @@ __global__ void __launch_bounds__(rrow_threads(N), prow_min_blocks(FIRST, FIX, N
                 for (int m = 0; m < V; ++m) Xg[base + l + m * Q] = v[m];
             }
         }
-        if constexpr (FIX) hio_tile_done<rrow_threads(N)>(J, wi.tile, tot, cnt);
+        if constexpr (FIX) hio_tile_done<rrow_threads(N)>(J, wi.tile, tot, cnt, J.n_row_tiles);
         fence_proxy_async_smem();
         __syncthreads();   // stage s is free for the copy issued next iteration; s_next[s] is visible
         item = s_next[s];
@@ -2528,6 +2528,148 @@ k_col_p16(const JobDev *jobs, const WorkList *L)
         item = s_item[(k + 1) % NST];   // written before the barriers above
     }
     if (threadIdx.x == 0) bulk_wait0();
+}
+
+// ---- small images: narrow tiles ----------------------------------------------
+// A plan of a small image leaves most SMs idle with the pipelined passes' tiles
+// (256^2: 32 row tiles, 16 column tiles), and what it waits for is one tile's
+// chain of latencies.  These passes take one or two rows, or four columns, per
+// block of 64 to 256 threads: every SM works, a block's warps do not queue for
+// the same SM's pipes, and nothing is staged -- a thread loads its values
+// straight into registers (X after pdl_wait; the modulus, the twiddles and the
+// job description before it) and stores them from there.  The transforms are the
+// pipelined passes', so are the bits.  One item per block.
+constexpr int kColN = 4;   // columns of a tile: 32-byte sectors
+__host__ __device__ constexpr bool narrow_length(int N) { return N >= 64 && N <= 1024 && (is_pow2(N) || is_3pow2(N)); }
+__host__ __device__ constexpr int row_n_rows(int N) { return N / reg_v(N) >= 64 ? 1 : 64 / (N / reg_v(N)); }
+__host__ __device__ constexpr int row_n_threads(int N) { return row_n_rows(N) * (N / reg_v(N)); }
+__host__ __device__ constexpr int row_n_smem(int N) { return row_n_rows(N) * N * 8; }
+__host__ __device__ constexpr int col_n_v(int N) { return is_pow2(N) && N >= 128 ? 16 : reg_v(N); }
+__host__ __device__ constexpr int col_n_threads(int N) { return kColN * N / col_n_v(N); }
+// exchange buffer, and the twiddle table of lengths that read it there
+__host__ __device__ constexpr int col_n_smem(int N) { return kColN * N * 8 + (col_n_v(N) == 16 ? 0 : N * 8); }
+
+// row pass (see k_row_hio_p)
+template <bool FIRST, int N, bool FIX = false>
+__global__ void __launch_bounds__(row_n_threads(N)) k_row_hio_n(const JobDev *jobs, const WorkList *L)
+{
+    extern __shared__ float4 smem4[];
+    float2 *const sm = reinterpret_cast<float2 *>(smem4);
+    constexpr int NB = row_n_rows(N), V = reg_v(N), Q = N / V;
+    const WorkList list = list_and_job0(jobs, L);
+    if ((int)blockIdx.x >= list.n) return;
+    const int b = threadIdx.x / Q, l = threadIdx.x % Q;
+    const WorkItem wi = list.items ? list.items[blockIdx.x] : WorkItem{0, (int)blockIdx.x};
+    const JobDev &J = jobs[wi.job];
+    JobState *const st = J.st;
+    const int y = wi.tile * NB + b;
+    const bool ok = y < J.H;
+    const size_t base = (size_t)y * N + l;
+    float2 *const X = J.X + base, *const G = J.G + base;
+    uint8_t *const mask = J.mask + base;
+    const float beta = J.beta;
+    RegTw<N> rtw;
+    rtw.load(J.prow.tw, l);
+    pdl_wait();
+    float2 v[V], gp[V];
+    uint8_t mk[V];
+#pragma unroll
+    for (int m = 0; m < V; ++m) v[m] = ok ? X[m * Q] : make_float2(0.f, 0.f);
+    const int stop = st->stop;
+    const float thr = FIRST ? st->thr : 0.f;
+    const int k = FIX ? st->cycle : FIRST ? st->hio_cycle : 1;
+#pragma unroll
+    for (int m = 0; m < V; ++m) {   // (g_prev of a first iteration, not yet written, is not used)
+        gp[m] = ok ? G[m * Q] : make_float2(0.f, 0.f);
+        if (FIRST) mk[m] = ok && J.vb[base + m * Q] < thr ? 1 : 0;
+        else mk[m] = ok ? mask[m * Q] : 0;
+    }
+    if (stop) return;
+    const bool init_gprev = k == 0;
+    const bool fin = FIX && k >= J.n_cycles;
+    const bool track = FIX && ok && (J.target > 0.f || fin);
+    reg_fft_1buf<N, RowSwz<N, NB>, +1>(v, sm, b, l, rtw);
+    pdl_trigger();
+    double tot = 0.0, cnt = 0.0;
+#pragma unroll
+    for (int m = 0; m < V; ++m) {
+        const float2 gp1 = v[m];
+        if (FIX && track) hio_track(J.out, base + m * Q, gp1, mk[m], tot, cnt);
+        const float2 p = init_gprev ? gp1 : gp[m];
+        float2 g;
+        if ((FIX ? mk[m] == 1 : mk[m] != 0) || gp1.x < 0.f)
+            g = make_float2(__fsub_rn(p.x, __fmul_rn(beta, gp1.x)), __fsub_rn(p.y, __fmul_rn(beta, gp1.y)));
+        else
+            g = gp1;
+        if (ok && !fin) {
+            G[m * Q] = g;
+            if (FIRST) mask[m * Q] = mk[m];
+        }
+        v[m] = g;
+    }
+    if (!fin) {
+        reg_fft_1buf<N, RowSwz<N, NB>, -1>(v, sm, b, l, rtw);
+        if (ok) {
+#pragma unroll
+            for (int m = 0; m < V; ++m) X[m * Q] = v[m];
+        }
+    }
+    if constexpr (FIX) hio_tile_done<row_n_threads(N)>(J, wi.tile, tot, cnt, list.n);
+}
+
+// column pass (see k_col_p16 and, for lengths without a 16-value transform, k_col_p)
+template <int N>
+__global__ void __launch_bounds__(col_n_threads(N)) k_col_n(const JobDev *jobs, const WorkList *L)
+{
+    extern __shared__ float4 smem4[];
+    float2 *const sm = reinterpret_cast<float2 *>(smem4);
+    constexpr int NB = kColN, V = col_n_v(N), Q = N / V;
+    const WorkList list = list_and_job0(jobs, L);
+    if ((int)blockIdx.x >= list.n) return;
+    const int b = threadIdx.x % NB, l = threadIdx.x / NB;
+    const WorkItem wi = list.items ? list.items[blockIdx.x] : WorkItem{0, (int)blockIdx.x};
+    const JobDev &J = jobs[wi.job];
+    const JobState *const st = J.st;
+    const int W = J.W, x = wi.tile * NB + b;
+    const bool ok = x < W, guard = J.mode == kModeShrinkWrap;
+    const size_t base = (size_t)l * W + x, step = (size_t)Q * W;
+    float2 *const X = J.X + base;
+    const float *const M = J.M + base;
+    const float2 *const tw = J.pcol.tw;
+    float mod[V];
+#pragma unroll
+    for (int m = 0; m < V; ++m) mod[m] = ok ? M[m * step] : 0.f;
+    auto run = [&](auto &&forward, auto &&inverse) {
+        pdl_wait();
+        float2 v[V];
+#pragma unroll
+        for (int m = 0; m < V; ++m) v[m] = ok ? X[m * step] : make_float2(0.f, 0.f);
+        if (st->stop) return;
+        forward(v);
+        pdl_trigger();
+#pragma unroll
+        for (int m = 0; m < V; ++m) {
+            const float f = modulus_factor(mod[m], v[m], guard);
+            v[m] = make_float2(__fmul_rn(v[m].x, f), __fmul_rn(v[m].y, f));
+        }
+        inverse(v);
+        if (ok) {
+#pragma unroll
+            for (int m = 0; m < V; ++m) X[m * step] = v[m];
+        }
+    };
+    if constexpr (V == 16) {
+        RegTw16<N> rtw;
+        rtw.load(tw, l);
+        run([&](float2 (&v)[V]) { reg16_fft<N, ColSwz16<N, NB>, -1>(v, sm, b, l, rtw); },
+            [&](float2 (&v)[V]) { reg16_fft<N, ColSwz16<N, NB>, +1>(v, sm, b, l, rtw); });
+    } else {
+        float2 *const stw = sm + NB * N;
+        for (int i = threadIdx.x; i < N; i += col_n_threads(N)) stw[i] = tw[i];
+        __syncthreads();
+        run([&](float2 (&v)[V]) { reg_fft_1buf<N, ColSwz<N, NB>, -1, true>(v, sm, b, l, stw); },
+            [&](float2 (&v)[V]) { reg_fft_1buf<N, ColSwz<N, NB>, +1, true>(v, sm, b, l, stw); });
+    }
 }
 
 }  // namespace imr

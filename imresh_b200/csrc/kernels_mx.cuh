@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_hio_mx(const JobDev *j
                 if (i < n) X[i] = sm[r + mx_row_at(i)];
             }
         }
-        if (FIX) hio_tile_done<T>(J, wi.tile, tot, cnt);
+        if (FIX) hio_tile_done<T>(J, wi.tile, tot, cnt, J.n_row_tiles);
         __syncthreads();
     }
 }
