@@ -512,7 +512,7 @@ static int launch_cycle(imr_engine *E, cudaStream_t s, const WorkList *L, std::v
     });
     if (rc) return rc;
     if (n_vb && e == cudaSuccess) {
-        k_vblur<<<item_grid((int)n_vb), kVbThreads, 0, s>>>(dj, L + vb_base);
+        k_vblur<kVbTileY><<<item_grid((int)n_vb), kVbThreads, 0, s>>>(dj, L + vb_base);
         e = cudaGetLastError();
         ++k;
     }

@@ -594,6 +594,7 @@ struct imr_plan {
     WorkList *Lrow_n = nullptr, *Lcol_n = nullptr;
     int prec = 0;   // column pass: 0 FP32, 1 BF16 hi+lo tensor cores, 2 FP16 hi+lo tensor cores
     int g_col_tc = 0;
+    void (*vblur)(const JobDev *, const WorkList *) = k_vblur<kVbTileY>;
     bool dependent = false;   // passes launched to start while the pass before drains
 };
 
@@ -640,7 +641,7 @@ static int plan_launch_cycle(imr_plan *P, cudaStream_t s)
     const bool dep = P->dependent;
     int rc = launch_finish(rk, J.n_row_tiles, P->smem_fin, s, dj, Lrow, P->dbg_gprime, 100, dep);
     if (rc) return rc;
-    cudaError_t e = launch_pass(dep, k_vblur, J.n_vb_tiles, kVbThreads, 0, s, dj, Lvb);
+    cudaError_t e = launch_pass(dep, P->vblur, J.n_vb_tiles, kVbThreads, 0, s, dj, Lvb);
     for (int i = 0; i < J.n_hio && e == cudaSuccess; ++i) {
         e = plan_launch_row(P, i == 0, s);
         if (e == cudaSuccess) e = plan_launch_col(P, s);
@@ -930,6 +931,10 @@ int imr_plan_create(imr_plan **out, unsigned W, unsigned H, const imr_params *pa
     }
     narrow_tiles(P->rk, P->ck, P->p_cols, P->W, P->H, &P->n_row_narrow, &P->n_col_narrow);
     P->dependent = passes_dependent(J, S, P->rk, P->ck, false, n_split, P->n_row_narrow > 0, P->n_col_narrow > 0);
+    if (J.n_vb_tiles < 2 * 148) {   // tiles of 128 rows would leave SMs idle
+        J.n_vb_tiles = J.vb_tiles_x * ((J.H + kVbTileYSmall - 1) / kVbTileYSmall);
+        P->vblur = k_vblur<kVbTileYSmall>;
+    }
     const WorkList lists[5] = {{nullptr, J.n_row_tiles, 0}, {nullptr, J.n_col_tiles, n_split}, {nullptr, J.n_vb_tiles, 0},
                                {nullptr, P->n_row_narrow, 0}, {nullptr, P->n_col_narrow, 0}};
     e = cudaMemcpy(P->Lrow, lists, sizeof(lists), cudaMemcpyHostToDevice);
@@ -970,7 +975,7 @@ int imr_plan_execute(imr_plan *P, const float *d_modulus, float *d_out, void *st
     for (int c = 0; c < P->n_chunks; ++c) CK(cudaGraphLaunch(P->gexec, s));
     if (P->gexec_rem) CK(cudaGraphLaunch(P->gexec_rem, s));
     if (int rc = launch_finish(P->rk, J.n_row_tiles, P->smem_fin, s, P->dj, P->Lrow, P->dbg_gprime)) return rc;
-    k_vblur<<<J.n_vb_tiles, kVbThreads, 0, s>>>(P->dj, P->Lvb);
+    P->vblur<<<J.n_vb_tiles, kVbThreads, 0, s>>>(P->dj, P->Lvb);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(d_out, J.out, N * 4, cudaMemcpyDeviceToDevice, s));
     return IMR_SUCCESS;
@@ -991,7 +996,7 @@ int imr_plan_execute_host(imr_plan *P, const float *h_modulus, float *h_out, voi
     for (int c = 0; c < P->n_chunks; ++c) CK(cudaGraphLaunch(P->gexec, s));
     if (P->gexec_rem) CK(cudaGraphLaunch(P->gexec_rem, s));
     if (int rc = launch_finish(P->rk, J.n_row_tiles, P->smem_fin, s, P->dj, P->Lrow, P->dbg_gprime)) return rc;
-    k_vblur<<<J.n_vb_tiles, kVbThreads, 0, s>>>(P->dj, P->Lvb);
+    P->vblur<<<J.n_vb_tiles, kVbThreads, 0, s>>>(P->dj, P->Lvb);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(h_out, J.out, N * 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1281,9 +1286,14 @@ int imr_gaussian_blur(float *d_data, float *d_tmp, unsigned W, unsigned H, doubl
                                                                                          (int)H, nr, t, K);
     }
     if (axes & 2) {
-        const int nt = (int)(((W + kVbTileX - 1) / kVbTileX) * ((H + kVbTileY - 1) / kVbTileY));
-        k_vblur_plain<<<nt, kVbThreads, 0, s>>>(axes == 3 ? d_tmp : d_data, axes == 3 ? d_data : d_tmp, (int)W, (int)H, t,
-                                                K, nullptr);
+        const int tx = (int)((W + kVbTileX - 1) / kVbTileX), nt = tx * (int)((H + kVbTileY - 1) / kVbTileY);
+        const float *const in = axes == 3 ? d_tmp : d_data;
+        float *const out = axes == 3 ? d_data : d_tmp;
+        if (nt >= 2 * 148)
+            k_vblur_plain<kVbTileY><<<nt, kVbThreads, 0, s>>>(in, out, (int)W, (int)H, t, K, nullptr);
+        else   // tiles of 128 rows would leave SMs idle
+            k_vblur_plain<kVbTileYSmall><<<tx * (int)((H + kVbTileYSmall - 1) / kVbTileYSmall), kVbThreads, 0, s>>>(
+                in, out, (int)W, (int)H, t, K, nullptr);
         if (axes == 2) CK(cudaMemcpyAsync(d_data, d_tmp, (size_t)W * H * 4, cudaMemcpyDeviceToDevice, s));
     }
     CK(cudaGetLastError());

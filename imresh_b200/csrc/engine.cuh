@@ -31,7 +31,8 @@ constexpr int kMaxTaps = 63;        // Gaussian kernel taps (half width <= 31)
 constexpr int kTapStride = 64;      // floats per cycle in the weight table
 constexpr int kRowThreads = 256;
 constexpr int kVbTileX = 32;
-constexpr int kVbTileY = 128;
+constexpr int kVbTileY = 128;       // rows of a vertical blur tile
+constexpr int kVbTileYSmall = 32;   // the same where 128 leaves SMs idle
 constexpr int kVbThreads = 256;
 
 struct JobState {

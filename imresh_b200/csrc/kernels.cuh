@@ -257,25 +257,38 @@ __device__ __forceinline__ void tap_sums(float (&acc)[R], const float *w, int K,
     }
 }
 
-// Vertical clamp-border convolution of a kVbTileY x kVbTileX tile of src
+// Blur of one chunk of kRowChunk neighbouring outputs (from x0) of a row of W
+// norms that starts at element `off` of nrm; element f sits at norm_at(f), so
+// that lanes 8 elements apart hit all banks.
+constexpr int kRowChunk = 8;
+__device__ __forceinline__ int norm_at(int f) { return f ^ ((f >> 5) & 7); }
+__device__ __forceinline__ void row_chunk(float (&sum)[kRowChunk], const float *nrm, int off, int x0, int W, const float *w,
+                                          int K)
+{
+    const int a = x0 - (K - 1) / 2;
+    tap_sums(sum, w, K, [&](int i) { return nrm[norm_at(off + min(max(a + i, 0), W - 1))]; });
+}
+
+// Vertical clamp-border convolution of a TY x kVbTileX tile of src
 // (row-major [H][W]) into dst; returns the tile's max of the outputs.
 // Tap order k = -N..N as in gaussianBlurVertical (src/imresh/libs/gaussian.cpp:706-712).
-// A thread makes kVbTileY / 8 neighbouring outputs of one column (tap_sums).
-constexpr int kVbTileFloats = (kVbTileY + 2 * 31 + 1) * kVbTileX;
+// A thread makes TY / 8 neighbouring outputs of one column (tap_sums).
+__host__ __device__ constexpr int vb_tile_floats(int TY) { return (TY + 2 * 31 + 1) * kVbTileX; }
+template <int TY>
 __device__ __forceinline__ float vblur_tile(const float *src, float *dst, int W, int H, int x0,
                                             int y0, const float *w, int K, float *tile)
 {
     const int N = (K - 1) / 2;
-    const int rows_in = kVbTileY + 2 * N;
+    const int rows_in = TY + 2 * N;
     const int tx = threadIdx.x & (kVbTileX - 1);
     const int ty = threadIdx.x / kVbTileX;
     const int x = x0 + tx;
     // all of a thread's tile rows are requested before any is stored, so the
-    // loads' latencies overlap (rows_in <= kVbTileY + 62 for K <= 63 taps); in
+    // loads' latencies overlap (rows_in <= TY + 62 for K <= 63 taps); in
     // 16-byte loads where rows allow it (a quarter of the address arithmetic)
     constexpr int RS = kVbThreads / kVbTileX;
     if (W % 4 == 0 && ((uintptr_t)src & 15) == 0) {
-        constexpr int RS4 = 4 * RS, NLD = (kVbTileY + 62 + RS4 - 1) / RS4;
+        constexpr int RS4 = 4 * RS, NLD = (TY + 62 + RS4 - 1) / RS4;
         const int q = threadIdx.x & (kVbTileX / 4 - 1), r0 = threadIdx.x / (kVbTileX / 4);
         const bool in = x0 + 4 * q < W;
         float4 ld[NLD];
@@ -291,7 +304,7 @@ __device__ __forceinline__ float vblur_tile(const float *src, float *dst, int W,
             if (r < rows_in && in) reinterpret_cast<float4 *>(tile + r * kVbTileX)[q] = ld[i];
         }
     } else {
-        constexpr int NLD = (kVbTileY + 62 + RS - 1) / RS;
+        constexpr int NLD = (TY + 62 + RS - 1) / RS;
         float ld[NLD];
 #pragma unroll
         for (int i = 0; i < NLD; ++i) {
@@ -306,7 +319,7 @@ __device__ __forceinline__ float vblur_tile(const float *src, float *dst, int W,
         }
     }
     __syncthreads();
-    constexpr int R = kVbTileY / RS;
+    constexpr int R = TY / RS;
     float sum[R];
     const float *const col = tile + ty * R * kVbTileX + tx;
     tap_sums(sum, w, K, [&](int i) { return col[i * kVbTileX]; });
@@ -532,9 +545,10 @@ __global__ void __launch_bounds__(row_threads(N)) k_row_finish(const JobDev *job
 // the previous cycle (cudaVectorReduce.cu:357-403) and the stop test
 // E < target (cudaShrinkWrap.cu:374-375), then the threshold
 // (cycle 0 ? cutOffAutoCorel : cutOff) * max (cudaShrinkWrap.cu:274-276).
+template <int TY>
 __device__ __forceinline__ void b_vblur(const JobDev *jobs, const WorkItem wi)
 {
-    __shared__ __align__(16) float tile[kVbTileFloats];
+    __shared__ __align__(16) float tile[vb_tile_floats(TY)];
     __shared__ float wsm[kTapStride];
     __shared__ float fred[kVbThreads / 32];
     __shared__ double red[2 * kVbThreads / 32];
@@ -547,7 +561,7 @@ __device__ __forceinline__ void b_vblur(const JobDev *jobs, const WorkItem wi)
     if (threadIdx.x < kTapStride) wsm[threadIdx.x] = J.weights[(size_t)c * kTapStride + threadIdx.x];
     const int tx = wi.tile % J.vb_tiles_x, ty = wi.tile / J.vb_tiles_x;
     __syncthreads();
-    float mx = vblur_tile(J.hb, J.vb, J.W, J.H, tx * kVbTileX, ty * kVbTileY, wsm, K, tile);
+    float mx = vblur_tile<TY>(J.hb, J.vb, J.W, J.H, tx * kVbTileX, ty * TY, wsm, K, tile);
     mx = block_max<kVbThreads>(mx, fred);
     if (threadIdx.x == 0) {
         atomicMax(&st->max_bits, __float_as_uint(mx));
@@ -584,9 +598,13 @@ __device__ __forceinline__ void b_vblur(const JobDev *jobs, const WorkItem wi)
         __threadfence();
     }
 }
+// TY: rows of a tile.  32 instead of 128 where that leaves SMs idle: a tile is a
+// chain of loads, a barrier and K taps per output, 12 us at 128 rows however few
+// the tiles.
+template <int TY>
 static __global__ void __launch_bounds__(kVbThreads, 4) k_vblur(const JobDev *jobs, const WorkList *L)
 {
-    IMR_ITEM_LOOP((b_vblur(jobs, wi)));
+    IMR_ITEM_LOOP((b_vblur<TY>(jobs, wi)));
 }
 
 // ---------------------------------------------------------------- plain FFT
@@ -713,17 +731,18 @@ static __global__ void __launch_bounds__(kRowThreads) k_hblur(const float *src, 
     }
 }
 
+template <int TY>
 static __global__ void __launch_bounds__(kVbThreads, 4) k_vblur_plain(const float *src, float *dst, int W, int H,
                                                            Taps w, int K, unsigned *max_bits)
 {
-    __shared__ __align__(16) float tile[kVbTileFloats];
+    __shared__ __align__(16) float tile[vb_tile_floats(TY)];
     __shared__ float wsm[kTapStride];
     __shared__ float fred[kVbThreads / 32];
     if (threadIdx.x < kTapStride) wsm[threadIdx.x] = w.w[threadIdx.x];
     __syncthreads();
     const int tiles_x = (W + kVbTileX - 1) / kVbTileX;
     const int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
-    float mx = vblur_tile(src, dst, W, H, tx * kVbTileX, ty * kVbTileY, wsm, K, tile);
+    float mx = vblur_tile<TY>(src, dst, W, H, tx * kVbTileX, ty * TY, wsm, K, tile);
     mx = block_max<kVbThreads>(mx, fred);
     if (threadIdx.x == 0 && max_bits) atomicMax(max_bits, __float_as_uint(mx));
 }
@@ -1652,14 +1671,14 @@ k_row_finish_bs16(const JobDev *jobs, const WorkList *L, float2 *dbg_gprime)
     reg16_bluestein<M, RowSwz16<M>, +1>(v, sm, b, l, LdTw16<M>{J.prow.tw, l}, W, J.prow.chirp, J.prow.bspec_b);
     pdl_trigger();
     __syncthreads();   // the last exchange has been read: the buffer now holds the norms
-    float *const nrow = reinterpret_cast<float *>(sm) + b * M;
+    float *const nrm = reinterpret_cast<float *>(sm);
     double tot = 0.0, cnt = 0.0;
 #pragma unroll
     for (int m = 0; m < H8; ++m) {
         const int j = l + m * Q;
         if (j >= W) continue;
         const float nv = cnorm_ref(v[m]);
-        nrow[j] = nv;
+        nrm[norm_at(b * M + j)] = nv;
         if (ok) {
             J.out[base + j] = v[m].x;
             if (dbg_gprime) dbg_gprime[base + j] = v[m];
@@ -1669,31 +1688,26 @@ k_row_finish_bs16(const JobDev *jobs, const WorkList *L, float2 *dbg_gprime)
             }
         }
     }
-    block_sum2<T>(tot, cnt, red);   // includes barriers: nrow complete after it
+    block_sum2<T>(tot, cnt, red);   // includes barriers: the norms are complete after it
     if (threadIdx.x == 0) {
         J.err_part[2 * wi.tile] = tot;
         J.err_part[2 * wi.tile + 1] = cnt;
     }
-    // the outputs' tap sums side by side (independent chains), each in the
-    // tap order of hblur_at
-    const int hw = (K - 1) / 2;
-    float sum[H8];
+    // M/16 threads per row make 8 outputs each: M/2 >= W.  They leave through the
+    // buffer's free half, coalesced whatever the width.
+    float *const out = nrm + bs16_rows(M) * M;
+    if (ok && l * kRowChunk < W) {
+        float sum[kRowChunk];
+        row_chunk(sum, nrm, b * M, l * kRowChunk, W, wsm, K);
 #pragma unroll
-    for (int m = 0; m < H8; ++m) sum[m] = 0.f;
-    for (int t = 0; t < K; ++t) {
-        const float wk = wsm[t];
-#pragma unroll
-        for (int m = 0; m < H8; ++m) {
-            int xs = l + m * Q - hw + t;
-            xs = xs < 0 ? 0 : (xs > W - 1 ? W - 1 : xs);
-            sum[m] = __fadd_rn(sum[m], __fmul_rn(nrow[xs], wk));
-        }
+        for (int o = 0; o < kRowChunk; ++o) out[norm_at(b * M + l * kRowChunk + o)] = sum[o];
     }
+    __syncthreads();
     if (ok) {
 #pragma unroll
         for (int m = 0; m < H8; ++m) {
             const int j = l + m * Q;
-            if (j < W) J.hb[base + j] = sum[m];
+            if (j < W) J.hb[base + j] = out[norm_at(b * M + j)];
         }
     }
 }
@@ -2123,13 +2137,13 @@ __global__ void __launch_bounds__(rrow_threads(N)) k_row_finish_p(const JobDev *
         reg_fft_1buf<N, RowSwz<N, NB>, +1>(v, sX, b, l, rtw);
         if (pdl_length(N) && s_next[s] >= n_items) pdl_trigger();
         __syncthreads();   // the FFT's last reads of the X region are done: it now holds the norms
-        float *nrow = reinterpret_cast<float *>(sX) + b * N;
+        float *const nrm = reinterpret_cast<float *>(sX);
         double tot = 0.0, cnt = 0.0;
 #pragma unroll
         for (int m = 0; m < V; ++m) {
             const int e = l + m * Q;
             const float nv = cnorm_ref(v[m]);
-            nrow[e] = nv;
+            nrm[norm_at(b * N + e)] = nv;
             if (ok) {
                 outp[base + e] = v[m].x;
                 if (dbg_gprime) dbg_gprime[base + e] = v[m];
@@ -2139,29 +2153,19 @@ __global__ void __launch_bounds__(rrow_threads(N)) k_row_finish_p(const JobDev *
                 }
             }
         }
-        block_sum2<T>(tot, cnt, red);   // includes barriers: nrow complete after it
+        block_sum2<T>(tot, cnt, red);   // includes barriers: the norms are complete after it
         if (threadIdx.x == 0) {
             J.err_part[2 * wi.tile] = tot;
             J.err_part[2 * wi.tile + 1] = cnt;
         }
-        if (ok) {
-            // the V outputs' tap sums side by side (independent chains), each
-            // in the tap order of hblur_at
-            const int hw = (K - 1) / 2;
-            float sum[V];
-#pragma unroll
-            for (int m = 0; m < V; ++m) sum[m] = 0.f;
-            for (int k = 0; k < K; ++k) {
-                const float wk = wsm[k];
-#pragma unroll
-                for (int m = 0; m < V; ++m) {
-                    int xs = l + m * Q - hw + k;
-                    xs = xs < 0 ? 0 : (xs > N - 1 ? N - 1 : xs);
-                    sum[m] = __fadd_rn(sum[m], __fmul_rn(nrow[xs], wk));
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < V; ++m) hbp[base + l + m * Q] = sum[m];
+        const int rows = min(rpc, H - wi.tile * rpc);
+        for (int q = threadIdx.x; q < rows * (N / kRowChunk); q += T) {
+            const int r = q / (N / kRowChunk), x0 = (q - r * (N / kRowChunk)) * kRowChunk;
+            float sum[kRowChunk];
+            row_chunk(sum, nrm, r * N, x0, N, wsm, K);
+            float4 *const o = reinterpret_cast<float4 *>(hbp + (size_t)(wi.tile * rpc + r) * N + x0);
+            o[0] = make_float4(sum[0], sum[1], sum[2], sum[3]);
+            o[1] = make_float4(sum[4], sum[5], sum[6], sum[7]);
         }
         fence_proxy_async_smem();
         __syncthreads();   // stage s is free for the copy issued next iteration; s_next[s] is visible

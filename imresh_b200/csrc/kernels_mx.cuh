@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_finish_mx(const JobDev
             J.out[base + i] = g.x;
             if (dbg_gprime) dbg_gprime[base + i] = g;
             const float v = cnorm_ref(g);
-            nrm[i] = v;
+            nrm[norm_at(i)] = v;
             if (c > 0 && mk[m]) {
                 tot += (double)v;
                 cnt += 1.0;
@@ -400,31 +400,23 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_finish_mx(const JobDev
             J.err_part[2 * wi.tile] = tot;
             J.err_part[2 * wi.tile + 1] = cnt;
         }
-        // the V outputs' tap sums side by side (independent chains), each in
-        // the tap order of hblur_at
-        const int hw = (K - 1) / 2;
-        float sum[V];
-        int x[V], row[V];
+        // chunks of 8 neighbouring outputs; they leave through the transform's
+        // buffer, coalesced whatever the width
+        float *const out = reinterpret_cast<float *>(sm + r);
+        const int cpr = (W + kRowChunk - 1) / kRowChunk;
+        for (int q = threadIdx.x; q < nr * cpr; q += T) {
+            const int row = q / cpr, x0 = (q - row * cpr) * kRowChunk;
+            float sum[kRowChunk];
+            row_chunk(sum, nrm, row * W, x0, W, wsm, K);
 #pragma unroll
-        for (int m = 0; m < V; ++m) {
-            const int i = min((int)(threadIdx.x + m * T), n - 1);
-            row[m] = i / W * W;
-            x[m] = i - row[m];
-            sum[m] = 0.f;
+            for (int o = 0; o < kRowChunk; ++o)
+                if (x0 + o < W) out[norm_at(row * W + x0 + o)] = sum[o];
         }
-        for (int t = 0; t < K; ++t) {
-            const float wk = wsm[t];
-#pragma unroll
-            for (int m = 0; m < V; ++m) {
-                int xs = x[m] - hw + t;
-                xs = xs < 0 ? 0 : (xs > W - 1 ? W - 1 : xs);
-                sum[m] = __fadd_rn(sum[m], __fmul_rn(nrm[row[m] + xs], wk));
-            }
-        }
+        __syncthreads();
 #pragma unroll
         for (int m = 0; m < V; ++m) {
             const int i = threadIdx.x + m * T;
-            if (i < n) J.hb[base + i] = sum[m];
+            if (i < n) J.hb[base + i] = out[norm_at(i)];
         }
         __syncthreads();
     }
