@@ -139,6 +139,7 @@ struct Group {
     RowKernels rk{};
     ColKernels ck{};
     size_t smem = 0, smem_fin = 0;
+    size_t px = 0;                 // pixels of its jobs
     std::vector<WorkItem> items;   // sorted by job n_hio, descending
     std::vector<int> hio_count;    // items whose job runs iteration i
     int list_base = 0;             // index of this group's first WorkList header
@@ -461,6 +462,7 @@ static void build_groups(const std::vector<EJob *> &jobs, bool rows, std::vector
         for (EJob *j : v) {
             g.smem = std::max(g.smem, rows ? j->S.smem_row : j->S.smem_col);
             g.smem_fin = std::max(g.smem_fin, j->S.smem_fin);
+            g.px += (size_t)j->W * j->H;
             const int nt = rows ? j->J.n_row_tiles : j->J.n_col_tiles;
             for (int t = 0; t < nt; ++t) g.items.push_back(WorkItem{j->slot, t});
             max_hio = std::max(max_hio, j->J.n_hio);
@@ -475,25 +477,26 @@ static void build_groups(const std::vector<EJob *> &jobs, bool rows, std::vector
 }
 
 // Run launch(g, stream) for the groups of one pass.  Groups do not depend on one
-// another, so on the capturing stream s each beyond the first is a branch of
-// the step graph, joined again after the pass: the groups fill one another's
-// partly empty waves (48 reconstructions of five sides each way: 54.2 -> 43.5 ms
-// of device time, five launches per pass one after another before).
+// another, so they run as two branches of the step graph that join after the
+// pass: each fills the other's partly empty waves.  They alternate between the
+// branches, largest first, so that one launch is always queued behind the running
+// one (dealt out by pixels instead, two launches end up in one branch: 49 ms).
+// Measured for 48 reconstructions of five sides each way (device time, then the
+// first step of a new engine, which instantiates the graph): one branch 54.2 ms and
+// 1.9 ms, two 41.9 and 2.1, three 39.9 and 5.3, five 39.8 and 8.7 -- more branches
+// cost a new set of requests more than they give it.
 template <class F>
 static cudaError_t branch_groups(imr_engine *E, cudaStream_t s, std::vector<Group> &groups, F &&launch)
 {
     if (groups.size() < 2) return groups.empty() ? cudaSuccess : launch(groups[0], s);
+    std::vector<Group *> order;
+    for (Group &g : groups) order.push_back(&g);
+    std::stable_sort(order.begin(), order.end(), [](const Group *a, const Group *b) { return a->px > b->px; });
     cudaError_t e = cudaEventRecord(E->ev_fork, s);
-    const int nb = (int)std::min<size_t>(groups.size(), kBranchStreams + 1);   // branch 0: s itself
-    for (int b = 1; b < nb && e == cudaSuccess; ++b) e = cudaStreamWaitEvent(E->bs[b - 1], E->ev_fork, 0);
-    for (size_t g = 0; g < groups.size() && e == cudaSuccess; ++g) {
-        const int b = (int)(g % nb);
-        e = launch(groups[g], b ? E->bs[b - 1] : s);
-    }
-    for (int b = 1; b < nb && e == cudaSuccess; ++b) {
-        e = cudaEventRecord(E->ev_join[b - 1], E->bs[b - 1]);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, E->ev_join[b - 1], 0);
-    }
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(E->bs[0], E->ev_fork, 0);
+    for (size_t g = 0; g < order.size() && e == cudaSuccess; ++g) e = launch(*order[g], g & 1 ? E->bs[0] : s);
+    if (e == cudaSuccess) e = cudaEventRecord(E->ev_join[0], E->bs[0]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, E->ev_join[0], 0);
     return e;
 }
 
