@@ -10,7 +10,7 @@
 namespace imr {
 
 template <int N>
-static void add_narrow(RowKernels &k)
+static void add_shapes(RowKernels &k)
 {
     if constexpr (narrow_length(N)) {
         k.n_hio_first = k_row_hio_n<true, N>;
@@ -22,8 +22,13 @@ static void add_narrow(RowKernels &k)
     }
 }
 template <int N>
-static void add_narrow(ColKernels &k)
+static void add_shapes(ColKernels &k)
 {
+    if constexpr (is_pow2(N)) {
+        k.f_nb = fcol_nb(N);
+        k.f_threads = fcol_threads(N);
+        k.f_smem = fcol_smem(N);
+    }
     if constexpr (narrow_length(N)) {
         k.n_col = k_col_n<N>;
         k.n_nb = kColN;
@@ -45,7 +50,7 @@ RowKernels row_set()
         k.p_hio_fix = k_row_hio_p<false, N, true>;
         k.p_finish = k_row_finish_p<N>;
         k.p_smem_fin = pfin_smem<N>();
-        add_narrow<N>(k);
+        add_shapes<N>(k);
     } else if constexpr (N >= 8 && is_pow2(N)) {
         k = RowKernels{k_row_hio_r<true, N>, k_row_hio_r<false, N>, k_row_finish_r<N>,
                        k_fft_rows_r<-1, N>, k_fft_rows_r<+1, N>, rrow_nb(N), rrow_threads(N),
@@ -59,7 +64,7 @@ RowKernels row_set()
         k.p_hio_fix = k_row_hio_p<false, N, true>;
         k.p_finish = k_row_finish_p<N>;
         k.p_smem_fin = pfin_smem<N>();
-        add_narrow<N>(k);
+        add_shapes<N>(k);
     } else if constexpr (N < 0 && -N >= 256) {   // Bluestein lengths, 16 values per thread
         constexpr int M = -N;
         k = RowKernels{k_row_hio_bs16<true, M>, k_row_hio_bs16<false, M>, k_row_finish_bs16<M>,
@@ -94,14 +99,14 @@ ColKernels col_set()
             k.fft_tc[1][1] = k_col_tc<N, T, kPrecFp16x3, 2>;
             k.p_smem_tc = pcol_tc_smem<N, T>();
         }
-        add_narrow<N>(k);
+        add_shapes<N>(k);
         if constexpr (T >= 4) k.p_col_split = k_col_p16<N, T, true>;   // half tiles of >= 2 columns (16-byte TMA rows)
         return k;
     } else if constexpr (N >= 16 && is_pow2(N)) {
         ColKernels k{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
                      rcol_nb(N), rcol_threads(N), rcol_smem(N), k_col_p<N>, pcol_smem<N>(),
                      pcol_box_rows(N), pcol_tma_m(N) ? 1 : 0, pcol_threads(N), 0, rcol_nb(N)};
-        add_narrow<N>(k);
+        add_shapes<N>(k);
         return k;
     } else if constexpr (N >= 8 && is_pow2(N))
         return ColKernels{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
@@ -110,7 +115,7 @@ ColKernels col_set()
         ColKernels k{k_col<N>, k_col_init<N>, k_fft_cols<-1, N>, k_fft_cols<+1, N>, col_nb(N),
                      col_threads(N), 0, k_col_p<N>, pcol_smem<N>(), pcol_box_rows(N),
                      pcol_tma_m(N) ? 1 : 0, pcol_threads(N), 0, rcol_nb(N)};
-        add_narrow<N>(k);
+        add_shapes<N>(k);
         return k;
     } else if constexpr (N < 0 && -N >= 256)   // Bluestein lengths, 16 values per thread
         return ColKernels{k_col_bs16<-N, 0>, k_col_bs16<-N, 1>, k_fft_cols_bs16<-1, -N>, k_fft_cols_bs16<+1, -N>,

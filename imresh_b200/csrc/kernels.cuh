@@ -620,9 +620,11 @@ __global__ void __launch_bounds__(row_threads(N)) k_fft_rows(float2 *data, FftPl
     const int nr = min(rpc, H - y0);
     const int n = nr * W;
     const size_t base = (size_t)y0 * W;
+    pdl_wait();
     for (int i = threadIdx.x; i < n; i += T) sm[i] = data[base + i];
     __syncthreads();
     fft_rows<N, S>(sm, nr, p);
+    pdl_trigger();
     for (int i = threadIdx.x; i < n; i += T) data[base + i] = sm[i];
 }
 
@@ -636,12 +638,14 @@ __global__ void __launch_bounds__(col_threads(N)) k_fft_cols(float2 *data, FftPl
     const int x0 = blockIdx.x * cpc;
     const int nc = min(cpc, W - x0);
     constexpr int es = col_nb(N);
+    pdl_wait();
     for (int i = threadIdx.x; i < H * nc; i += T) {
         const int y = i / nc, c = i - y * nc;
         sm[y * es + c] = data[(size_t)y * W + x0 + c];
     }
     __syncthreads();
     fft_cols<N, S>(sm, nc, p);
+    pdl_trigger();
     for (int i = threadIdx.x; i < H * nc; i += T) {
         const int y = i / nc, c = i - y * nc;
         data[(size_t)y * W + x0 + c] = sm[y * es + c];
@@ -1136,29 +1140,38 @@ __global__ void __launch_bounds__(rrow_threads(N)) k_fft_rows_r(float2 *data, Ff
     const int y = blockIdx.x * rpc + b;
     const bool ok = b < rpc && y < H;
     const size_t base = (size_t)y * N;
+    pdl_wait();
     float2 v[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) v[m] = ok ? data[base + l + m * Q] : make_float2(0.f, 0.f);
     reg_fft<N, rrow_nb(N), false, S>(v, sm, b, l, p.tw);
+    pdl_trigger();
     if (ok) {
 #pragma unroll
         for (int m = 0; m < 8; ++m) data[base + l + m * Q] = v[m];
     }
 }
 
+// Columns of a tile: four (two at 4096): smaller blocks fill the SMs of a small
+// image (128 x 1024: 12.3 -> 8.5 us a transform; two columns at 2048^2: 59 us, four 51).
+__host__ __device__ constexpr int fcol_nb(int N) { return N <= 2048 ? 4 : 2; }
+__host__ __device__ constexpr int fcol_threads(int N) { return fcol_nb(N) * N / 8; }
+__host__ __device__ constexpr int fcol_smem(int N) { return reg_smem_bytes(N, fcol_nb(N)); }
 template <int S, int N>
-__global__ void __launch_bounds__(rcol_threads(N)) k_fft_cols_r(float2 *data, FftPlanDev p, int W, int cpc)
+__global__ void __launch_bounds__(fcol_threads(N)) k_fft_cols_r(float2 *data, FftPlanDev p, int W, int cpc)
 {
     extern __shared__ float4 smem4[];
     float2 *sm = reinterpret_cast<float2 *>(smem4);
-    constexpr int NB = rcol_nb(N), Q = N / 8;
+    constexpr int NB = fcol_nb(N), Q = N / 8;
     const int b = threadIdx.x % NB, l = threadIdx.x / NB;
     const int x = blockIdx.x * cpc + b;
     const bool ok = b < cpc && x < W;
+    pdl_wait();
     float2 v[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) v[m] = ok ? data[(size_t)(l + m * Q) * W + x] : make_float2(0.f, 0.f);
     reg_fft<N, NB, true, S>(v, sm, b, l, p.tw);
+    pdl_trigger();
     if (ok) {
 #pragma unroll
         for (int m = 0; m < 8; ++m) data[(size_t)(l + m * Q) * W + x] = v[m];
@@ -1431,6 +1444,7 @@ __global__ void __launch_bounds__(rrow_threads(M)) k_fft_rows_bs(float2 *data, F
     const int y = blockIdx.x * rpc + b;
     const bool ok = b < rpc && y < H;
     const size_t base = (size_t)y * n;
+    pdl_wait();
     float2 v[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
@@ -1438,6 +1452,7 @@ __global__ void __launch_bounds__(rrow_threads(M)) k_fft_rows_bs(float2 *data, F
         v[m] = ok && j < n ? data[base + j] : make_float2(0.f, 0.f);
     }
     reg_bluestein<M, rrow_nb(M), false, S>(v, sm, b, l, p);
+    pdl_trigger();
     if (ok) {
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
@@ -1457,6 +1472,7 @@ __global__ void __launch_bounds__(rcol_threads(M)) k_fft_cols_bs(float2 *data, F
     const int b = threadIdx.x % NB, l = threadIdx.x / NB;
     const int x = blockIdx.x * cpc + b;
     const bool ok = b < cpc && x < W;
+    pdl_wait();
     float2 v[8];
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
@@ -1464,6 +1480,7 @@ __global__ void __launch_bounds__(rcol_threads(M)) k_fft_cols_bs(float2 *data, F
         v[m] = ok && j < n ? data[(size_t)j * W + x] : make_float2(0.f, 0.f);
     }
     reg_bluestein<M, NB, true, S>(v, sm, b, l, p);
+    pdl_trigger();
     if (ok) {
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
@@ -1808,6 +1825,7 @@ k_fft_rows_bs16(float2 *data, FftPlanDev p, int H, int rpc)
     const bool ok = b < rpc && y < H;
     const size_t base = (size_t)y * n;
     const LdTw16<M> rtw{p.tw, l};
+    pdl_wait();
     float2 v[16];
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
@@ -1815,6 +1833,7 @@ k_fft_rows_bs16(float2 *data, FftPlanDev p, int H, int rpc)
         v[m] = ok && j < n ? data[base + j] : make_float2(0.f, 0.f);
     }
     reg16_bluestein<M, RowSwz16<M>, S>(v, sm, b, l, rtw, n, p.chirp, S < 0 ? p.bspec_f : p.bspec_b);
+    pdl_trigger();
     if (ok) {
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
@@ -1830,6 +1849,7 @@ k_fft_cols_bs16(float2 *data, FftPlanDev p, int W, int cpc)
 {
     constexpr int NB = bs16_col_nb(M), MODE = S < 0 ? 2 : 3;
     const int b = threadIdx.x % NB, l = threadIdx.x / NB;
+    pdl_wait();
     float2 v[16];
     col_bs16_load<M, MODE>(v, data, nullptr, W, p.n, blockIdx.x * cpc, b, l);
     col_bs16_run<M, MODE>(v, data, W, p.n, blockIdx.x * cpc, p.chirp, p.bspec_f, p.bspec_b, LdTw16<M>{p.tw, l}, true, b,

@@ -432,13 +432,14 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_fft_rows_mx(float2 *data, 
     const int W = p.n, oa = 0, ob = mx_row_pad(rpc * W), ot = 2 * ob + rpc * W;
     const int y0 = blockIdx.x * rpc, nr = min(rpc, H - y0), n = nr * W;
     float2 *const X = data + (size_t)y0 * W;
+    for (int i = threadIdx.x; i < W; i += T) cp_async8(sm + ot + i, p.tw + i);
+    pdl_wait();
     float2 xv[V];
 #pragma unroll
     for (int m = 0; m < V; ++m) {
         const int i = threadIdx.x + m * T;
         if (i < n) xv[m] = X[i];
     }
-    for (int i = threadIdx.x; i < W; i += T) cp_async8(sm + ot + i, p.tw + i);
 #pragma unroll
     for (int m = 0; m < V; ++m) {
         const int i = threadIdx.x + m * T;
@@ -447,6 +448,7 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_fft_rows_mx(float2 *data, 
     cp_async_wait();
     __syncthreads();
     const int r = mx_fft<false, T>(oa, ob, ot, p, nr, S > 0);
+    pdl_trigger();
 #pragma unroll
     for (int m = 0; m < V; ++m) {
         const int i = threadIdx.x + m * T;
@@ -560,6 +562,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_fft_cols_mx(float2 *dat
     float2 *const sm = reinterpret_cast<float2 *>(smem4);
     constexpr int MODE = S < 0 ? 2 : 3;
     const int H = p.n, x0 = blockIdx.x * kMxColW;
+    pdl_wait();
     mx_col_request<MODE, T>(data, nullptr, W, H, x0);
     for (int i = threadIdx.x; i < H; i += T) cp_async8(sm + 2 * mx_col_pad(H) + i, p.tw + i);
     cp_async_wait();
