@@ -78,6 +78,8 @@ struct alignas(64) JobDev {
     double *err_part;       // [2 * n_row_tiles]  (sum mask*|g'|, sum mask)
     float *errors;          // [n_cycles] error after each cycle (mode 1: [n_err] per iteration)
     int n_err;              // mode 1: length of errors
+    int defer_err;          // mode 1: one more block of the column pass forms the error
+    int n_err_tiles;        // mode 1: tiles of the row pass (entries of err_part)
     JobState *st;
     int rpc;                // rows per row-pass CTA
     int cpc;                // columns per column-pass CTA

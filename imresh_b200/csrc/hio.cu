@@ -35,7 +35,7 @@
 namespace imr {
 
 constexpr int kHioChunk = 16;
-constexpr int kRandPowTable = 24;   // B^(2^j), j < 24: up to 2^24 chunks
+constexpr int kRandPowTable = 27;   // B^(2^j), j < 27: up to 2^27 chunks
 constexpr int kHioMaxErrors = 1 << 16;
 
 #define HCK(call)                                 \
@@ -187,9 +187,9 @@ static int hio_launch_iteration(imr_hio_plan *P, cudaStream_t s)
                     : P->p_rows     ? launch_pass(dep, rk.p_hio_fix, P->g_row, rk.threads, rk.p_smem, s, dj, Lrow)
                                     : launch_pass(dep, rk.hio_fix, J.n_row_tiles, rk.threads, P->smem_row, s, dj, Lrow);
     if (e == cudaSuccess)
-        e = P->n_col_narrow ? launch_pass(dep, ck.n_col, P->n_col_narrow, ck.n_threads, ck.n_smem, s, dj, Lcol)
+        e = P->n_col_narrow ? launch_pass(dep, ck.n_col, P->n_col_narrow + J.defer_err, ck.n_threads, ck.n_smem, s, dj, Lcol)
             : P->p_cols     ? launch_pass(dep, ck.p_col, P->g_col, ck.p_threads, ck.p_smem, s, dj, Lcol)
-                            : launch_pass(dep, ck.col, J.n_col_tiles, ck.threads, P->smem_col, s, dj, Lcol);
+                            : launch_pass(dep, ck.col, J.n_col_tiles + J.defer_err, ck.threads, P->smem_col, s, dj, Lcol);
     if (e != cudaSuccess) {
         set_error("kernel launch", e);
         return IMR_ERR_CUDA;
@@ -280,6 +280,8 @@ int imr_hio_plan_create(imr_hio_plan **out, unsigned W, unsigned H, unsigned nCy
     }
     narrow_tiles(P->rk, P->ck, P->p_cols, P->W, P->H, &P->n_row_narrow, &P->n_col_narrow);
     P->dependent = passes_dependent(J, S, P->rk, P->ck, true, n_split, P->n_row_narrow > 0, P->n_col_narrow > 0);
+    J.defer_err = P->n_col_narrow || (!P->p_cols && P->ck.checks) ? 1 : 0;
+    J.n_err_tiles = P->n_row_narrow ? P->n_row_narrow : J.n_row_tiles;
     const WorkList lists[4] = {{nullptr, J.n_row_tiles, 0}, {nullptr, J.n_col_tiles, n_split},
                                {nullptr, P->n_row_narrow, 0}, {nullptr, P->n_col_narrow, 0}};
     e = cudaMemcpy(P->Lrow, lists, sizeof(lists), cudaMemcpyHostToDevice);

@@ -118,8 +118,12 @@ ColKernels col_set()
         add_shapes<N>(k);
         return k;
     } else if constexpr (N < 0 && -N >= 256)   // Bluestein lengths, 16 values per thread
-        return ColKernels{k_col_bs16<-N, 0>, k_col_bs16<-N, 1>, k_fft_cols_bs16<-1, -N>, k_fft_cols_bs16<+1, -N>,
-                          bs16_col_nb(-N), bs16_col_threads(-N), bs16_col_smem(-N), nullptr, 0, 0, 0, 0, -N, 0};
+    {
+        ColKernels k{k_col_bs16<-N, 0>, k_col_bs16<-N, 1>, k_fft_cols_bs16<-1, -N>, k_fft_cols_bs16<+1, -N>,
+                     bs16_col_nb(-N), bs16_col_threads(-N), bs16_col_smem(-N), nullptr, 0, 0, 0, 0, -N, 0};
+        k.checks = 1;
+        return k;
+    }
     else if constexpr (N < 0 && -N >= 8)   // Bluestein lengths: register chirp-z transforms
         return ColKernels{k_col_bs<-N>, k_col_init_bs<-N>, k_fft_cols_bs<-1, -N>, k_fft_cols_bs<+1, -N>,
                           rcol_nb(-N), rcol_threads(-N), rcol_smem(-N), nullptr, 0, 0, 0, 0, -N, 0};

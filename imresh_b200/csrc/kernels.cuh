@@ -146,24 +146,15 @@ __device__ __forceinline__ void block_sum2(double &a, double &b, double *scratch
 // forms E_k = sqrt(sum)/count (calculateHioError, cpp:67-103, summed in double
 // in a fixed order), applies the stop tests E_k < target (cpp:251-254) and
 // k == nCycles (cpp:255-256), and moves the job to iteration k + 1.
+// Where the plan's column pass can take it (JobDev::defer_err), one more block of
+// that pass forms E_k beside the others (hio_check_block): the last tile's fence,
+// atomic and sum were a serial 3 us at the end of every row pass.  The column
+// pass of the iteration that stops then still runs; nothing reads its X.
 template <int T>
-__device__ __forceinline__ void hio_tile_done(const JobDev &J, int tile, double tot, double cnt, int n_tiles)
+__device__ __forceinline__ void hio_form_error(const JobDev &J, int n_tiles, double *red)
 {
-    __shared__ double red[2 * (T / 32 > 1 ? T / 32 : 1)];
-    __shared__ int s_last;
     JobState *st = J.st;
-    block_sum2<T>(tot, cnt, red);
-    if (threadIdx.x == 0) {
-        J.err_part[2 * tile] = tot;
-        J.err_part[2 * tile + 1] = cnt;
-        __threadfence();
-        s_last = atomicAdd(&st->counter, 1u) == (unsigned)n_tiles - 1u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    tot = 0.0;
-    cnt = 0.0;
+    double tot = 0.0, cnt = 0.0;
     const volatile double *ep = J.err_part;
     for (int t = threadIdx.x; t < n_tiles; t += T) {
         tot += ep[2 * t];
@@ -186,14 +177,47 @@ __device__ __forceinline__ void hio_tile_done(const JobDev &J, int tile, double 
         __threadfence();
     }
 }
+template <int T>
+__device__ __forceinline__ void hio_tile_done(const JobDev &J, int tile, double tot, double cnt, int n_tiles)
+{
+    __shared__ double red[2 * (T / 32 > 1 ? T / 32 : 1)];
+    __shared__ int s_last;
+    JobState *st = J.st;
+    block_sum2<T>(tot, cnt, red);
+    if (threadIdx.x == 0) {
+        J.err_part[2 * tile] = tot;
+        J.err_part[2 * tile + 1] = cnt;
+    }
+    if (J.defer_err) return;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&st->counter, 1u) == (unsigned)n_tiles - 1u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    hio_form_error<T>(J, n_tiles, red);
+}
+// The block after a column pass's last item: forms the error of the row pass
+// ahead of a plan (one job) whose row passes defer it.  Called by all T threads.
+template <int T>
+__device__ __forceinline__ void hio_check_block(const JobDev *jobs, const WorkList &list)
+{
+    __shared__ double red[2 * (T / 32 > 1 ? T / 32 : 1)];
+    if (list.items || (int)blockIdx.x != list.n || !jobs[0].defer_err) return;
+    pdl_wait();
+    if (jobs[0].st->stop == 0) hio_form_error<T>(jobs[0], jobs[0].n_err_tiles, red);
+}
 
 // Per-element part of the fixed-support HIO row pass: error terms of g' and
 // out = Re(g') when this iteration is tested (or is the last).
-__device__ __forceinline__ void hio_track(float *out, size_t idx, float2 gp1, uint8_t m, double &tot, double &cnt)
+__device__ __forceinline__ void hio_track(float *out, size_t idx, float2 gp1, uint8_t m, double &tot, unsigned &cnt)
 {
     if (m) {
-        tot += (double)m * (double)cnorm_ref(gp1);
-        cnt += (double)m;
+        // (m |z| is exact in double, so the fused sum rounds as the separate one)
+        const double v = (double)cnorm_ref(gp1);
+        tot = m == 1 ? tot + v : fma((double)m, v, tot);
+        cnt += m;
     }
     out[idx] = gp1.x;
 }
@@ -445,7 +469,8 @@ __device__ __forceinline__ void b_row_hio(const JobDev *jobs, const WorkItem wi)
     const bool init_gprev = FIX ? k == 0 : FIRST && st->hio_cycle == 0;
     const bool fin = FIX && k >= J.n_cycles;
     const bool track = FIX && (J.target > 0.f || fin);
-    double tot = 0.0, cnt = 0.0;
+    double tot = 0.0;
+    unsigned cnt = 0u;
     for (int i = threadIdx.x; i < n; i += T) {
         const size_t idx = base + i;
         const float2 gp1 = sm[i];   // g'
@@ -774,7 +799,10 @@ static __global__ void k_complex_norm(const float2 *src, float *dst, long n)
 // composed from the table pow[j] = B^(2^j); then it runs the recurrence.
 // Element k of X becomes ((float)rand_k / RAND_MAX, 0) (cpp:163-167).
 constexpr int kRandLag = 31;
-constexpr int kRandChunk = 31 * 32;
+// Numbers of a chunk: few, since a chunk is one thread's serial recurrence and the
+// jump to its start costs only two to three more matrix products: 992 numbers took
+// 117 us for 512 x 384 on 198 threads, 124 take 35.
+constexpr int kRandChunk = 31 * 4;
 constexpr int kRandThreads = 128;
 struct RandBase {
     uint32_t s[kRandLag];
@@ -814,7 +842,7 @@ static __global__ void __launch_bounds__(kRandThreads) k_rand_field(float2 *X, l
             const uint32_t r = s[q] + s[(q + kRandLag - 3) % kRandLag];   // r[i-31] + r[i-3]
             s[q] = r;
             const long k = k0 + (long)o * kRandLag + q;
-            if (k < kend) X[k] = make_float2(__fdiv_rn((float)(int)(r >> 1), 2147483648.0f), 0.f);
+            if (k < kend) X[k] = make_float2(__fmul_rn((float)(int)(r >> 1), 0x1p-31f), 0.f);   // / 2^31, exact
         }
     }
 }
@@ -1028,7 +1056,8 @@ __device__ __forceinline__ void b_row_hio_r(const JobDev *jobs, const WorkItem w
     const bool init_gprev = FIX ? k == 0 : FIRST && st->hio_cycle == 0;
     const bool fin = FIX && k >= J.n_cycles;
     const bool track = FIX && (J.target > 0.f || fin);
-    double tot = 0.0, cnt = 0.0;
+    double tot = 0.0;
+    unsigned cnt = 0u;
     if (ok) {
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
@@ -1247,7 +1276,8 @@ __device__ __forceinline__ void b_row_hio_bs(const JobDev *jobs, const WorkItem 
     const bool init_gprev = FIX ? k == 0 : FIRST && st->hio_cycle == 0;
     const bool fin = FIX && k >= J.n_cycles;
     const bool track = FIX && (J.target > 0.f || fin);
-    double tot = 0.0, cnt = 0.0;
+    double tot = 0.0;
+    unsigned cnt = 0u;
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
         const int j = l + m * Q;
@@ -1615,7 +1645,8 @@ k_row_hio_bs16(const JobDev *jobs, const WorkList *L)
     cp_async_wait();   // each thread reads back what it copied
     float2 *const G = J.G + base;
     const float beta = J.beta;
-    double tot = 0.0, cnt = 0.0;
+    double tot = 0.0;
+    unsigned cnt = 0u;
 #pragma unroll
     for (int m = 0; m < H8; ++m) {
         const int j = l + m * Q;
@@ -1794,7 +1825,10 @@ k_col_bs16(const JobDev *jobs, const WorkList *L)
 {
     constexpr int NB = bs16_col_nb(M);
     const WorkList list = list_and_job0(jobs, L);
-    if ((int)blockIdx.x >= list.n) return;
+    if ((int)blockIdx.x >= list.n) {
+        if (MODE == 0) hio_check_block<bs16_col_threads(M)>(jobs, list);
+        return;
+    }
     const LdTw16<M> rtw{jobs[list.items ? list.items[blockIdx.x].job : 0].pcol.tw, (int)threadIdx.x / NB};
     const WorkItem wi = list.items ? list.items[blockIdx.x] : WorkItem{0, (int)blockIdx.x};
     const JobDev &J = jobs[wi.job];
@@ -1889,9 +1923,12 @@ __host__ __device__ constexpr int prow_smem() { return 128 + 2 * prow_stage_byte
 // and two for the first pass of a cycle at powers of two (150 registers free,
 // 0-28 B of spills at 128; 2048^2: 3.22 -> 3.05 ms for 24 cycles x 1 HIO).
 // Other variants keep their registers.
+// The fixed-support pass is held to two at all lengths up to 2048 (139 registers
+// free, one CTA per SM: 2048^2 108 -> 84 us per iteration).
 __host__ __device__ constexpr int prow_min_blocks(bool FIRST, bool FIX, int N)
 {
-    return !FIRST && !FIX && is_pow2(N) && N <= 2048 ? 3 : (!FIX && (N % 3 == 0 ? !FIRST : is_pow2(N) && N <= 2048) ? 2 : 1);
+    if (FIX) return N <= 2048 ? 2 : 1;
+    return !FIRST && is_pow2(N) && N <= 2048 ? 3 : ((N % 3 == 0 ? !FIRST : is_pow2(N) && N <= 2048) ? 2 : 1);
 }
 
 __device__ __forceinline__ bool job_live(const JobDev *jobs, const WorkList *L, int item)
@@ -2024,7 +2061,8 @@ __global__ void __launch_bounds__(rrow_threads(N), prow_min_blocks(FIRST, FIX, N
         if (pdl_length(N) && s_next[s] >= n_items) pdl_trigger();
         const bool init_gprev = FIX ? kit == 0 : first_cycle;
         const bool track = tested && ok;
-        double tot = 0.0, cnt = 0.0;
+        double tot = 0.0;
+        unsigned cnt = 0u;
 #pragma unroll
         for (int m = 0; m < V; ++m) {
             const int e = b * N + l + m * Q;
@@ -2614,7 +2652,8 @@ __global__ void __launch_bounds__(row_n_threads(N)) k_row_hio_n(const JobDev *jo
     const bool track = FIX && ok && (J.target > 0.f || fin);
     reg_fft_1buf<N, RowSwz<N, NB>, +1>(v, sm, b, l, rtw);
     pdl_trigger();
-    double tot = 0.0, cnt = 0.0;
+    double tot = 0.0;
+    unsigned cnt = 0u;
 #pragma unroll
     for (int m = 0; m < V; ++m) {
         const float2 gp1 = v[m];
@@ -2649,7 +2688,10 @@ __global__ void __launch_bounds__(col_n_threads(N)) k_col_n(const JobDev *jobs, 
     float2 *const sm = reinterpret_cast<float2 *>(smem4);
     constexpr int NB = kColN, V = col_n_v(N), Q = N / V;
     const WorkList list = list_and_job0(jobs, L);
-    if ((int)blockIdx.x >= list.n) return;
+    if ((int)blockIdx.x >= list.n) {
+        hio_check_block<col_n_threads(N)>(jobs, list);
+        return;
+    }
     const int b = threadIdx.x % NB, l = threadIdx.x / NB;
     const WorkItem wi = list.items ? list.items[blockIdx.x] : WorkItem{0, (int)blockIdx.x};
     const JobDev &J = jobs[wi.job];

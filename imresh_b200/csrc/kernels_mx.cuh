@@ -267,7 +267,8 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_hio_mx(const JobDev *j
         __syncthreads();
         if (stop) continue;
         int r = oa;
-        double tot = 0.0, cnt = 0.0;
+        double tot = 0.0;
+        unsigned cnt = 0u;
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
             r = mx_fft<false, T>(r, oa + ob - r, ot, sp, nr, h == 0);
@@ -527,6 +528,10 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_col_mx(const JobDev *jo
     float2 *const sm = reinterpret_cast<float2 *>(smem4);
     __shared__ FftPlanDev sp;
     const WorkList l = list_and_job0(jobs, L);
+    if (MODE == 0 && (int)blockIdx.x >= l.n) {
+        hio_check_block<T>(jobs, l);
+        return;
+    }
     int job = -1;
     for (int it = blockIdx.x; it < l.n; it += gridDim.x) {
         const WorkItem wi = l.items ? l.items[it] : WorkItem{0, it};

@@ -15,8 +15,10 @@ RowKernels row_set_mx(int n)
 template <int T>
 static ColKernels col_set_mx_t(int n)
 {
-    return ColKernels{k_col_mx<0, T>, k_col_mx<1, T>, k_fft_cols_mx<-1, T>, k_fft_cols_mx<+1, T>, kMxColW, T,
-                      mx_col_smem(n), nullptr, 0, 0, 0, 0, 0, 0};
+    ColKernels k{k_col_mx<0, T>, k_col_mx<1, T>, k_fft_cols_mx<-1, T>, k_fft_cols_mx<+1, T>, kMxColW, T,
+                 mx_col_smem(n), nullptr, 0, 0, 0, 0, 0, 0};
+    k.checks = 1;
+    return k;
 }
 ColKernels col_set_mx(int n)
 {
