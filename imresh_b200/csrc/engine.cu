@@ -1048,7 +1048,6 @@ int imr_plan_copy_state(imr_plan *P, int what, void *h_dst, void *stream)
 // plain record inside a capture only orders streams.
 static cudaError_t profile_replay(imr_plan *P, int iters, bool split, cudaStream_t s, std::vector<cudaEvent_t> &ev)
 {
-    const JobDev &J = P->hj;
     cudaStream_t cs = nullptr;
     cudaError_t e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
     if (e != cudaSuccess) return e;
