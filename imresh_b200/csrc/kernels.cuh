@@ -209,6 +209,14 @@ __device__ __forceinline__ void hio_check_block(const JobDev *jobs, const WorkLi
     if (jobs[0].st->stop == 0) hio_form_error<T>(jobs[0], jobs[0].n_err_tiles, red);
 }
 
+// Whether a column block skips its tile.  In a fixed-support pass the check block
+// may set the flag meanwhile and threads may read different values: the block
+// decides as one (either way: nothing reads X then).
+__device__ __forceinline__ bool col_stopped(bool shrink_wrap, int stop)
+{
+    return shrink_wrap ? stop != 0 : __syncthreads_or(stop) != 0;
+}
+
 // Per-element part of the fixed-support HIO row pass: error terms of g' and
 // out = Re(g') when this iteration is tested (or is the last).
 __device__ __forceinline__ void hio_track(float *out, size_t idx, float2 gp1, uint8_t m, double &tot, unsigned &cnt)
@@ -1842,7 +1850,7 @@ k_col_bs16(const JobDev *jobs, const WorkList *L)
     const int b = threadIdx.x % NB, l = threadIdx.x / NB;
     pdl_wait();
     col_bs16_load<M, MODE>(v, X, Mod, W, H, x0, b, l);
-    if (MODE == 0 && st->stop) return;
+    if (MODE == 0 && col_stopped(guard, st->stop)) return;
     col_bs16_run<M, MODE>(v, X, W, H, x0, chirp, sf, sb, LdTw16<M>{J.pcol.tw, l}, guard, b, l);
 }
 
@@ -2710,7 +2718,7 @@ __global__ void __launch_bounds__(col_n_threads(N)) k_col_n(const JobDev *jobs, 
         float2 v[V];
 #pragma unroll
         for (int m = 0; m < V; ++m) v[m] = ok ? X[m * step] : make_float2(0.f, 0.f);
-        if (st->stop) return;
+        if (col_stopped(guard, st->stop)) return;
         forward(v);
         pdl_trigger();
 #pragma unroll

@@ -548,12 +548,11 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_col_mx(const JobDev *jo
         mx_col_request<MODE, T>(X, M, W, H, x0);
         if (other)
             for (int i = threadIdx.x; i < H; i += T) cp_async8(sm + 2 * mx_col_pad(H) + i, gtw + i);
-        const int stop = MODE == 0 ? st->stop : 0;
+        const int stop = MODE == 0 ? st->stop : 0;   // (the check block may be setting it: decided as one)
         if (other) mx_store_plan(&sp, word);
         job = wi.job;
         cp_async_wait();
-        __syncthreads();
-        if (stop) continue;
+        if (__syncthreads_or(stop)) continue;
         mx_col_run<MODE, T>(X, W, H, x0, sp, guard, it + (int)gridDim.x >= l.n);
         __syncthreads();
     }
