@@ -1850,7 +1850,8 @@ k_col_bs16(const JobDev *jobs, const WorkList *L)
     const int b = threadIdx.x % NB, l = threadIdx.x / NB;
     pdl_wait();
     col_bs16_load<M, MODE>(v, X, Mod, W, H, x0, b, l);
-    if (MODE == 0 && col_stopped(guard, st->stop)) return;
+    // (see col_stopped; always by the vote: the two ways apart cost 12 bytes of spills, 1021 x 733 8.46 -> 8.70 ms)
+    if (MODE == 0 && col_stopped(false, st->stop)) return;
     col_bs16_run<M, MODE>(v, X, W, H, x0, chirp, sf, sb, LdTw16<M>{J.pcol.tw, l}, guard, b, l);
 }
 
