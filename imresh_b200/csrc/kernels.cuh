@@ -317,7 +317,8 @@ __device__ __forceinline__ float vblur_tile(const float *src, float *dst, int W,
     const int x = x0 + tx;
     // all of a thread's tile rows are requested before any is stored, so the
     // loads' latencies overlap (rows_in <= TY + 62 for K <= 63 taps); in
-    // 16-byte loads where rows allow it (a quarter of the address arithmetic)
+    // 16-byte loads where rows allow it (a quarter of the address arithmetic).
+    // Ordinary loads: the pass that writes src may still run when this one starts.
     constexpr int RS = kVbThreads / kVbTileX;
     if (W % 4 == 0 && ((uintptr_t)src & 15) == 0) {
         constexpr int RS4 = 4 * RS, NLD = (TY + 62 + RS4 - 1) / RS4;
@@ -328,7 +329,7 @@ __device__ __forceinline__ float vblur_tile(const float *src, float *dst, int W,
         for (int i = 0; i < NLD; ++i) {
             const int r = r0 + i * RS4;
             const int ys = min(max(y0 - N + r, 0), H - 1);
-            if (r < rows_in && in) ld[i] = __ldg(reinterpret_cast<const float4 *>(src + (size_t)ys * W + x0) + q);
+            if (r < rows_in && in) ld[i] = reinterpret_cast<const float4 *>(src + (size_t)ys * W + x0)[q];
         }
 #pragma unroll
         for (int i = 0; i < NLD; ++i) {
@@ -342,7 +343,7 @@ __device__ __forceinline__ float vblur_tile(const float *src, float *dst, int W,
         for (int i = 0; i < NLD; ++i) {
             const int r = ty + i * RS;
             const int ys = min(max(y0 - N + r, 0), H - 1);
-            ld[i] = r < rows_in && x < W ? __ldg(src + (size_t)ys * W + x) : 0.f;
+            ld[i] = r < rows_in && x < W ? src[(size_t)ys * W + x] : 0.f;
         }
 #pragma unroll
         for (int i = 0; i < NLD; ++i) {

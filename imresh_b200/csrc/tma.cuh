@@ -127,7 +127,10 @@ __device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_
 // ended: once all of that pass's CTAs have called pdl_trigger or exited.  What
 // it does before pdl_wait may touch only what no pass writes (work lists, job
 // descriptions, tables); pdl_wait returns when the passes ahead are complete
-// and their writes visible.  A pass triggers half-way through its last item,
+// and their writes visible to ordinary loads.  What a pass writes is never read
+// with __ldg or through a const __restrict__ pointer: a non-coherent load wants
+// memory that stays unwritten for the whole life of the kernel, and that life now
+// overlaps the writing pass's.  A pass triggers half-way through its last item,
 // after its own pdl_wait, so no pass runs beside the one before the last.  Both
 // are no-ops in a launch without the attribute.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
