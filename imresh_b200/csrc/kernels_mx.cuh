@@ -363,7 +363,8 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_finish_mx(const JobDev
             const int i = threadIdx.x + m * T;
             mk[m] = i < n ? mask[i] : 0;
         }
-        const int stop = st->stop, c = st->cycle;
+        // (a job that ended by its count has gone one cycle past the tables)
+        const int stop = st->stop, c = min(st->cycle, J.n_cycles);
         const int K = J.ntaps[c];
         if (threadIdx.x < kTapStride) wsm[threadIdx.x] = J.weights[(size_t)c * kTapStride + threadIdx.x];
         if (other) mx_store_plan(&sp, word);

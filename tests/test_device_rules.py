@@ -26,3 +26,32 @@ READ_ONLY = {"tw", "gtw", "chirp", "p.chirp", "spec", "mt", "mt_base", "J.M"}
 def test_non_coherent_loads_only_of_what_no_pass_writes(name):
     args = re.findall(r"__ldg\(\s*([^)]*)", _code(name))
     assert [a for a in args if re.split(r"[\s+]", a)[0] not in READ_ONLY] == []
+
+
+def _bodies(name):
+    """(head, body) of each function: the text before its braces, and what they hold."""
+    s = _code(name)
+    for m in re.finditer(r"\)\s*\{", s):
+        start = s.rfind("\n\n", 0, m.start()) + 1
+        depth, i = 1, m.end()
+        while depth and i < len(s):
+            depth += {"{": 1, "}": -1}.get(s[i], 0)
+            i += 1
+        yield s[start:m.start()], s[m.end():i - 1]
+
+
+@pytest.mark.parametrize("name", HEADERS)
+def test_tap_tables_are_read_within_their_cycles(name):
+    """The tables hold n_cycles + 1 cycles; a job that ended by its count stands at
+    cycle n_cycles + 1.  A pass reads them after its stop test (or walks live jobs
+    only), or at a cycle held to the last one."""
+    found = 0
+    for head, body in _bodies(name):
+        if "__device__" not in head and "__global__" not in head:
+            continue
+        at = body.find("J.ntaps[")
+        if at < 0:
+            continue
+        found += 1
+        assert re.search(r"if \((st->)?stop\)|next_live|c = min\(st->cycle, J\.n_cycles\)", body[:at]), head
+    assert found or name not in ("kernels.cuh", "kernels_mx.cuh")
