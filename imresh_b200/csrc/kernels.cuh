@@ -1638,7 +1638,10 @@ k_row_hio_bs16(const JobDev *jobs, const WorkList *L)
     const bool init_gprev = k == 0;
     const bool fin = FIX && k >= J.n_cycles;
     const bool track = FIX && (J.target > 0.f || fin);
-    if (stop) return;
+    if (stop) {
+        cp_async_wait();   // a block does not end with copies into its shared memory in flight
+        return;
+    }
     reg16_bluestein<M, RowSwz16<M>, +1>(v, sm, b, l, LdTw16<M>{J.prow.tw, l}, W, J.prow.chirp, J.prow.bspec_b);
     if (FIRST) {
         const float *const vb = J.vb + base;
@@ -1852,7 +1855,10 @@ k_col_bs16(const JobDev *jobs, const WorkList *L)
     pdl_wait();
     col_bs16_load<M, MODE>(v, X, Mod, W, H, x0, b, l);
     // (see col_stopped; always by the vote: the two ways apart cost 12 bytes of spills, 1021 x 733 8.46 -> 8.70 ms)
-    if (MODE == 0 && col_stopped(false, st->stop)) return;
+    if (MODE == 0 && col_stopped(false, st->stop)) {
+        cp_async_wait();   // (see k_row_hio_bs16)
+        return;
+    }
     col_bs16_run<M, MODE>(v, X, W, H, x0, chirp, sf, sb, LdTw16<M>{J.pcol.tw, l}, guard, b, l);
 }
 

@@ -55,3 +55,20 @@ def test_tap_tables_are_read_within_their_cycles(name):
         found += 1
         assert re.search(r"if \((st->)?stop\)|next_live|c = min\(st->cycle, J\.n_cycles\)", body[:at]), head
     assert found or name not in ("kernels.cuh", "kernels_mx.cuh")
+
+
+@pytest.mark.parametrize("name", HEADERS)
+def test_no_block_leaves_with_copies_in_flight(name):
+    """After a kernel has requested asynchronous copies into shared memory, a
+    return or a skipped item comes after a wait for them."""
+    request = re.compile(r"cp_async[48]\(|col_bs16_load<|mx_col_request<")
+    for head, body in _bodies(name):
+        if "__global__" not in head:
+            continue
+        m = request.search(body)
+        if not m:
+            continue
+        rest = body[m.end():]
+        leave = re.search(r"\b(return|continue)\b", rest)
+        if leave:
+            assert "cp_async_wait()" in rest[:leave.start()], head
