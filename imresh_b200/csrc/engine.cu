@@ -543,10 +543,14 @@ static int fft_launch(float2 *d, int W, int H, int sign, int axes, const FftPlan
     const int nrt = (H + rpc - 1) / rpc, nct = (W + cpc - 1) / cpc, ct = ck.f_nb ? ck.f_threads : ck.threads;
     const size_t sr = rk.smem ? (size_t)row_tile_smem(rk, W, rpc) : ((size_t)rpc * W + rk.bs_m) * 8;
     const size_t sc = ck.f_nb ? (size_t)ck.f_smem : ck.smem ? (size_t)ck.smem : ((size_t)H + ck.bs_m) * cpc * 8;
-    // the second transform starts while the first one drains: 1-2 us of a call at
-    // every size up to 2048 x 1024 (256^2 8.2 -> 7.1 us, 768^2 22.6 -> 19, 1000 x 800 21.3 ->
-    // 18.5), nothing beyond
-    const bool dep = axes == 3;
+    // the second transform may start while the first one drains (fft_rows_start_early)
+    const int every = 1 << 30;
+    auto rows_early = [&] {
+        return nrt <= 111 ||   // (asks for nothing where the count decides)
+               fft_rows_start_early(nct, persistent_grid((const void *)ck.fft_inv, ct, (int)sc, every), nrt,
+                                    persistent_grid((const void *)rk.fft_inv, rk.threads, (int)sr, every));
+    };
+    const bool dep = axes == 3 && (sign < 0 || rows_early());
     cudaError_t e = cudaSuccess;
     if (sign < 0) {
         if (axes & 1) e = launch_pass(false, rk.fft_fwd, nrt, rk.threads, sr, s, d, pr, H, rpc);

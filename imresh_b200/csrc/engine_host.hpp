@@ -4,6 +4,7 @@
 #include <vector>
 #include "imresh_b200.h"
 #include "engine.cuh"
+#include "rules.hpp"
 
 namespace imr {
 

@@ -1,0 +1,55 @@
+"""The dispatch rules on sizes (imresh_b200/csrc/rules.hpp), compiled on the CPU, at
+the shapes they were measured at; and results on both sides of each line."""
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import imresh_b200 as imr
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "imresh_b200", "csrc")
+
+
+@pytest.fixture(scope="module")
+def rule(tmp_path_factory):
+    def run(expr):
+        d = tmp_path_factory.mktemp("rules")
+        src, exe = os.path.join(d, "r.cpp"), os.path.join(d, "r")
+        with open(src, "w") as f:
+            f.write('#include <stdio.h>\n#include "rules.hpp"\nint main() { printf("%%ld", (long)(imr::%s)); }\n' % expr)
+        subprocess.run(["g++", "-std=c++17", "-I", CSRC, src, "-o", exe], check=True)
+        return int(subprocess.run([exe], check=True, capture_output=True, text=True).stdout)
+    return run
+
+
+def _check_fft(h, w, sign):
+    import torch
+    rng = np.random.default_rng(h * 4 + w)
+    x = (rng.standard_normal((h, w)) + 1j * rng.standard_normal((h, w))).astype(np.complex64)
+    d = torch.from_numpy(x.copy()).cuda()
+    imr.fft2d(d, w, h, sign)
+    xd = x.astype(np.complex128)
+    ref = np.fft.fft2(xd) if sign < 0 else np.fft.ifft2(xd) * x.size
+    assert np.linalg.norm(d.cpu().numpy() - ref) / np.linalg.norm(ref) < 1e-5   # the transforms' bar
+
+
+# inverse transforms as measured: column blocks, resident, row blocks, resident, start early
+@pytest.mark.parametrize("cols,cres,rows,rres,early", [
+    (96, 148, 256, 740, 0),      # 384 x 2048: 15.9 us, early 22.4
+    (256, 888, 192, 444, 0),     # 4096 x 192: 15.9, 18.9
+    (128, 148, 512, 888, 0),     # 512 x 2048: 13.4, 15.0
+    (32, 148, 128, 888, 0),      # 128 x 2048: 10.4, 10.7
+    (64, 888, 64, 592, 1),       # 256 x 256: 5.2, 4.9
+    (128, 592, 128, 888, 1),     # 512 x 512: 6.25, 5.9
+    (512, 444, 768, 444, 1),     # 4096 x 768: 44.2, 43.7
+    (192, 148, 700, 592, 1)])
+def test_rows_do_not_start_beside_few_column_blocks(rule, cols, cres, rows, rres, early):
+    assert rule("fft_rows_start_early(%d, %d, %d, %d)" % (cols, cres, rows, rres)) == early
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,w", [(2048, 384), (888, 64), (889, 64), (1184, 128), (1185, 128), (192, 4096), (148, 2048), (149, 2048)])
+@pytest.mark.parametrize("sign", [-1, 1])
+def test_transforms_on_both_sides_of_the_early_start(cuda, h, w, sign):
+    _check_fft(h, w, sign)
