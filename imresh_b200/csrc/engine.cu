@@ -475,6 +475,8 @@ int ensure_kernel_attributes()
         if (e == cudaSuccess) e = allow_smem(c.init);
         if (e == cudaSuccess) e = allow_smem(c.fft_fwd);
         if (e == cudaSuccess) e = allow_smem(c.fft_inv);
+        if (e == cudaSuccess && c.f_fwd) e = allow_smem(c.f_fwd);
+        if (e == cudaSuccess && c.f_inv) e = allow_smem(c.f_inv);
         if (e == cudaSuccess && r.p_hio) e = allow_smem(r.p_hio);
         if (e == cudaSuccess && r.p_hio_first) e = allow_smem(r.p_hio_first);
         if (e == cudaSuccess) e = allow_smem(r.hio_fix);
@@ -539,25 +541,28 @@ int build_weight_table(const imr_params &p, std::vector<float> &w, std::vector<i
 static int fft_launch(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr, const FftPlanDev &pc,
                       const RowKernels &rk, const ColKernels &ck, cudaStream_t s)
 {
-    const int rpc = rk.mx ? rows_per_tile(rk, W, H) : rk.nb, cpc = ck.f_nb ? ck.f_nb : ck.nb;
-    const int nrt = (H + rpc - 1) / rpc, nct = (W + cpc - 1) / cpc, ct = ck.f_nb ? ck.f_threads : ck.threads;
+    const bool narrow = ck.f_fwd && fft_narrow_columns((W + ck.nb - 1) / ck.nb);
+    const int rpc = rk.mx ? rows_per_tile(rk, W, H) : rk.nb, cpc = narrow ? ck.f_nb : ck.nb;
+    const int nrt = (H + rpc - 1) / rpc, nct = (W + cpc - 1) / cpc, ct = narrow ? ck.f_threads : ck.threads;
     const size_t sr = rk.smem ? (size_t)row_tile_smem(rk, W, rpc) : ((size_t)rpc * W + rk.bs_m) * 8;
-    const size_t sc = ck.f_nb ? (size_t)ck.f_smem : ck.smem ? (size_t)ck.smem : ((size_t)H + ck.bs_m) * cpc * 8;
+    const size_t sc = narrow ? (size_t)ck.f_smem : ck.smem ? (size_t)ck.smem : ((size_t)H + ck.bs_m) * cpc * 8;
+    const auto rows = sign < 0 ? rk.fft_fwd : rk.fft_inv;
+    const auto cols = sign < 0 ? (narrow ? ck.f_fwd : ck.fft_fwd) : (narrow ? ck.f_inv : ck.fft_inv);
     // the second transform may start while the first one drains (fft_rows_start_early)
     const int every = 1 << 30;
     auto rows_early = [&] {
         return nrt <= 111 ||   // (asks for nothing where the count decides)
-               fft_rows_start_early(nct, persistent_grid((const void *)ck.fft_inv, ct, (int)sc, every), nrt,
-                                    persistent_grid((const void *)rk.fft_inv, rk.threads, (int)sr, every));
+               fft_rows_start_early(nct, persistent_grid((const void *)cols, ct, (int)sc, every), nrt,
+                                    persistent_grid((const void *)rows, rk.threads, (int)sr, every));
     };
     const bool dep = axes == 3 && (sign < 0 || rows_early());
     cudaError_t e = cudaSuccess;
     if (sign < 0) {
-        if (axes & 1) e = launch_pass(false, rk.fft_fwd, nrt, rk.threads, sr, s, d, pr, H, rpc);
-        if ((axes & 2) && e == cudaSuccess) e = launch_pass(dep, ck.fft_fwd, nct, ct, sc, s, d, pc, W, cpc);
+        if (axes & 1) e = launch_pass(false, rows, nrt, rk.threads, sr, s, d, pr, H, rpc);
+        if ((axes & 2) && e == cudaSuccess) e = launch_pass(dep, cols, nct, ct, sc, s, d, pc, W, cpc);
     } else {
-        if (axes & 2) e = launch_pass(false, ck.fft_inv, nct, ct, sc, s, d, pc, W, cpc);
-        if ((axes & 1) && e == cudaSuccess) e = launch_pass(dep, rk.fft_inv, nrt, rk.threads, sr, s, d, pr, H, rpc);
+        if (axes & 2) e = launch_pass(false, cols, nct, ct, sc, s, d, pc, W, cpc);
+        if ((axes & 1) && e == cudaSuccess) e = launch_pass(dep, rows, nrt, rk.threads, sr, s, d, pr, H, rpc);
     }
     if (e != cudaSuccess) {
         set_error("fft launch", e);

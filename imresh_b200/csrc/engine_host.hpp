@@ -103,7 +103,9 @@ struct ColKernels {
     void (*p_col_split)(const JobDev *, const WorkList *);   // p_col running WorkList::n_split
                                                               // tiles as half tiles (JobDev::tmXh), or null
     int checks;      // 1: `col` takes a block more for the deferred error of a fixed-support plan
-    int f_nb, f_threads, f_smem;   // launch shape of fft_fwd / fft_inv (0: nb, threads, smem)
+    void (*f_fwd)(float2 *, FftPlanDev, int, int);   // fft_fwd, fft_inv in narrow tiles, or null
+    void (*f_inv)(float2 *, FftPlanDev, int, int);
+    int f_nb, f_threads, f_smem;
     void (*n_col)(const JobDev *, const WorkList *);   // pass of small images (n_nb columns per one-item block), or null
     int n_nb, n_threads, n_smem;
 };

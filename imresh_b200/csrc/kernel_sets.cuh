@@ -24,10 +24,12 @@ static void add_shapes(RowKernels &k)
 template <int N>
 static void add_shapes(ColKernels &k)
 {
-    if constexpr (is_pow2(N)) {
-        k.f_nb = fcol_nb(N);
-        k.f_threads = fcol_threads(N);
-        k.f_smem = fcol_smem(N);
+    if constexpr (is_pow2(N) && fcol_narrow(N)) {
+        k.f_fwd = k_fft_cols_r<-1, N, kFcolN>;
+        k.f_inv = k_fft_cols_r<+1, N, kFcolN>;
+        k.f_nb = kFcolN;
+        k.f_threads = kFcolN * N / 8;
+        k.f_smem = reg_smem_bytes(N, kFcolN);
     }
     if constexpr (narrow_length(N)) {
         k.n_col = k_col_n<N>;
@@ -87,7 +89,7 @@ ColKernels col_set()
 {
     if constexpr (N >= 128 && N <= 4096 && is_pow2(N)) {   // 16 values per thread in the pipelined pass
         constexpr int T = pcol16_nbt(N);
-        ColKernels k{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
+        ColKernels k{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N, rcol_nb(N)>, k_fft_cols_r<+1, N, rcol_nb(N)>,
                      rcol_nb(N), rcol_threads(N), rcol_smem(N), k_col_p16<N, T, false>, pcol16_smem<N, T>(),
                      pcol_box_rows(N), 0, pcol16_threads(N, T), 0, T, 1};
         if constexpr (N >= 256) {   // split-precision tensor-core variants
@@ -103,13 +105,13 @@ ColKernels col_set()
         if constexpr (T >= 4) k.p_col_split = k_col_p16<N, T, true>;   // half tiles of >= 2 columns (16-byte TMA rows)
         return k;
     } else if constexpr (N >= 16 && is_pow2(N)) {
-        ColKernels k{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
+        ColKernels k{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N, rcol_nb(N)>, k_fft_cols_r<+1, N, rcol_nb(N)>,
                      rcol_nb(N), rcol_threads(N), rcol_smem(N), k_col_p<N>, pcol_smem<N>(),
                      pcol_box_rows(N), pcol_tma_m(N) ? 1 : 0, pcol_threads(N), 0, rcol_nb(N)};
         add_shapes<N>(k);
         return k;
     } else if constexpr (N >= 8 && is_pow2(N))
-        return ColKernels{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N>, k_fft_cols_r<+1, N>,
+        return ColKernels{k_col_r<N>, k_col_init_r<N>, k_fft_cols_r<-1, N, rcol_nb(N)>, k_fft_cols_r<+1, N, rcol_nb(N)>,
                           rcol_nb(N), rcol_threads(N), rcol_smem(N), nullptr, 0, 0, 0, 0, 0};
     else if constexpr (is_3pow2(N)) {
         ColKernels k{k_col<N>, k_col_init<N>, k_fft_cols<-1, N>, k_fft_cols<+1, N>, col_nb(N),

@@ -1190,17 +1190,16 @@ __global__ void __launch_bounds__(rrow_threads(N)) k_fft_rows_r(float2 *data, Ff
     }
 }
 
-// Columns of a tile: four (two at 4096): smaller blocks fill the SMs of a small
-// image (128 x 1024: 12.3 -> 8.5 us a transform; two columns at 2048^2: 59 us, four 51).
-__host__ __device__ constexpr int fcol_nb(int N) { return N <= 2048 ? 4 : 2; }
-__host__ __device__ constexpr int fcol_threads(int N) { return fcol_nb(N) * N / 8; }
-__host__ __device__ constexpr int fcol_smem(int N) { return reg_smem_bytes(N, fcol_nb(N)); }
-template <int S, int N>
-__global__ void __launch_bounds__(fcol_threads(N)) k_fft_cols_r(float2 *data, FftPlanDev p, int W, int cpc)
+// Columns of a narrow tile (fft_narrow_columns).  Columns of 64 are as fast in wide
+// ones (64 x 64: 3.8 us, narrow 4.0), and from 2048 on the wide tile is no wider.
+constexpr int kFcolN = 4;
+__host__ __device__ constexpr bool fcol_narrow(int N) { return N >= 128 && rcol_nb(N) > kFcolN; }
+template <int S, int N, int NB>
+__global__ void __launch_bounds__(NB * N / 8) k_fft_cols_r(float2 *data, FftPlanDev p, int W, int cpc)
 {
     extern __shared__ float4 smem4[];
     float2 *sm = reinterpret_cast<float2 *>(smem4);
-    constexpr int NB = fcol_nb(N), Q = N / 8;
+    constexpr int Q = N / 8;
     const int b = threadIdx.x % NB, l = threadIdx.x / NB;
     const int x = blockIdx.x * cpc + b;
     const bool ok = b < cpc && x < W;

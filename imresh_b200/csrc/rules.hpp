@@ -20,4 +20,12 @@ inline bool fft_rows_start_early(int cols, int cols_resident, int rows, int rows
     return rows <= 111 || cols >= 2 * kSms || rows > rows_resident || (rows <= kSms && cols_resident > kSms);
 }
 
+// Whether the columns of a plain transform run in narrow tiles (4 columns) instead
+// of the wide ones (`wide_tiles` of them; 16 columns up to H = 512, 8 at 1024):
+// where the wide tiles leave half of the SMs without one.  Whole transform, wide ->
+// narrow: 256 x 256 6.2 -> 5.2 us (16 wide tiles), 512 x 1024 10.5 -> 8.9 (64); beyond
+// that narrow tiles only make the strides shorter: 2048 x 512 13.0 -> 13.9 (128),
+// 2048 x 1024 23.8 -> 25.0 (256), 4096 x 64 7.7 -> 8.0.
+inline bool fft_narrow_columns(int wide_tiles) { return 2 * wide_tiles < kSms; }
+
 }  // namespace imr

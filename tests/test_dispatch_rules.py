@@ -53,3 +53,17 @@ def test_rows_do_not_start_beside_few_column_blocks(rule, cols, cres, rows, rres
 @pytest.mark.parametrize("sign", [-1, 1])
 def test_transforms_on_both_sides_of_the_early_start(cuda, h, w, sign):
     _check_fft(h, w, sign)
+
+
+# (W, H, wide tile of H, narrow): images with many wide tiles keep them
+@pytest.mark.parametrize("w,h,tile,narrow", [(256, 256, 16, 1), (512, 1024, 8, 1), (1168, 512, 16, 1), (1169, 512, 16, 0),
+                                             (1024, 1024, 8, 0), (2048, 512, 16, 0), (4096, 128, 16, 0)])
+def test_narrow_columns_where_wide_tiles_leave_sms_idle(rule, w, h, tile, narrow):
+    assert rule("fft_narrow_columns(%d)" % ((w + tile - 1) // tile)) == narrow
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,w", [(64, 33), (128, 3), (128, 1165), (128, 1169), (512, 1168), (512, 1171), (1024, 583), (1024, 585)])
+@pytest.mark.parametrize("sign", [-1, 1])
+def test_transforms_on_both_sides_of_the_narrow_columns(cuda, h, w, sign):
+    _check_fft(h, w, sign)
