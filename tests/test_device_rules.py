@@ -72,3 +72,15 @@ def test_no_block_leaves_with_copies_in_flight(name):
         leave = re.search(r"\b(return|continue)\b", rest)
         if leave:
             assert "cp_async_wait()" in rest[:leave.start()], head
+
+
+def test_pipelined_passes_trigger_by_their_length():
+    """The pipelined passes let the next pass start early only at lengths that gain."""
+    triggers = {}
+    for head, body in _bodies("kernels.cuh"):
+        name = re.search(r"\b(k_row_hio_p|k_row_finish_p|k_col_p|k_col_p16)\(const JobDev", head)
+        if name and "__global__" in head and name.group(1) not in triggers:
+            triggers[name.group(1)] = re.findall(r"if \(([^;]*)\) pdl_trigger\(\)", body)
+    assert set(triggers) == {"k_row_hio_p", "k_row_finish_p", "k_col_p", "k_col_p16"}
+    for name, conds in triggers.items():
+        assert conds and all(c.startswith("pdl_length(N) && ") for c in conds), name
