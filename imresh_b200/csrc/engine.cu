@@ -327,6 +327,7 @@ bool passes_dependent(const JobDev &J, const JobShape &S, const RowKernels &rk, 
                         : dependent_pass(J.n_col_tiles,
                                          persistent_grid((const void *)ck.col, ck.threads, (int)S.smem_col, every));
     };
+    if (!row_narrow && rk.p_hio && !pipelined_rows_dependent(J.W)) return false;
     return (row_narrow || row_ok()) && (col_narrow || col_ok());
 }
 

@@ -143,18 +143,6 @@ int scaled_grid(const void *kernel, int threads, int smem, int items, int grid_p
 // most g_max CTAs resident (its grid: min(g_max, n_tiles + n_split)): every
 // tile when their halves fit the resident CTAs, else none.
 int col_split(int n_tiles, int g_max);
-// Whether the passes of an iteration are launched dependently (launch_pass):
-// `tiles` work items on at most `resident` CTAs for each of the two passes.
-// It takes 1.1-1.6 us off an iteration (256^2 9.4 -> 8.0 us, 192^2 11.4 -> 10.3,
-// 1021 x 733 54.2 -> 51.5), but CTAs that start early go to the SMs that are idle
-// then: a pass of one wave that needs all SMs evenly gets several CTAs on some of
-// them (1024^2 20.3 -> 22.4, 1000 x 800 35.1 -> 40.5).  So a pass either leaves a
-// quarter of the SMs without work, or has more tiles than one wave takes; with
-// more than three waves the gap is too small a part to gain (2048^2: 2 % slower).
-inline bool dependent_pass(int tiles, int resident)
-{
-    return tiles <= 111 || (tiles > resident && tiles <= 3 * resident);
-}
 // 2D tensor map over a row-major [H][W] array of `elem`-byte elements with a
 // (box_w, box_h) box; returns false when the shape cannot be described.
 bool encode_tensor_map(CUtensorMap *map, const void *base, int W, int H, int elem, int box_w, int box_h);

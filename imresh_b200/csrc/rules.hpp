@@ -28,4 +28,22 @@ inline bool fft_rows_start_early(int cols, int cols_resident, int rows, int rows
 // 2048 x 1024 23.8 -> 25.0 (256), 4096 x 64 7.7 -> 8.0.
 inline bool fft_narrow_columns(int wide_tiles) { return 2 * wide_tiles < kSms; }
 
+// Whether the passes of an iteration are launched dependently (launch_pass):
+// `tiles` work items on at most `resident` CTAs for each of the two passes.
+// It takes 1.1-1.6 us off an iteration (256^2 9.4 -> 8.0 us, 192^2 11.4 -> 10.3,
+// 1021 x 733 54.2 -> 51.5), but CTAs that start early go to the SMs that are idle
+// then: a pass of one wave that needs all SMs evenly gets several CTAs on some of
+// them (1024^2 20.3 -> 22.4, 1000 x 800 35.1 -> 40.5).  So a pass either leaves a
+// quarter of the SMs without work, or has more tiles than one wave takes; with
+// more than three waves the gap is too small a part to gain (2048^2: 2 % slower).
+inline bool dependent_pass(int tiles, int resident)
+{
+    return tiles <= 111 || (tiles > resident && tiles <= 3 * resident);
+}
+// Pipelined rows of 2048 and more do not prepare before their wait nor release the
+// columns half-way, so an early start gives them nothing, and rows that sit beside
+// the columns' last tiles cost 2048 x 1024 38.1 -> 39.8 us (3072 x 512 39.5 and 39.9 the
+// other way).
+inline bool pipelined_rows_dependent(int W) { return W < 2048; }
+
 }  // namespace imr

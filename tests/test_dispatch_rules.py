@@ -67,3 +67,9 @@ def test_narrow_columns_where_wide_tiles_leave_sms_idle(rule, w, h, tile, narrow
 @pytest.mark.parametrize("sign", [-1, 1])
 def test_transforms_on_both_sides_of_the_narrow_columns(cuda, h, w, sign):
     _check_fft(h, w, sign)
+
+
+# an iteration of 2048 x 1024: 38.1 us, rows that start early 39.8
+@pytest.mark.parametrize("w,dependent", [(64, 1), (1536, 1), (2048, 0), (4096, 0)])
+def test_long_pipelined_rows_do_not_start_early(rule, w, dependent):
+    assert rule("pipelined_rows_dependent(%d)" % w) == dependent
