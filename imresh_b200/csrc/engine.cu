@@ -495,7 +495,9 @@ int ensure_kernel_attributes()
                 if (e == cudaSuccess && c.fft_tc[pr][d]) e = allow_smem(c.fft_tc[pr][d]);
         }
     }
-    if (e == cudaSuccess) e = allow_smem(k_hblur);
+    if (e == cudaSuccess) e = allow_smem(k_hblur<true>);
+    if (e == cudaSuccess) e = allow_smem(k_hblur<false>);
+    if (e == cudaSuccess) e = allow_smem(k_hblur_px);
     if (e != cudaSuccess) {
         set_error("cudaFuncSetAttribute", e);
         return IMR_ERR_CUDA;
@@ -1292,11 +1294,22 @@ int imr_gaussian_blur(float *d_data, float *d_tmp, unsigned W, unsigned H, doubl
     // both axes: rows into the scratch image, columns back from it
     float *const rows_out = axes == 3 ? d_tmp : d_data;
     if (axes & 1) {
-        const int chunks = hb_row_floats((int)W) / kHbOut;
-        const int nr = std::max(1, std::min(kRowThreads / chunks, (int)H / 296));
-        const int threads = std::min(kRowThreads, (nr * chunks + 31) / 32 * 32);
-        k_hblur<<<(H + nr - 1) / nr, threads, (size_t)nr * hb_row_floats((int)W) * 4, s>>>(d_data, rows_out, (int)W,
-                                                                                         (int)H, nr, t, K);
+        const bool vec = W % 4 == 0 && (((uintptr_t)d_data | (uintptr_t)rows_out) & 15) == 0;
+        if (hblur_rolling((int)W, (int)H, K, vec)) {
+            const int rs = hb_row_floats((int)W), chunks = rs / kHbOut, pw = (int)W / (vec ? 4 : 1);
+            const int nr = std::max(1, std::min(kRowThreads / chunks, (int)H / 296));
+            const int threads = std::max(nr == 1 ? 32 : vec ? 128 : kRowThreads,
+                                         std::min(kRowThreads, (nr * chunks + 31) / 32 * 32));
+            int lgx = 0;   // 2^lgx threads a row
+            while ((1 << lgx) < pw) ++lgx;
+            if ((1 << lgx) > threads) lgx = -1;
+            const size_t rows_bytes = (size_t)nr * rs * 4;
+            const bool staged = chunks > kRowThreads && rows_bytes + kHbStage * 4 + kTapStride * 4 <= (size_t)g_optin_smem;
+            (vec ? k_hblur<true> : k_hblur<false>)<<<(H + nr - 1) / nr, threads, rows_bytes + (staged ? kHbStage * 4 : 0),
+                                                     s>>>(d_data, rows_out, (int)W, (int)H, nr, lgx, staged, t, K);
+        } else {
+            k_hblur_px<<<H, kRowThreads, (size_t)W * 4, s>>>(d_data, rows_out, (int)W, t, K);
+        }
     }
     if (axes & 2) {
         const int tx = (int)((W + kVbTileX - 1) / kVbTileX), nt = tx * (int)((H + kVbTileY - 1) / kVbTileY);

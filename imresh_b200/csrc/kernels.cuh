@@ -691,81 +691,102 @@ struct Taps {
     float w[kTapStride];
 };
 
-// Rows src -> dst (which may be src): nr rows per CTA in shared memory, a thread
-// making kHbOut neighbouring outputs (tap_sums).  Element e of a row sits at
-// e ^ ((e >> 5) & 15): lanes 16 elements apart hit all banks.  The sums go back
-// to the row buffer so that the row leaves coalesced whatever its width.
+// Rows src -> dst (which may be src), one row per CTA, one output per thread and turn.
+static __global__ void __launch_bounds__(kRowThreads) k_hblur_px(const float *src, float *dst, int W, Taps w, int K)
+{
+    extern __shared__ float4 smem4[];
+    float *const row = reinterpret_cast<float *>(smem4);
+    __shared__ float wsm[kTapStride];
+    if (threadIdx.x < kTapStride) wsm[threadIdx.x] = w.w[threadIdx.x];
+    const size_t base = (size_t)blockIdx.x * W;
+    for (int x = threadIdx.x; x < W; x += kRowThreads) row[x] = src[base + x];
+    __syncthreads();
+    for (int x = threadIdx.x; x < W; x += kRowThreads) dst[base + x] = hblur_at(row, W, x, wsm, K);
+}
+
+// The same with nr rows per CTA in shared memory, a thread making kHbOut
+// neighbouring outputs (tap_sums).  Element e of a row sits at
+// e ^ ((e >> 5) & 15): lanes 16 elements apart hit all banks.  Rows come and go in
+// pieces (VEC: of 16 bytes): 2^lgx threads a row where that covers one, so that all
+// pieces of narrow rows are requested at once, else (lgx < 0) the CTA row by row.
+// The sums go back to the row buffer and leave from there; a row of more than one
+// round of the CTA sends them through a stage behind it, or straight from the
+// registers where that does not fit.
 constexpr int kHbOut = 16;
+constexpr int kHbStage = kRowThreads * kHbOut;   // floats
 __host__ __device__ constexpr int hb_row_floats(int W) { return (W + 15) & ~15; }
 __device__ __forceinline__ int hb_at(int e) { return e ^ ((e >> 5) & 15); }
-static __global__ void __launch_bounds__(kRowThreads) k_hblur(const float *src, float *dst, int W, int H, int nr, Taps w,
-                                                              int K)
+template <bool VEC>
+static __global__ void __launch_bounds__(kRowThreads) k_hblur(const float *src, float *dst, int W, int H, int nr, int lgx,
+                                                              bool staged, Taps w, int K)
 {
     extern __shared__ float4 smem4[];
     float *const buf = reinterpret_cast<float *>(smem4);
     __shared__ float wsm[kTapStride];
-    const int T = blockDim.x, rs = hb_row_floats(W), chunks = rs / kHbOut, hw = (K - 1) / 2;
+    const int T = blockDim.x, rs = hb_row_floats(W), chunks = rs / kHbOut;
     for (int i = threadIdx.x; i < kTapStride; i += T) wsm[i] = w.w[i];
     const int y0 = blockIdx.x * nr, rows = min(nr, H - y0);
-    // rows in 16-byte pieces where they allow it
-    const bool vec = W % 4 == 0 && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0;
-    for (int r = 0; r < rows; ++r) {
-        const float *const s = src + (size_t)(y0 + r) * W;
-        float *const b = buf + r * rs;
-        if (vec) {
-#pragma unroll 2
-            for (int x = 4 * threadIdx.x; x < W; x += 4 * T) {
-                const float4 z = *reinterpret_cast<const float4 *>(s + x);
-                b[hb_at(x)] = z.x;
-                b[hb_at(x + 1)] = z.y;
-                b[hb_at(x + 2)] = z.z;
-                b[hb_at(x + 3)] = z.w;
-            }
+    const float *const s = src + (size_t)y0 * W;
+    float *const d = dst + (size_t)y0 * W;
+    constexpr int PC = VEC ? 4 : 1;
+    const int pw = W / PC;
+    // f(row, element) for the pieces of elements [e0, e1) of every row
+    auto pieces = [&](int e0, int e1, auto &&f) {
+        if (lgx >= 0) {
+            const int x = threadIdx.x & ((1 << lgx) - 1);
+#pragma unroll 4
+            for (int r = threadIdx.x >> lgx; r < rows; r += T >> lgx)
+                if (x < pw) f(r, x * PC);
         } else {
+            for (int r = 0; r < rows; ++r)
 #pragma unroll 4
-            for (int x = threadIdx.x; x < W; x += T) b[hb_at(x)] = s[x];
+                for (int e = e0 + threadIdx.x * PC; e < e1; e += T * PC) f(r, e);
         }
-    }
-    __syncthreads();
-    auto sums = [&](int c, float (&sum)[kHbOut], int &r, int &x0) {
-        r = c / chunks;
-        x0 = (c - r * chunks) * kHbOut;
-        const float *const row = buf + r * rs;
-        const int a = x0 - hw;
-        tap_sums(sum, wsm, K, [&](int i) { return row[hb_at(min(max(a + i, 0), W - 1))]; });
     };
-    float sum[kHbOut];
-    int r, x0;
-    if (rows * chunks <= T) {
-        const bool has = (int)threadIdx.x < rows * chunks;
-        if (has) sums(threadIdx.x, sum, r, x0);
-        __syncthreads();   // the rows have been read
-        if (has) {
-#pragma unroll
-            for (int o = 0; o < kHbOut; ++o) buf[r * rs + hb_at(x0 + o)] = sum[o];
+    pieces(0, W, [&](int r, int e) {
+        float *const b = buf + r * rs;
+        if constexpr (VEC) {
+            const float4 z = *reinterpret_cast<const float4 *>(s + r * W + e);
+            b[hb_at(e)] = z.x;
+            b[hb_at(e + 1)] = z.y;
+            b[hb_at(e + 2)] = z.z;
+            b[hb_at(e + 3)] = z.w;
+        } else {
+            b[hb_at(e)] = s[r * W + e];
         }
-        __syncthreads();
-        for (int q = 0; q < rows; ++q) {
-            float *const d = dst + (size_t)(y0 + q) * W;
-            const float *const b = buf + q * rs;
-            if (vec) {
-#pragma unroll 2
-                for (int x = 4 * threadIdx.x; x < W; x += 4 * T)
-                    *reinterpret_cast<float4 *>(d + x) =
-                        make_float4(b[hb_at(x)], b[hb_at(x + 1)], b[hb_at(x + 2)], b[hb_at(x + 3)]);
-            } else {
-#pragma unroll 4
-                for (int x = threadIdx.x; x < W; x += T) d[x] = b[hb_at(x)];
-            }
+    });
+    __syncthreads();
+    const int total = rows * chunks;   // chunk c of all rows starts at 16 c of the buffer
+    const bool one = total <= T;
+    for (int c0 = 0; c0 < total; c0 += T) {
+        const int c = c0 + threadIdx.x, r = c / chunks, x0 = (c - r * chunks) * kHbOut;
+        float sum[kHbOut];
+        if (c < total) {
+            const float *const row = buf + r * rs;
+            const int a = x0 - (K - 1) / 2;
+            tap_sums(sum, wsm, K, [&](int i) { return row[hb_at(min(max(a + i, 0), W - 1))]; });
         }
-    } else {   // rows longer than one round of the block
-        for (int c = threadIdx.x; c < rows * chunks; c += T) {
-            sums(c, sum, r, x0);
-            float *const out = dst + (size_t)(y0 + r) * W + x0;
+        if (!one && !staged) {
 #pragma unroll
             for (int o = 0; o < kHbOut; ++o)
-                if (x0 + o < W) out[o] = sum[o];
+                if (c < total && x0 + o < W) d[x0 + o] = sum[o];
+            continue;
         }
+        float *const out = one ? buf : buf + rs - kHbOut * c0;   // where chunk 0 would be
+        __syncthreads();   // the inputs have been read; the stage has been sent
+        if (c < total) {
+#pragma unroll
+            for (int o = 0; o < kHbOut; ++o) out[c * kHbOut + (o ^ ((x0 >> 5) & 15))] = sum[o];
+        }
+        __syncthreads();
+        pieces(c0 * kHbOut, one ? W : min(W, (c0 + T) * kHbOut), [&](int r, int e) {
+            const float *const b = out + r * rs;
+            if constexpr (VEC)
+                *reinterpret_cast<float4 *>(d + r * W + e) =
+                    make_float4(b[hb_at(e)], b[hb_at(e + 1)], b[hb_at(e + 2)], b[hb_at(e + 3)]);
+            else
+                d[r * W + e] = b[hb_at(e)];
+        });
     }
 }
 

@@ -46,4 +46,20 @@ inline bool dependent_pass(int tiles, int resident)
 // other way).
 inline bool pipelined_rows_dependent(int W) { return W < 2048; }
 
+// Whether the rows of a Gaussian blur of K taps run the kernel that makes 16
+// neighbouring outputs per thread from rolling registers, instead of the one that
+// makes one output per thread and turn (256 a turn, one row per CTA).  The rolling
+// kernel loads each tap once and takes several rows per CTA, but its code is long and
+// runs cold: 64 x 64 takes 3.1 us instead of 2.0, 256 x 256 (19 taps) 4.1 instead of
+// 2.5; 1000 x 800 5.6 instead of 9.0, 2048 x 1536 14 instead of 26, 64 x 16384 9.8
+// instead of 18.3.  Left side: what it saves, right side: what it costs, in us, a
+// least-squares fit of both kernels' times at 200 sizes with 3 to 59 taps (`vec`: rows
+// of 16-byte pieces).  On the mean its choice is within 1 % of the faster kernel.
+inline bool hblur_rolling(int W, int H, int K, bool vec)
+{
+    const double turns = (W + 255) / 256, mpx = 1e-6 * W * H;
+    return 0.16 * turns + 0.006 * turns * K + 0.56e-3 * H + (0.1 * K - 0.41) * mpx >
+           0.94 + 0.015 * K + (vec ? 0.0 : 1.0 + 0.8 * mpx);
+}
+
 }  // namespace imr

@@ -73,3 +73,32 @@ def test_transforms_on_both_sides_of_the_narrow_columns(cuda, h, w, sign):
 @pytest.mark.parametrize("w,dependent", [(64, 1), (1536, 1), (2048, 0), (4096, 0)])
 def test_long_pipelined_rows_do_not_start_early(rule, w, dependent):
     assert rule("pipelined_rows_dependent(%d)" % w) == dependent
+
+
+# rows of a blur: W, H, taps, 16-byte pieces, rolling kernel (measured us: rolling, other)
+@pytest.mark.parametrize("w,h,taps,vec,rolling", [
+    (64, 64, 19, 1, 0),          # 4.2, 2.2
+    (256, 256, 19, 1, 0),        # 4.5, 2.5
+    (16, 1024, 59, 1, 0),        # 5.9, 3.2
+    (331, 2649, 5, 0, 0),        # 10.4, 6.8
+    (64, 16384, 3, 1, 1),        # 7.6, 16.6
+    (1000, 800, 19, 1, 1),       # 5.6, 9.0
+    (2048, 1536, 19, 1, 1),      # 14, 26
+    (4100, 1000, 59, 1, 1)])     # 35, 82
+def test_rolling_row_blur_where_its_long_code_pays(rule, w, h, taps, vec, rolling):
+    assert rule("hblur_rolling(%d, %d, %d, %d)" % (w, h, taps, vec)) == rolling
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,w", [(16384, 64), (5003, 61), (4000, 30), (600, 256), (297, 1000), (593, 331), (7, 4100), (2, 9002),
+                                 (2, 53952), (2, 53956), (1, 58048)])
+@pytest.mark.parametrize("sigma", [0.4, 3.0])
+def test_rows_of_a_blur_bitexact(cuda, h, w, sigma):
+    """Many narrow rows per block, rows with and without a stage for their sums."""
+    import torch
+
+    import oracle
+    img = np.random.default_rng(h + w).random((h, w)).astype(np.float32)
+    d = torch.from_numpy(img).cuda()
+    imr.gaussian_blur(d, None, w, h, sigma, 1)
+    assert np.array_equal(d.cpu().numpy(), oracle.blur(img, sigma, "h"))
