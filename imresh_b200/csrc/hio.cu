@@ -137,12 +137,13 @@ static int launch_rand_field(float2 *X, long n, unsigned seed, cudaStream_t s)
     uint32_t *pow = nullptr;
     int rc = rand_pow_table(&pow);
     if (rc) return rc;
-    const long chunks = (n + kRandChunk - 1) / kRandChunk;
+    const int shift = rand_chunk_shift(n);
+    const long chunk = (long)kRandChunk << shift, chunks = (n + chunk - 1) / chunk;
     int n_pow = 0;
     while ((1L << n_pow) < chunks) ++n_pow;
-    if (n_pow > kRandPowTable) return IMR_ERR_UNSUPPORTED_SIZE;
+    if (n_pow + shift > kRandPowTable) return IMR_ERR_UNSUPPORTED_SIZE;
     const long blocks = (chunks + kRandThreads - 1) / kRandThreads;
-    k_rand_field<<<(unsigned)blocks, kRandThreads, 0, s>>>(X, n, rand_base(seed), pow, n_pow);
+    k_rand_field<<<(unsigned)blocks, kRandThreads, 0, s>>>(X, n, rand_base(seed), pow, n_pow, shift);
     HCK(cudaGetLastError());
     return IMR_SUCCESS;
 }

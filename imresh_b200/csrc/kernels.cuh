@@ -823,22 +823,20 @@ static __global__ void k_complex_norm(const float2 *src, float *dst, long n)
 // srand(2623091912) (src/imresh/libs/hybridInputOutput.cpp:160-167): glibc's
 // additive feedback generator, r[i] = r[i-31] + r[i-3] (mod 2^32) for i >= 34,
 // rand() number k = r[k + 344] >> 1.  Thread c makes the numbers
-// [c*kRandChunk, (c+1)*kRandChunk): its 31-word state (r[i-31..i-1]) starts
-// from the base state at i = 344 and jumps by B^c, B = A^kRandChunk the
-// recurrence's 31x31 step matrix over Z/2^32 raised to the chunk length,
-// composed from the table pow[j] = B^(2^j); then it runs the recurrence.
+// [c*m, (c+1)*m), m = kRandChunk << shift: its 31-word state (r[i-31..i-1]) starts
+// from the base state at i = 344 and jumps by (B^(2^shift))^c, B = A^kRandChunk the
+// recurrence's 31x31 step matrix over Z/2^32 raised to the smallest chunk, composed
+// from the table pow[j] = B^(2^j); then it runs the recurrence.
 // Element k of X becomes ((float)rand_k / RAND_MAX, 0) (cpp:163-167).
 constexpr int kRandLag = 31;
-// Numbers of a chunk: few, since a chunk is one thread's serial recurrence and the
-// jump to its start costs only two to three more matrix products: 992 numbers took
-// 117 us for 512 x 384 on 198 threads, 124 take 35.
+// Numbers of the smallest chunk; a launch takes 2^shift of them (rand_chunk_shift).
 constexpr int kRandChunk = 31 * 4;
 constexpr int kRandThreads = 128;
 struct RandBase {
     uint32_t s[kRandLag];
 };
 static __global__ void __launch_bounds__(kRandThreads) k_rand_field(float2 *X, long n, RandBase base,
-                                                                    const uint32_t *pow, int n_pow)
+                                                                    const uint32_t *pow, int n_pow, int shift)
 {
     __shared__ uint32_t P[kRandLag * kRandLag];
     const long c = (long)blockIdx.x * kRandThreads + threadIdx.x;
@@ -848,7 +846,7 @@ static __global__ void __launch_bounds__(kRandThreads) k_rand_field(float2 *X, l
     for (int j = 0; j < n_pow; ++j) {
         __syncthreads();
         for (int i = threadIdx.x; i < kRandLag * kRandLag; i += kRandThreads)
-            P[i] = pow[(size_t)j * kRandLag * kRandLag + i];
+            P[i] = pow[(size_t)(j + shift) * kRandLag * kRandLag + i];
         __syncthreads();
         if ((c >> j) & 1) {
             uint32_t t[kRandLag];
@@ -863,10 +861,10 @@ static __global__ void __launch_bounds__(kRandThreads) k_rand_field(float2 *X, l
             for (int i = 0; i < kRandLag; ++i) s[i] = t[i];
         }
     }
-    const long k0 = c * kRandChunk;
+    const long k0 = c * (kRandChunk << shift);
     if (k0 >= n) return;
-    const long kend = min(n, k0 + kRandChunk);
-    for (int o = 0; o < kRandChunk / kRandLag; ++o) {
+    const long kend = min(n, k0 + (kRandChunk << shift));
+    for (int o = 0; o < (kRandChunk << shift) / kRandLag; ++o) {
 #pragma unroll
         for (int q = 0; q < kRandLag; ++q) {
             const uint32_t r = s[q] + s[(q + kRandLag - 3) % kRandLag];   // r[i-31] + r[i-3]

@@ -62,4 +62,16 @@ inline bool hblur_rolling(int W, int H, int K, bool vec)
            0.94 + 0.015 * K + (vec ? 0.0 : 1.0 + 0.8 * mpx);
 }
 
+// A thread of the random field makes 124 << shift numbers (kRandChunk) one after
+// another, from a start that it reaches by matrix products.  Few numbers leave a
+// short chain, many leave few products: us at shifts 0, 1, 2, 3 for 512 x 384 numbers
+// 32, 43, 70, 113; 2048^2 56, 56, 84, 128; 6 Mi 75, 83, 85, 129; 8 Mi 103, 83, 88, 131; 12 Mi 141, 116, 148, 130;
+// 4096^2 181, 157, 148, 137; 32 Mi 334, 293, 342, 313.  Shift 3 is the best of them only
+// while its blocks of 128 threads are about one per SM.
+inline int rand_chunk_shift(long n)
+{
+    if (n < 7000000) return 0;
+    return n > 14000000 && n <= kSms * 128L * (124 << 3) ? 3 : 1;
+}
+
 }  // namespace imr
