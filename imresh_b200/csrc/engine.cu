@@ -1315,9 +1315,9 @@ int imr_gaussian_blur(float *d_data, float *d_tmp, unsigned W, unsigned H, doubl
         const int tx = (int)((W + kVbTileX - 1) / kVbTileX), nt = tx * (int)((H + kVbTileY - 1) / kVbTileY);
         const float *const in = axes == 3 ? d_tmp : d_data;
         float *const out = axes == 3 ? d_data : d_tmp;
-        if (nt >= 2 * 148)
+        if (!vblur_small_tiles(nt))
             k_vblur_plain<kVbTileY><<<nt, kVbThreads, 0, s>>>(in, out, (int)W, (int)H, t, K, nullptr);
-        else   // tiles of 128 rows would leave SMs idle
+        else
             k_vblur_plain<kVbTileYSmall><<<tx * (int)((H + kVbTileYSmall - 1) / kVbTileYSmall), kVbThreads, 0, s>>>(
                 in, out, (int)W, (int)H, t, K, nullptr);
         if (axes == 2) CK(cudaMemcpyAsync(d_data, d_tmp, (size_t)W * H * 4, cudaMemcpyDeviceToDevice, s));

@@ -62,6 +62,13 @@ inline bool hblur_rolling(int W, int H, int K, bool vec)
            0.94 + 0.015 * K + (vec ? 0.0 : 1.0 + 0.8 * mpx);
 }
 
+// Whether the columns of a plain blur run in tiles of 32 rows instead of 128 (`tiles` of
+// them, 32 columns each): where those leave SMs without a tile.  Columns of a blur with
+// 19 taps, 32 rows and 128: 640 x 1024 (160 tiles) 6.4 and 6.6 us, 900 x 700 (174) 7.3 and
+// 7.4, 1500 x 500 (188) 8.5 and 7.8, 1024 x 1024 (256) 8.1 and 6.9; 3 taps 5.2 and 5.3, 6.0 and
+// 6.1, 7.1 and 6.5, 6.7 and 5.7.
+inline bool vblur_small_tiles(int tiles) { return tiles < 6 * kSms / 5; }
+
 // A thread of the random field makes 124 << shift numbers (kRandChunk) one after
 // another, from a start that it reaches by matrix products.  Few numbers leave a
 // short chain, many leave few products: us at shifts 0, 1, 2, 3 for 512 x 384 numbers

@@ -104,6 +104,25 @@ def test_rows_of_a_blur_bitexact(cuda, h, w, sigma):
     assert np.array_equal(d.cpu().numpy(), oracle.blur(img, sigma, "h"))
 
 
+# columns of a blur: tiles of 128 rows, 32 rows instead (us: 32 rows, 128)
+@pytest.mark.parametrize("tiles,small", [(32, 1), (160, 1), (174, 1), (188, 0), (256, 0)])   # 188: 8.5, 7.8; 256: 8.1, 6.9
+def test_small_blur_tiles_only_where_large_ones_leave_sms_idle(rule, tiles, small):
+    assert rule("vblur_small_tiles(%d)" % tiles) == small
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,w", [(700, 900), (500, 1500), (4095, 199)])
+@pytest.mark.parametrize("sigma", [0.4, 10.0])
+def test_columns_of_a_blur_bitexact(cuda, h, w, sigma):
+    import torch
+
+    import oracle
+    img = np.random.default_rng(h + w).random((h, w)).astype(np.float32)
+    d = torch.from_numpy(img).cuda()
+    imr.gaussian_blur(d, torch.empty_like(d), w, h, sigma, 2)
+    assert np.array_equal(d.cpu().numpy(), oracle.blur(img, sigma, "v"))
+
+
 # numbers, shift: 4096^2 numbers in the smallest chunks took 181 us, 137 at shift 3
 @pytest.mark.parametrize("n,shift", [(1, 0), (512 * 384, 0), (2048 * 2048, 0), (8 << 20, 1), (4096 * 4096, 3), (32 << 20, 1)])
 def test_chunks_of_a_large_random_field(rule, n, shift):
