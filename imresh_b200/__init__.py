@@ -298,6 +298,11 @@ def vector_max(d_data, n: int, stream=None) -> float:
     return r.value
 
 
+def release_scratch():
+    """Give back the device memory that the synchronous host calls keep (up to 256 MB)."""
+    _check(lib().imr_release_scratch(), "imr_release_scratch")
+
+
 # ------------------------------------------------------------------ engine
 class CResult(C.Structure):
     _fields_ = [("tag", C.c_longlong), ("width", C.c_uint), ("height", C.c_uint),

@@ -367,6 +367,10 @@ static int admit(imr_engine *E)
             e = cudaErrorMemoryAllocation;
         } else {
             e = cudaMallocFromPoolAsync((void **)&j->arena, j->S.bytes, E->pool, E->s);
+            if (e == cudaErrorMemoryAllocation && scratch_release() == cudaSuccess) {
+                cudaGetLastError();
+                e = cudaMallocFromPoolAsync((void **)&j->arena, j->S.bytes, E->pool, E->s);
+            }
         }
         if (e != cudaSuccess) {
             ++E->alloc_failures;
@@ -1102,6 +1106,7 @@ int imr_engine_create(imr_engine **out, size_t device_bytes, int max_jobs, void 
     }
     if (device_bytes == 0) {
         size_t fr = 0, tot = 0;
+        scratch_release();   // memory that nothing uses counts as free
         cudaMemGetInfo(&fr, &tot);
         device_bytes = fr / 10 * 8;
     }

@@ -217,7 +217,8 @@ int gaussian_weights(double sigma, float *w, int cap)
 // calls and gives the rest back.  The default pool gives everything back at each
 // synchronisation, and mapping it again took half of a 1000 x 800 forward model
 // (0.5 of 1.0 ms).  Stream-ordered, so calls on several streams and threads may
-// overlap.
+// overlap.  What it keeps is given back before an engine counts the free memory,
+// when an allocation of a plan or a request fails, and by imr_release_scratch.
 constexpr uint64_t kScratchKeep = 256ull << 20;
 static std::mutex g_pool_mu;
 static std::map<int, cudaMemPool_t> g_pool;
@@ -251,6 +252,25 @@ cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s)
         }
     }
     return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
+cudaError_t scratch_release()
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    auto it = g_pool.find(dev);
+    return it == g_pool.end() ? cudaSuccess : cudaMemPoolTrimTo(it->second, 0);
+}
+
+cudaError_t device_alloc(void **p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    e = scratch_release();
+    return e == cudaSuccess ? cudaMalloc(p, bytes) : e;
 }
 
 // ---------------------------------------------------------------- dispatch
@@ -906,7 +926,7 @@ int imr_plan_create(imr_plan **out, unsigned W, unsigned H, const imr_params *pa
     }
     const size_t extra = (sizeof(JobState) + 255) / 256 * 256 + (sizeof(JobDev) + 255) / 256 * 256 +
                          (5 * sizeof(WorkList) + 255) / 256 * 256;
-    cudaError_t e = cudaMalloc(&P->arena, S.bytes + extra);
+    cudaError_t e = device_alloc((void **)&P->arena, S.bytes + extra);
     if (e != cudaSuccess) {
         set_error("cudaMalloc plan arena", e);
         delete P;
@@ -1352,6 +1372,12 @@ int imr_diffraction_intensity(float *h_io, unsigned W, unsigned H, void *stream)
     if (rc) return rc;
     CK(e);
     CK(cudaStreamSynchronize(s));
+    return IMR_SUCCESS;
+}
+
+int imr_release_scratch(void)
+{
+    CK(scratch_release());
     return IMR_SUCCESS;
 }
 

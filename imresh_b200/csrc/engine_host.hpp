@@ -45,6 +45,10 @@ int gaussian_weights(double sigma, float *w, int cap);
 int ensure_kernel_attributes();
 // Scratch of a synchronous call (free with cudaFreeAsync on the same stream).
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t s);
+// Give the kept scratch memory of the current device back to the driver.
+cudaError_t scratch_release();
+// cudaMalloc that gives the kept scratch back and tries again when memory is out.
+cudaError_t device_alloc(void **p, size_t bytes);
 void resolve_params(const imr_params *in, imr_params &out);
 int build_weight_table(const imr_params &p, std::vector<float> &w, std::vector<int> &taps);
 

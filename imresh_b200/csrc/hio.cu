@@ -246,7 +246,7 @@ int imr_hio_plan_create(imr_hio_plan **out, unsigned W, unsigned H, unsigned nCy
     J.n_err = n_cycles < kHioMaxErrors ? n_cycles + 1 : kHioMaxErrors;
     S.bytes = S.oErr + ((size_t)J.n_err * 4 + 255) / 256 * 256;
     const size_t sst = (sizeof(JobState) + 255) / 256 * 256, sdj = (sizeof(JobDev) + 255) / 256 * 256;
-    cudaError_t e = cudaMalloc(&P->arena, S.bytes + sst + sdj + 256);
+    cudaError_t e = device_alloc((void **)&P->arena, S.bytes + sst + sdj + 256);
     if (e != cudaSuccess) {
         set_error("cudaMalloc HIO plan arena", e);
         delete P;

@@ -184,6 +184,11 @@ int imr_diffraction_intensity(float *h_io, unsigned W, unsigned H, void *stream)
 /* Global maximum of n floats (cudaVectorMax, cudaVectorReduce.cu:229-239);
  * the result goes to HOST *h_max; synchronous. */
 int imr_vector_max(const float *d_data, size_t n, float *h_max, void *stream);
+/* imr_diffraction_intensity, imr_vector_max, imr_calculate_hio_error and
+ * imr_fft2d_split keep up to 256 MB of device memory per device between calls.
+ * It is given back when an engine counts the free memory and when the memory of
+ * a plan or a request runs out; this call gives it back at once. */
+int imr_release_scratch(void);
 
 /* Mask element types of imr_calculate_hio_error. */
 #define IMR_MASK_F32 0
