@@ -1146,7 +1146,7 @@ static int submit(imr_engine *E, const float *h_in, bool intensity, float *h_out
     j->W = W;
     j->H = H;
     resolve_params(params, j->p);
-    int rc = job_prepare(W, H, j->p, j->J, j->S);
+    int rc = job_prepare(W, H, j->p, j->J, j->S, false);
     if (rc) {
         delete j;
         return rc;
@@ -1417,7 +1417,7 @@ int imr_engine_resume(imr_engine *E, const void *h_buf, size_t bytes, float *h_o
     j->W = h.W;
     j->H = h.H;
     j->p = h.p;
-    int rc = job_prepare(h.W, h.H, j->p, j->J, j->S);
+    int rc = job_prepare(h.W, h.H, j->p, j->J, j->S, false);
     if (rc) {
         delete j;
         return rc;

@@ -433,7 +433,7 @@ int rows_per_tile(const RowKernels &rk, int W, int H)
 }
 int row_tile_smem(const RowKernels &rk, int W, int rpc) { return rk.mx ? mx_row_smem(W, rpc) : rk.smem; }
 
-ColKernels col_kernels(int N)
+ColKernels col_kernels(int N, int W)
 {
     std::vector<int> rad;
     if (!factor_len(N, rad) && length_supported(N)) N = -bluestein_m(N);
@@ -442,7 +442,7 @@ ColKernels col_kernels(int N)
         IMR_SIZES(COLCASE)
         IMR_BS_SIZES(COLCASE)
 #undef COLCASE
-    default: return col_set_mx(N);
+    default: return col_set_mx(N, W);
     }
 }
 
@@ -481,6 +481,8 @@ int ensure_kernel_attributes()
         rks.push_back(row_kernels(n));
         cks.push_back(col_kernels(n));
     }
+    rks.push_back(rks.front());   // (a pair for the few-column kernels)
+    cks.push_back(col_kernels(2000, 1));
 #define PUSHBS(n) rks.push_back(row_set<n>()); cks.push_back(col_set<n>());
     IMR_BS_SIZES(PUSHBS)
 #undef PUSHBS
@@ -596,7 +598,7 @@ static int fft_launch(float2 *d, int W, int H, int sign, int axes, const FftPlan
 int fft_passes(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr, const FftPlanDev &pc,
                cudaStream_t s)
 {
-    return fft_launch(d, W, H, sign, axes, pr, pc, row_kernels(W), col_kernels(H), s);
+    return fft_launch(d, W, H, sign, axes, pr, pc, row_kernels(W), col_kernels(H, W), s);
 }
 
 }  // namespace imr
@@ -706,7 +708,7 @@ namespace imr {
 // X, G (c64) | M, hb, vb, out (f32) | mask (u8) | weights | taps | error
 // partials | per-cycle errors.  The JobState lives wherever the caller puts
 // it (plans: after the arena; the engine: in one array for all jobs).
-int job_prepare(unsigned W, unsigned H, const imr_params &p, JobDev &J, JobShape &S)
+int job_prepare(unsigned W, unsigned H, const imr_params &p, JobDev &J, JobShape &S, bool alone)
 {
     int rc;
     memset(&J, 0, sizeof(J));
@@ -715,7 +717,7 @@ int job_prepare(unsigned W, unsigned H, const imr_params &p, JobDev &J, JobShape
     if ((rc = make_fft_plan((int)W, J.prow)) || (rc = make_fft_plan((int)H, J.pcol))) return rc;
     if ((rc = build_weight_table(p, S.wt, S.taps))) return rc;
     S.rk = row_kernels(J.W);
-    S.ck = col_kernels(J.H);
+    S.ck = col_kernels(J.H, alone ? J.W : kManyColumns);
     J.rpc = rows_per_tile(S.rk, J.W, J.H);
     J.cpc = S.ck.nb < J.W ? S.ck.nb : J.W;
     S.p_rows = S.rk.p_hio != nullptr;
@@ -1289,7 +1291,7 @@ int imr_fft2d(void *d_data, unsigned W, unsigned H, int sign, void *stream)
         if (rc) return rc;
         if ((rc = make_fft_plan((int)W, last.pr)) || (rc = make_fft_plan((int)H, last.pc))) return rc;
         last.rk = row_kernels((int)W);
-        last.ck = col_kernels((int)H);
+        last.ck = col_kernels((int)H, (int)W);
         last.W = W;
         last.H = H;
         last.dev = dev;

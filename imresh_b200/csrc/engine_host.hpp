@@ -118,7 +118,9 @@ RowKernels row_kernels(int N);
 // shared memory of such a tile.
 int rows_per_tile(const RowKernels &rk, int W, int H);
 int row_tile_smem(const RowKernels &rk, int W, int rpc);
-ColKernels col_kernels(int N);
+// W: columns of the one image of a launch (several images of a launch: many).
+constexpr int kManyColumns = 1 << 30;
+ColKernels col_kernels(int N, int W = kManyColumns);
 // Lengths with kernels specialised at compile time and Bluestein transform
 // lengths M (power of two >= 2n - 1 for n <= 2048); any other supported length
 // runs the grouped-pass kernels (row_set_mx, col_set_mx).
@@ -129,7 +131,7 @@ RowKernels row_set();
 template <int N>
 ColKernels col_set();
 RowKernels row_set_mx(int n);
-ColKernels col_set_mx(int n);
+ColKernels col_set_mx(int n, int W);
 // Plain 2D transform passes (axes: 1 rows, 2 columns, 3 both).
 int fft_passes(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr, const FftPlanDev &pc,
                cudaStream_t s);
@@ -165,7 +167,8 @@ struct JobShape {
 };
 bool passes_dependent(const JobDev &J, const JobShape &S, const RowKernels &rk, const ColKernels &ck, bool fix, int n_split,
                       bool row_narrow, bool col_narrow);
-int job_prepare(unsigned W, unsigned H, const imr_params &p, JobDev &J, JobShape &S);
+// alone: no launch holds passes of other jobs.
+int job_prepare(unsigned W, unsigned H, const imr_params &p, JobDev &J, JobShape &S, bool alone = true);
 void job_bind(JobDev &J, JobShape &S, char *arena, JobState *st);
 int job_upload(const JobDev &J, const JobShape &S, char *arena, JobDev *dj, cudaStream_t s);
 // Fill JobDev::Mt from the modulus (stream-ordered; nothing to do when Mt is

@@ -33,26 +33,32 @@ namespace imr {
 constexpr int kMxRowThreads = 256;
 constexpr int kMxRowElems = 2048;     // values of a row tile at most
 constexpr int kMxColW = 4;            // columns of a column tile: 32-byte sectors
+constexpr int kMxColWFew = 2;         // the same for few long columns (mx_few_columns)
+// Blocks of a column pass per SM: few columns are no more than one.
+__host__ __device__ constexpr int mx_col_blocks(int T, int C) { return C == kMxColWFew ? 1 : T == 256 ? 3 : 2; }
 // Threads of a column tile: one butterfly of a grouped pass each, about (4 n / 16).
 __host__ __device__ constexpr int mx_col_threads(int n) { return n > 1024 ? 512 : 256; }
 
 // ---- shared-memory indices -----------------------------------------------------
 // Rows are flat (sequence b at b*n): one spare value per 32; column tiles hold
-// element e of column c at (e ^ ((e >> 4) & 15))*kMxColW + c.  Of the paddings
+// element e of column c at (e ^ ((e >> 4) & 15))*C + c.  Of the paddings
 // and swizzles tried over all passes of all lengths in a model of the banks these
 // needed the fewest wavefronts that one layout for every length gets: 1.36 and
 // 1.24 of a conflict-free exchange (none: 1.63 and 1.33).
 __host__ __device__ constexpr int mx_row_pad(int n) { return n + (n >> 5) + 1; }
-__host__ __device__ constexpr int mx_col_pad(int n) { return ((n + 15) & ~15) * kMxColW; }
+template <int C>
+__host__ __device__ constexpr int mx_col_pad(int n) { return ((n + 15) & ~15) * C; }
 __device__ __forceinline__ int mx_row_at(int f) { return f + (f >> 5); }
-__device__ __forceinline__ int mx_col_at(int e, int c) { return (e ^ ((e >> 4) & 15)) * kMxColW + c; }
+template <int C>
+__device__ __forceinline__ int mx_col_at(int e, int c) { return (e ^ ((e >> 4) & 15)) * C + c; }
 
 // bytes: two exchange buffers, one operand per value (g_prev rows / modulus
 // column tile), the twiddle table
 __host__ __device__ constexpr int mx_row_smem(int n, int nb) { return (2 * mx_row_pad(nb * n) + nb * n + n) * 8; }
+template <int C>
 __host__ __device__ constexpr int mx_col_smem(int n)
 {
-    return 2 * mx_col_pad(n) * 8 + mx_col_pad(n) * 4 + n * 8;
+    return 2 * mx_col_pad<C>(n) * 8 + mx_col_pad<C>(n) * 4 + n * 8;
 }
 
 // z *= w, the twiddle step.  The schedule's rounding, pinned: forward
@@ -68,20 +74,20 @@ __device__ __forceinline__ float2 mx_cmul_inv(float2 z, float2 w)
 }
 
 // ---- one grouped pass ------------------------------------------------------------
-// COLS: column tile of kMxColW sequences, else nseq flat rows.  T threads.
-template <int R1, int R2, bool COLS, int T>
+// C > 0: column tile of C sequences, else nseq flat rows.  T threads.
+template <int R1, int R2, int C, int T>
 __device__ __forceinline__ void mx_pass(const float2 *src, float2 *dst, const float2 *tw, const FftPass &P, int n,
                                         int nseq, bool inv)
 {
     constexpr int R = R1 * R2;
     const int L = P.L, Ns = P.Ns;
     const int st1 = P.st1, st2 = P.st2;
-    const int total = COLS ? kMxColW * L : nseq * L;
+    const int total = C ? C * L : nseq * L;
     for (int u = threadIdx.x; u < total; u += T) {
         int b, j;
-        if (COLS) {
-            b = u % kMxColW;
-            j = u / kMxColW;
+        if constexpr (C > 0) {
+            b = u % C;
+            j = u / C;
         } else {
             b = P.mL ? (int)__umulhi((unsigned)u, P.mL) : u;   // u / L
             j = u - b * L;
@@ -89,7 +95,7 @@ __device__ __forceinline__ void mx_pass(const float2 *src, float2 *dst, const fl
         const int k = P.mNs ? j - (int)__umulhi((unsigned)j, P.mNs) * Ns : 0;   // j mod Ns
         float2 v[R];
 #pragma unroll
-        for (int s = 0; s < R; ++s) v[s] = src[COLS ? mx_col_at(j + s * L, b) : mx_row_at(b * n + j + s * L)];
+        for (int s = 0; s < R; ++s) v[s] = src[C ? mx_col_at<C>(j + s * L, b) : mx_row_at(b * n + j + s * L)];
         if (k != 0) {
             float2 w[R1];
 #pragma unroll
@@ -141,7 +147,7 @@ __device__ __forceinline__ void mx_pass(const float2 *src, float2 *dst, const fl
 #pragma unroll
             for (int q2 = 0; q2 < R2; ++q2) {
                 const int e = o + (q1 + q2 * R1) * Ns;
-                dst[COLS ? mx_col_at(e, b) : mx_row_at(b * n + e)] = v[q1 * R2 + q2];
+                dst[C ? mx_col_at<C>(e, b) : mx_row_at(b * n + e)] = v[q1 * R2 + q2];
             }
     }
 }
@@ -161,7 +167,7 @@ __device__ __forceinline__ void mx_pass(const float2 *src, float2 *dst, const fl
 // body, in a loop: a kernel is short and its code cold, and with a second copy
 // of the passes the second transform took twice the first one's time (7400
 // cycles after 3700 for a row of 600, waiting for instructions).
-template <bool COLS, int T>
+template <int C, int T>
 __device__ __forceinline__ int mx_fft(int a, int b, int otw, const FftPlanDev &p, int nseq, bool inv)
 {
     extern __shared__ float4 smem4[];
@@ -172,7 +178,7 @@ __device__ __forceinline__ int mx_fft(int a, int b, int otw, const FftPlanDev &p
         switch (P.r1 * 16 + P.r2) {
 #define MXP(R1, R2)                                                                \
     case (R1) * 16 + (R2):                                                         \
-        mx_pass<R1, R2, COLS, T>(sm + a, sm + b, sm + otw, P, n, nseq, inv);     \
+        mx_pass<R1, R2, C, T>(sm + a, sm + b, sm + otw, P, n, nseq, inv);     \
         break;
             MXP(8, 2) MXP(8, 1)
             MXP(4, 4) MXP(4, 3) MXP(4, 1)
@@ -271,7 +277,7 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_hio_mx(const JobDev *j
         unsigned cnt = 0u;
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
-            r = mx_fft<false, T>(r, oa + ob - r, ot, sp, nr, h == 0);
+            r = mx_fft<0, T>(r, oa + ob - r, ot, sp, nr, h == 0);
             if (h == 1) break;
             if (it + (int)gridDim.x >= l.n) pdl_trigger();
             if (FIRST) {
@@ -378,7 +384,7 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_row_finish_mx(const JobDev
         __syncthreads();
         if (stop) continue;
         if (wi.tile == 0 && threadIdx.x == 0) st->max_bits = 0u;
-        const int r = mx_fft<false, T>(oa, ob, ot, sp, nr, true);
+        const int r = mx_fft<0, T>(oa, ob, ot, sp, nr, true);
         if (it + (int)gridDim.x >= l.n) pdl_trigger();
         float *const nrm = reinterpret_cast<float *>(sm + oa + ob - r);
         double tot = 0.0, cnt = 0.0;
@@ -449,7 +455,7 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_fft_rows_mx(float2 *data, 
     }
     cp_async_wait();
     __syncthreads();
-    const int r = mx_fft<false, T>(oa, ob, ot, p, nr, S > 0);
+    const int r = mx_fft<0, T>(oa, ob, ot, p, nr, S > 0);
     pdl_trigger();
 #pragma unroll
     for (int m = 0; m < V; ++m) {
@@ -464,36 +470,36 @@ __global__ void __launch_bounds__(kMxRowThreads, 3) k_fft_rows_mx(float2 *data, 
 // mode 0 column pass (forward, modulus projection, inverse; see b_col),
 // 1 column init (inverse of (M, 0)), 2 plain forward, 3 plain inverse
 // request the tile (and the modulus of mode 0)
-template <int MODE, int T>
+template <int MODE, int T, int C>
 __device__ __forceinline__ void mx_col_request(const float2 *X, const float *M, int W, int H, int x0)
 {
     extern __shared__ float4 smem4[];
     float2 *const sm = reinterpret_cast<float2 *>(smem4);
-    constexpr int C = kMxColW, RS = T / C;   // rows per round of the block
-    float *const smod = reinterpret_cast<float *>(sm + 2 * mx_col_pad(H) + H);
+    constexpr int RS = T / C;   // rows per round of the block
+    float *const smod = reinterpret_cast<float *>(sm + 2 * mx_col_pad<C>(H) + H);
     const int c = threadIdx.x % C, y_ = threadIdx.x / C;
     if (x0 + c < W) {
         const size_t col = x0 + c;
 #pragma unroll 4
         for (int y = y_; y < H; y += RS) {
-            if (MODE == 1) sm[mx_col_at(y, c)] = make_float2(M[(size_t)y * W + col], 0.f);
-            else if (MODE == 3) sm[mx_col_at(y, c)] = make_float2(X[(size_t)y * W + col].x, -X[(size_t)y * W + col].y);
-            else cp_async8(sm + mx_col_at(y, c), X + (size_t)y * W + col);
+            if (MODE == 1) sm[mx_col_at<C>(y, c)] = make_float2(M[(size_t)y * W + col], 0.f);
+            else if (MODE == 3) sm[mx_col_at<C>(y, c)] = make_float2(X[(size_t)y * W + col].x, -X[(size_t)y * W + col].y);
+            else cp_async8(sm + mx_col_at<C>(y, c), X + (size_t)y * W + col);
             if (MODE == 0) cp_async4(smod + y * C + c, M + (size_t)y * W + col);
         }
     } else {
-        for (int y = y_; y < H; y += RS) sm[mx_col_at(y, c)] = make_float2(0.f, 0.f);
+        for (int y = y_; y < H; y += RS) sm[mx_col_at<C>(y, c)] = make_float2(0.f, 0.f);
     }
 }
 // the tile's work once it has arrived
-template <int MODE, int T>
+template <int MODE, int T, int C>
 __device__ __forceinline__ void mx_col_run(float2 *X, int W, int H, int x0, const FftPlanDev &p, bool guard,
                                            bool last)
 {
     extern __shared__ float4 smem4[];
     float2 *const sm = reinterpret_cast<float2 *>(smem4);
-    constexpr int C = kMxColW, RS = T / C;
-    const int ob = mx_col_pad(H), ot = 2 * ob;
+    constexpr int RS = T / C;
+    const int ob = mx_col_pad<C>(H), ot = 2 * ob;
     const float *const smod = reinterpret_cast<const float *>(sm + ot + H);
     const int c = threadIdx.x % C, y_ = threadIdx.x / C;
     const bool ok = x0 + c < W;
@@ -501,14 +507,14 @@ __device__ __forceinline__ void mx_col_run(float2 *X, int W, int H, int x0, cons
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
         if (last && h == 1) pdl_trigger();
-        r = mx_fft<true, T>(r, ob - r, ot, p, C, MODE == 1 || MODE == 3 || h == 1);
+        r = mx_fft<C, T>(r, ob - r, ot, p, C, MODE == 1 || MODE == 3 || h == 1);
         if (MODE != 0 || h == 1) break;
         if (ok) {
 #pragma unroll 4
             for (int y = y_; y < H; y += RS) {
-                const float2 g = sm[r + mx_col_at(y, c)];
+                const float2 g = sm[r + mx_col_at<C>(y, c)];
                 const float f = modulus_factor(smod[y * C + c], g, guard);
-                sm[r + mx_col_at(y, c)] = make_float2(__fmul_rn(g.x, f), -__fmul_rn(g.y, f));
+                sm[r + mx_col_at<C>(y, c)] = make_float2(__fmul_rn(g.x, f), -__fmul_rn(g.y, f));
             }
         }
         __syncthreads();
@@ -516,14 +522,14 @@ __device__ __forceinline__ void mx_col_run(float2 *X, int W, int H, int x0, cons
     if (ok) {
 #pragma unroll 4
         for (int y = y_; y < H; y += RS) {
-            const float2 z = sm[r + mx_col_at(y, c)];
+            const float2 z = sm[r + mx_col_at<C>(y, c)];
             X[(size_t)y * W + x0 + c] = make_float2(z.x, MODE == 2 ? z.y : -z.y);
         }
     }
 }
 
-template <int MODE, int T>
-__global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_col_mx(const JobDev *jobs, const WorkList *L)
+template <int MODE, int T, int C>
+__global__ void __launch_bounds__(T, mx_col_blocks(T, C)) k_col_mx(const JobDev *jobs, const WorkList *L)
 {
     extern __shared__ float4 smem4[];
     float2 *const sm = reinterpret_cast<float2 *>(smem4);
@@ -538,7 +544,7 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_col_mx(const JobDev *jo
         const WorkItem wi = l.items ? l.items[it] : WorkItem{0, it};
         const JobDev &J = jobs[wi.job];
         const JobState *const st = J.st;
-        const int W = J.W, H = J.H, x0 = wi.tile * kMxColW;
+        const int W = J.W, H = J.H, x0 = wi.tile * C;
         float2 *const X = J.X;
         const float *const M = J.M;
         const float2 *const gtw = J.pcol.tw;
@@ -546,33 +552,33 @@ __global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_col_mx(const JobDev *jo
         const bool other = job != wi.job;
         const int word = other ? mx_plan_word(J.pcol) : 0;
         if (job < 0) pdl_wait();
-        mx_col_request<MODE, T>(X, M, W, H, x0);
+        mx_col_request<MODE, T, C>(X, M, W, H, x0);
         if (other)
-            for (int i = threadIdx.x; i < H; i += T) cp_async8(sm + 2 * mx_col_pad(H) + i, gtw + i);
+            for (int i = threadIdx.x; i < H; i += T) cp_async8(sm + 2 * mx_col_pad<C>(H) + i, gtw + i);
         const int stop = MODE == 0 ? st->stop : 0;   // (the check block may be setting it: decided as one)
         if (other) mx_store_plan(&sp, word);
         job = wi.job;
         cp_async_wait();
         if (__syncthreads_or(stop)) continue;
-        mx_col_run<MODE, T>(X, W, H, x0, sp, guard, it + (int)gridDim.x >= l.n);
+        mx_col_run<MODE, T, C>(X, W, H, x0, sp, guard, it + (int)gridDim.x >= l.n);
         __syncthreads();
     }
 }
 
-template <int S, int T>
-__global__ void __launch_bounds__(T, T == 256 ? 3 : 2) k_fft_cols_mx(float2 *data, const __grid_constant__ FftPlanDev p,
+template <int S, int T, int C>
+__global__ void __launch_bounds__(T, mx_col_blocks(T, C)) k_fft_cols_mx(float2 *data, const __grid_constant__ FftPlanDev p,
                                                                     int W, int)
 {
     extern __shared__ float4 smem4[];
     float2 *const sm = reinterpret_cast<float2 *>(smem4);
     constexpr int MODE = S < 0 ? 2 : 3;
-    const int H = p.n, x0 = blockIdx.x * kMxColW;
+    const int H = p.n, x0 = blockIdx.x * C;
     pdl_wait();
-    mx_col_request<MODE, T>(data, nullptr, W, H, x0);
-    for (int i = threadIdx.x; i < H; i += T) cp_async8(sm + 2 * mx_col_pad(H) + i, p.tw + i);
+    mx_col_request<MODE, T, C>(data, nullptr, W, H, x0);
+    for (int i = threadIdx.x; i < H; i += T) cp_async8(sm + 2 * mx_col_pad<C>(H) + i, p.tw + i);
     cp_async_wait();
     __syncthreads();
-    mx_col_run<MODE, T>(data, W, H, x0, p, true, false);
+    mx_col_run<MODE, T, C>(data, W, H, x0, p, true, false);
 }
 
 }  // namespace imr

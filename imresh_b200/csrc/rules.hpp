@@ -62,6 +62,14 @@ inline bool hblur_rolling(int W, int H, int K, bool vec)
            0.94 + 0.015 * K + (vec ? 0.0 : 1.0 + 0.8 * mpx);
 }
 
+// Whether grouped-pass columns of n > 1024 values run in tiles of two columns instead
+// of four, for an image of W columns that has the launch to itself: where the tiles of
+// two still leave a quarter of the SMs without one.  A tile is then half the work of a
+// block (one round of its threads in most passes, 123 registers instead of 64 and
+// spills).  An iteration of 64 x 1280 21.4 -> 14.5 us, 128 x 1792 26.5 -> 18.9, 222 x 2000
+// 33 -> 29; a transform of 128 x 1715 11.7 -> 10.3 us.
+inline bool mx_few_columns(int n, int W) { return n > 1024 && (W + 1) / 2 <= 111; }
+
 // Whether the columns of a plain blur run in tiles of 32 rows instead of 128 (`tiles` of
 // them, 32 columns each): where those leave SMs without a tile.  Columns of a blur with
 // 19 taps, 32 rows and 128: 640 x 1024 (160 tiles) 6.4 and 6.6 us, 900 x 700 (174) 7.3 and

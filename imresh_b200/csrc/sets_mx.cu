@@ -12,18 +12,18 @@ RowKernels row_set_mx(int n)
     k.mx = 1;
     return k;
 }
-template <int T>
+template <int T, int C>
 static ColKernels col_set_mx_t(int n)
 {
-    ColKernels k{k_col_mx<0, T>, k_col_mx<1, T>, k_fft_cols_mx<-1, T>, k_fft_cols_mx<+1, T>, kMxColW, T,
-                 mx_col_smem(n), nullptr, 0, 0, 0, 0, 0, 0};
+    ColKernels k{k_col_mx<0, T, C>, k_col_mx<1, T, C>, k_fft_cols_mx<-1, T, C>, k_fft_cols_mx<+1, T, C>, C, T,
+                 mx_col_smem<C>(n), nullptr, 0, 0, 0, 0, 0, 0};
     k.checks = 1;
     return k;
 }
-ColKernels col_set_mx(int n)
+ColKernels col_set_mx(int n, int W)
 {
-    return mx_col_threads(n) == 256 ? col_set_mx_t<256>(n) : col_set_mx_t<512>(n);
+    if (mx_few_columns(n, W)) return col_set_mx_t<512, kMxColWFew>(n);
+    return mx_col_threads(n) == 256 ? col_set_mx_t<256, kMxColW>(n) : col_set_mx_t<512, kMxColW>(n);
 }
-
 
 }  // namespace imr
