@@ -569,8 +569,8 @@ static int fft_launch(float2 *d, int W, int H, int sign, int axes, const FftPlan
     const bool narrow = ck.f_fwd && fft_narrow_columns((W + ck.nb - 1) / ck.nb);
     const int rpc = rk.mx ? rows_per_tile(rk, W, H) : rk.nb, cpc = narrow ? ck.f_nb : ck.nb;
     const int nrt = (H + rpc - 1) / rpc, nct = (W + cpc - 1) / cpc, ct = narrow ? ck.f_threads : ck.threads;
-    const size_t sr = rk.smem ? (size_t)row_tile_smem(rk, W, rpc) : ((size_t)rpc * W + rk.bs_m) * 8;
-    const size_t sc = narrow ? (size_t)ck.f_smem : ck.smem ? (size_t)ck.smem : ((size_t)H + ck.bs_m) * cpc * 8;
+    const size_t sr = rk.smem ? (size_t)row_tile_smem(rk, W, rpc) : (size_t)rpc * W * 8;
+    const size_t sc = narrow ? (size_t)ck.f_smem : ck.smem ? (size_t)ck.smem : (size_t)H * cpc * 8;
     const auto rows = sign < 0 ? rk.fft_fwd : rk.fft_inv;
     const auto cols = sign < 0 ? (narrow ? ck.f_fwd : ck.fft_fwd) : (narrow ? ck.f_inv : ck.fft_inv);
     // the second transform may start while the first one drains (fft_rows_start_early)
@@ -737,15 +737,12 @@ int job_prepare(unsigned W, unsigned H, const imr_params &p, JobDev &J, JobShape
     // the image has fewer rows / columns than NB
     if (S.rk.smem) {
         S.smem_row = S.smem_fin = (size_t)row_tile_smem(S.rk, J.W, J.rpc);   // norms reuse the FFT buffers
-    } else if (S.rk.bs_m) {   // row + Bluestein work area (the norms reuse the work area)
-        S.smem_row = S.smem_fin = ((size_t)J.W + S.rk.bs_m) * sizeof(float2);
     } else {
         S.smem_row = (size_t)S.rk.nb * J.W * sizeof(float2);
         S.smem_fin = S.smem_row + (size_t)S.rk.nb * J.W * sizeof(float);
     }
     S.smem_col = S.ck.smem ? (size_t)S.ck.smem
-                 : S.ck.bs_m ? ((size_t)J.H + S.ck.bs_m) * S.ck.nb * sizeof(float2)
-                             : (size_t)S.ck.nb * J.H * sizeof(float2);
+                           : (size_t)S.ck.nb * J.H * sizeof(float2);
     const size_t N = (size_t)W * H;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     size_t off = 0;

@@ -66,7 +66,6 @@ struct RowKernels {
     void (*p_hio_first)(const JobDev *, const WorkList *);
     void (*p_hio)(const JobDev *, const WorkList *);
     int p_smem_first, p_smem;
-    int bs_m;      // Bluestein work length (0: direct transform)
     // fixed-support HIO row passes (libs::hybridInputOutput): per-tile kernel
     // and, where the length has one, the pipelined kernel (shared memory p_smem)
     void (*hio_fix)(const JobDev *, const WorkList *);
@@ -95,7 +94,6 @@ struct ColKernels {
     int p_box_rows;  // rows per 2D TMA box
     int p_tma_m;     // 1: the modulus tile also arrives by TMA
     int p_threads;   // threads of the pipelined column pass
-    int bs_m;        // Bluestein work length (0: direct transform)
     int p_nb;        // columns per tile of the pipelined pass (its TMA box width)
     int p_mt;        // 1: the pipelined pass reads the modulus from JobDev::Mt when set
     // split-precision tensor-core column passes ([0] BF16 hi+lo, [1] FP16 hi+lo;

@@ -1549,9 +1549,8 @@ __global__ void __launch_bounds__(rcol_threads(M)) k_fft_cols_bs(float2 *data, F
 
 // ---- Bluestein with 16 values per thread (work lengths M >= 256) ------------
 // The same chain as reg_bluestein on the 16-value register FFT: two
-// exchanges per length-M transform up to M = 4096 instead of three, and
-// twiddle powers in registers (loaded once per CTA; every job of a launch has
-// the same work length).  n <= M/2, so a thread's values m >= 8 are the zero
+// exchanges per length-M transform up to M = 4096 instead of three; the twiddle
+// powers are read from the table at each use (LdTw16).  n <= M/2, so a thread's values m >= 8 are the zero
 // padding: they are neither loaded, updated nor stored, the first radix-16 pass
 // skips the operations with them, and the last pass does not form them.
 //
@@ -1568,8 +1567,9 @@ __host__ __device__ constexpr int bs16_col_nb(int M) { return M >= 4096 ? 2 : (4
 __host__ __device__ constexpr int bs16_col_threads(int M) { return bs16_col_nb(M) * M / 16; }
 // exchange buffer | modulus of the columns
 __host__ __device__ constexpr int bs16_col_smem(int M) { return bs16_col_nb(M) * (M * 8 + M / 2 * 4); }
-// 16 warps per SM at 128 registers, no spills; 20 and 24 warps (96, 80 registers,
-// 180-480 bytes of spills) measured 0-10 % slower.
+// 16 warps per SM at 128 registers: the passes of an iteration spill at most 32
+// bytes, the finish pass about 100.  20 and 24 warps (96, 80 registers, 180-480
+// bytes of spills) measured 0-10 % slower.
 __host__ __device__ constexpr int bs16_min_blocks(int threads) { return threads <= 512 ? 512 / threads : 1; }
 
 // The length-n transform of v (positions l + m*M/16, m < 8; the others are
@@ -1859,7 +1859,6 @@ k_col_bs16(const JobDev *jobs, const WorkList *L)
         if (MODE == 0) hio_check_block<bs16_col_threads(M)>(jobs, list);
         return;
     }
-    const LdTw16<M> rtw{jobs[list.items ? list.items[blockIdx.x].job : 0].pcol.tw, (int)threadIdx.x / NB};
     const WorkItem wi = list.items ? list.items[blockIdx.x] : WorkItem{0, (int)blockIdx.x};
     const JobDev &J = jobs[wi.job];
     const JobState *const st = J.st;
