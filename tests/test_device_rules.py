@@ -84,3 +84,14 @@ def test_pipelined_passes_trigger_by_their_length():
     assert set(triggers) == {"k_row_hio_p", "k_row_finish_p", "k_col_p", "k_col_p16"}
     for name, conds in triggers.items():
         assert conds and all(c.startswith("pdl_length(N) && ") for c in conds), name
+
+
+def test_pipelined_passes_of_a_batch_request_their_first_tile_first():
+    """Where an item has to be read to know the job (a batch's lists), the tables come
+    after the first live tile has been found."""
+    seen = {}
+    for head, body in _bodies("kernels.cuh"):
+        name = re.search(r"\b(k_row_hio_p|k_row_finish_p|k_col_p|k_col_p16)\(const JobDev", head)
+        if name and "__global__" in head and name.group(1) not in seen:
+            seen[name.group(1)] = re.search(r"const bool early = (pdl_length\(N\) && )?!walk\.items;", body)
+    assert len(seen) == 4 and all(seen.values()), seen
