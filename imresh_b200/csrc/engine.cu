@@ -634,6 +634,7 @@ struct imr_plan {
     int g_col_tc = 0;
     void (*vblur)(const JobDev *, const WorkList *) = k_vblur<kVbTileY>;
     bool dependent = false;   // passes launched to start while the pass before drains
+    bool cols_dependent = false;   // the column passes too
 };
 
 // The pipelined column pass of the plan's precision.
@@ -664,10 +665,10 @@ static cudaError_t plan_launch_col(imr_plan *P, cudaStream_t s)
     const WorkList *L = P->Lcol;
     if (P->prec) return launch_pass(false, plan_col_kernel(P), P->g_col_tc, ck.p_threads, ck.p_smem_tc, s, dj, L);
     if (P->n_col_narrow)
-        return launch_pass(P->dependent, ck.n_col, P->n_col_narrow, ck.n_threads, ck.n_smem, s, dj,
+        return launch_pass(P->cols_dependent, ck.n_col, P->n_col_narrow, ck.n_threads, ck.n_smem, s, dj,
                            (const WorkList *)P->Lcol_n);
-    if (!P->p_cols) return launch_pass(P->dependent, ck.col, P->hj.n_col_tiles, ck.threads, P->smem_col, s, dj, L);
-    return launch_pass(P->dependent, plan_col_kernel(P), P->g_col, ck.p_threads, ck.p_smem, s, dj, L);
+    if (!P->p_cols) return launch_pass(P->cols_dependent, ck.col, P->hj.n_col_tiles, ck.threads, P->smem_col, s, dj, L);
+    return launch_pass(P->cols_dependent, plan_col_kernel(P), P->g_col, ck.p_threads, ck.p_smem, s, dj, L);
 }
 
 static int plan_launch_cycle(imr_plan *P, cudaStream_t s)
@@ -966,6 +967,10 @@ int imr_plan_create(imr_plan **out, unsigned W, unsigned H, const imr_params *pa
     }
     narrow_tiles(P->rk, P->ck, P->p_cols, P->W, P->H, &P->n_row_narrow, &P->n_col_narrow);
     P->dependent = passes_dependent(J, S, P->rk, P->ck, false, n_split, P->n_row_narrow > 0, P->n_col_narrow > 0);
+    const bool one_item_cols = P->n_col_narrow || !P->p_cols;
+    P->cols_dependent = P->dependent && (!P->n_row_narrow || !one_item_cols ||
+                                         small_plan_columns_early(P->n_col_narrow ? P->n_col_narrow : J.n_col_tiles,
+                                                                  P->n_col_narrow ? P->ck.n_threads : P->ck.threads));
     if (J.n_vb_tiles < 2 * 148) {   // tiles of 128 rows would leave SMs idle
         J.n_vb_tiles = J.vb_tiles_x * ((J.H + kVbTileYSmall - 1) / kVbTileYSmall);
         P->vblur = k_vblur<kVbTileYSmall>;

@@ -45,6 +45,12 @@ inline bool dependent_pass(int tiles, int resident)
 // the columns' last tiles cost 2048 x 1024 38.1 -> 39.8 us (3072 x 512 39.5 and 39.9 the
 // other way).
 inline bool pipelined_rows_dependent(int W) { return W < 2048; }
+// Whether the columns of a small plan start while its narrow rows drain.  A column
+// block of 256 threads takes half an SM: more than 64 of them but less than one per SM
+// go two to those SMs that are free first, and the others wait for them: 384 x 1024
+// (96 blocks) 16.3 us an iteration, in turn 14.5; 384 x 640 between 15.0 and 17.1 from
+// run to run, 14.7; 384 x 768 14.3 and 14.6.
+inline bool small_plan_columns_early(int blocks, int threads) { return threads < 256 || blocks <= 64 || blocks >= 128; }
 
 // Whether the rows of a Gaussian blur of K taps run the kernel that makes 16
 // neighbouring outputs per thread from rolling registers, instead of the one that

@@ -55,6 +55,12 @@ def test_transforms_on_both_sides_of_the_early_start(cuda, h, w, sign):
     _check_fft(h, w, sign)
 
 
+# column blocks of a small plan: 384 x 1024 started early 16.3 us an iteration, in turn 14.5
+@pytest.mark.parametrize("blocks,threads,early", [(96, 256, 0), (64, 256, 1), (128, 256, 1), (96, 128, 1), (192, 512, 1)])
+def test_half_sm_column_blocks_do_not_pair_up(rule, blocks, threads, early):
+    assert rule("small_plan_columns_early(%d, %d)" % (blocks, threads)) == early
+
+
 # (W, H, wide tile of H, narrow): images with many wide tiles keep them
 @pytest.mark.parametrize("w,h,tile,narrow", [(256, 256, 16, 1), (512, 1024, 8, 1), (1168, 512, 16, 1), (1169, 512, 16, 0),
                                              (1024, 1024, 8, 0), (2048, 512, 16, 0), (4096, 128, 16, 0)])
