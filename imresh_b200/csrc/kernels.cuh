@@ -1558,7 +1558,8 @@ __global__ void __launch_bounds__(rcol_threads(M)) k_fft_cols_bs(float2 *data, F
 // because what bounds these passes is how evenly a few hundred to a thousand
 // sequences fill 148 SMs: two rows per 256-thread CTA at two CTAs per SM ran
 // the 733 rows of a 1021 x 733 image as 367 CTAs in 296 places.  All of a tile's
-// operands (X, g_prev, mask, modulus) are requested before its first transform.
+// operands (X, g_prev, mask, modulus) are requested before its first transform, those
+// that arrive in shared memory once the tile is known to run.
 __host__ __device__ constexpr int bs16_rows(int M) { return M >= 2048 ? 1 : 2048 / M; }
 __host__ __device__ constexpr int bs16_row_threads(int M) { return bs16_rows(M) * M / 16; }
 // exchange buffer | g_prev of the rows
@@ -1637,11 +1638,6 @@ k_row_hio_bs16(const JobDev *jobs, const WorkList *L)
         const int j = l + m * Q;
         v[m] = ok && j < W ? Xi[j] : make_float2(0.f, 0.f);
     }
-#pragma unroll
-    for (int m = 0; m < H8; ++m) {   // (g_prev of a first iteration, not yet written, is not used)
-        const int j = l + m * Q;
-        if (ok && j < W) cp_async8(sg + j, Gi + j);
-    }
     uint32_t mk[2] = {0u, 0u};   // mask bytes of m = 0..3, 4..7
     if (!FIRST) {
 #pragma unroll
@@ -1656,9 +1652,11 @@ k_row_hio_bs16(const JobDev *jobs, const WorkList *L)
     const bool init_gprev = k == 0;
     const bool fin = FIX && k >= J.n_cycles;
     const bool track = FIX && (J.target > 0.f || fin);
-    if (stop) {
-        cp_async_wait();   // a block does not end with copies into its shared memory in flight
-        return;
+    if (stop) return;   // (before the copies: a block does not end with one in flight)
+#pragma unroll
+    for (int m = 0; m < H8; ++m) {   // (g_prev of a first iteration, not yet written, is not used)
+        const int j = l + m * Q;
+        if (ok && j < W) cp_async8(sg + j, Gi + j);
     }
     reg16_bluestein<M, RowSwz16<M>, +1>(v, sm, b, l, LdTw16<M>{J.prow.tw, l}, W, J.prow.chirp, J.prow.bspec_b);
     if (FIRST) {
@@ -1793,12 +1791,10 @@ k_row_finish_bs16(const JobDev *jobs, const WorkList *L, float2 *dbg_gprime)
 // column kernels: mode 0 column pass (fwd, modulus, inv), 1 column init
 // (inverse of (M, 0)), 2 plain forward, 3 plain inverse
 template <int M, int MODE>
-__device__ __forceinline__ void col_bs16_load(float2 (&v)[16], const float2 *X, const float *Mod, int W, int H, int x0,
+__device__ __forceinline__ void col_bs16_read(float2 (&v)[16], const float2 *X, const float *Mod, int W, int H, int x0,
                                               int b, int l)
 {
-    extern __shared__ float4 smem4[];
-    constexpr int NB = bs16_col_nb(M), Q = M / 16;
-    float *const smod = reinterpret_cast<float *>(reinterpret_cast<float2 *>(smem4) + NB * M);
+    constexpr int Q = M / 16;
     const int x = x0 + b;
     const bool ok = x < W;
 #pragma unroll
@@ -1807,11 +1803,20 @@ __device__ __forceinline__ void col_bs16_load(float2 (&v)[16], const float2 *X, 
         if (MODE == 1) v[m] = make_float2(ok && j < H ? Mod[(size_t)j * W + x] : 0.f, 0.f);
         else v[m] = ok && j < H ? X[(size_t)j * W + x] : make_float2(0.f, 0.f);
     }
+}
+// request the modulus of mode 0
+template <int M, int MODE>
+__device__ __forceinline__ void col_bs16_load(const float *Mod, int W, int H, int x0, int b, int l)
+{
+    extern __shared__ float4 smem4[];
+    constexpr int NB = bs16_col_nb(M), Q = M / 16;
+    float *const smod = reinterpret_cast<float *>(reinterpret_cast<float2 *>(smem4) + NB * M);
+    const int x = x0 + b;
     if (MODE == 0) {
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
             const int j = l + m * Q;
-            if (ok && j < H) cp_async4(smod + j * NB + b, Mod + (size_t)j * W + x);
+            if (x < W && j < H) cp_async4(smod + j * NB + b, Mod + (size_t)j * W + x);
         }
     }
 }
@@ -1870,12 +1875,10 @@ k_col_bs16(const JobDev *jobs, const WorkList *L)
     float2 v[16];
     const int b = threadIdx.x % NB, l = threadIdx.x / NB;
     pdl_wait();
-    col_bs16_load<M, MODE>(v, X, Mod, W, H, x0, b, l);
+    col_bs16_read<M, MODE>(v, X, Mod, W, H, x0, b, l);
     // (see col_stopped; always by the vote: the two ways apart cost 12 bytes of spills, 1021 x 733 8.46 -> 8.70 ms)
-    if (MODE == 0 && col_stopped(false, st->stop)) {
-        cp_async_wait();   // (see k_row_hio_bs16)
-        return;
-    }
+    if (MODE == 0 && col_stopped(false, st->stop)) return;
+    col_bs16_load<M, MODE>(Mod, W, H, x0, b, l);
     col_bs16_run<M, MODE>(v, X, W, H, x0, chirp, sf, sb, LdTw16<M>{J.pcol.tw, l}, guard, b, l);
 }
 
@@ -1918,7 +1921,7 @@ k_fft_cols_bs16(float2 *data, FftPlanDev p, int W, int cpc)
     const int b = threadIdx.x % NB, l = threadIdx.x / NB;
     pdl_wait();
     float2 v[16];
-    col_bs16_load<M, MODE>(v, data, nullptr, W, p.n, blockIdx.x * cpc, b, l);
+    col_bs16_read<M, MODE>(v, data, nullptr, W, p.n, blockIdx.x * cpc, b, l);
     col_bs16_run<M, MODE>(v, data, W, p.n, blockIdx.x * cpc, p.chirp, p.bspec_f, p.bspec_b, LdTw16<M>{p.tw, l}, true, b,
                           l);
 }
