@@ -633,8 +633,8 @@ __device__ __forceinline__ void b_vblur(const JobDev *jobs, const WorkItem wi)
     }
 }
 // TY: rows of a tile.  32 instead of 128 where that leaves SMs idle: a tile is a
-// chain of loads, a barrier and K taps per output, 12 us at 128 rows however few
-// the tiles.
+// chain of loads, a barrier and K taps per output, the longer the more outputs a
+// thread makes (the plain form, 256 x 256 with 19 taps: 5.3 us at 128 rows, 4.4 at 32).
 template <int TY>
 static __global__ void __launch_bounds__(kVbThreads, 4) k_vblur(const JobDev *jobs, const WorkList *L)
 {
