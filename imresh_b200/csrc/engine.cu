@@ -576,9 +576,10 @@ static int fft_launch(float2 *d, int W, int H, int sign, int axes, const FftPlan
     // the second transform may start while the first one drains (fft_rows_start_early)
     const int every = 1 << 30;
     auto rows_early = [&] {
-        return nrt <= 111 ||   // (asks for nothing where the count decides)
-               fft_rows_start_early(nct, persistent_grid((const void *)cols, ct, (int)sc, every), nrt,
-                                    persistent_grid((const void *)rows, rk.threads, (int)sr, every));
+        if (nrt <= 111 || !rk.p_hio) return true;   // (few, or grouped or chirp-z rows: nothing to ask)
+        const int cols_resident = persistent_grid((const void *)cols, ct, (int)sc, every);
+        return fft_rows_start_early(nct, cols_resident, nrt, persistent_grid((const void *)rows, rk.threads, (int)sr, every),
+                                    is_pow2(W) && is_pow2(H) && cols_resident > kSms);
     };
     const bool dep = axes == 3 && (sign < 0 || rows_early());
     cudaError_t e = cudaSuccess;

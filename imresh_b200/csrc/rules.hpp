@@ -14,10 +14,13 @@ constexpr int kSms = 148;
 // 13.4 -> 15.0).  So rows start early when they are too few to crowd, when two column
 // blocks per SM leave no SM idle, or when they are more than one wave takes.  Row
 // blocks are short and small: columns after them gain at every size measured.
-// `cols_resident`, `rows_resident`: blocks that run at the same time.
-inline bool fft_rows_start_early(int cols, int cols_resident, int rows, int rows_resident)
+// `cols_resident`, `rows_resident`: blocks that run at the same time.  `mixes`: the two
+// kinds of blocks were never seen to crowd -- grouped and chirp-z rows (896 x 512 9.2 ->
+// 8.4 us, 1920 x 256 9.0 -> 8.4), or powers of two both ways with more than one column
+// block to an SM (1024 x 512 8.6 -> 8.2).
+inline bool fft_rows_start_early(int cols, int cols_resident, int rows, int rows_resident, bool mixes = false)
 {
-    return rows <= 111 || cols >= 2 * kSms || rows > rows_resident || (rows <= kSms && cols_resident > kSms);
+    return mixes || rows <= 111 || cols >= 2 * kSms || rows > rows_resident || (rows <= kSms && cols_resident > kSms);
 }
 
 // Whether the columns of a plain transform run in narrow tiles (4 columns) instead

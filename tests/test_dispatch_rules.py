@@ -55,6 +55,12 @@ def test_transforms_on_both_sides_of_the_early_start(cuda, h, w, sign):
     _check_fft(h, w, sign)
 
 
+# grouped rows beside 224 column blocks (896 x 512: 9.2 us, early 8.4); powers of two both ways
+@pytest.mark.parametrize("args,early", [("224, 592, 256, 444, true", 1), ("256, 592, 256, 740, true", 1), ("96, 148, 256, 740, false", 0)])
+def test_rows_that_do_not_crowd_start_early(rule, args, early):
+    assert rule("fft_rows_start_early(%s)" % args) == early
+
+
 # column blocks of a small plan: 384 x 1024 started early 16.3 us an iteration, in turn 14.5
 @pytest.mark.parametrize("blocks,threads,early", [(96, 256, 0), (64, 256, 1), (128, 256, 1), (96, 128, 1), (192, 512, 1)])
 def test_half_sm_column_blocks_do_not_pair_up(rule, blocks, threads, early):
