@@ -566,7 +566,9 @@ int build_weight_table(const imr_params &p, std::vector<float> &w, std::vector<i
 static int fft_launch(float2 *d, int W, int H, int sign, int axes, const FftPlanDev &pr, const FftPlanDev &pc,
                       const RowKernels &rk, const ColKernels &ck, cudaStream_t s)
 {
-    const bool narrow = ck.f_fwd && fft_narrow_columns((W + ck.nb - 1) / ck.nb);
+    const int every = 1 << 30, wide = (W + ck.nb - 1) / ck.nb;
+    const bool narrow = ck.f_fwd && (fft_narrow_columns(wide) ||   // (asks only where the count does not decide)
+                                     fft_narrow_columns(wide, persistent_grid((const void *)ck.fft_fwd, ck.threads, ck.smem, every)));
     const int rpc = rk.mx ? rows_per_tile(rk, W, H) : rk.nb, cpc = narrow ? ck.f_nb : ck.nb;
     const int nrt = (H + rpc - 1) / rpc, nct = (W + cpc - 1) / cpc, ct = narrow ? ck.f_threads : ck.threads;
     const size_t sr = rk.smem ? (size_t)row_tile_smem(rk, W, rpc) : (size_t)rpc * W * 8;
@@ -574,7 +576,6 @@ static int fft_launch(float2 *d, int W, int H, int sign, int axes, const FftPlan
     const auto rows = sign < 0 ? rk.fft_fwd : rk.fft_inv;
     const auto cols = sign < 0 ? (narrow ? ck.f_fwd : ck.fft_fwd) : (narrow ? ck.f_inv : ck.fft_inv);
     // the second transform may start while the first one drains (fft_rows_start_early)
-    const int every = 1 << 30;
     auto rows_early = [&] {
         if (nrt <= 111 || !rk.p_hio) return true;   // (few, or grouped or chirp-z rows: nothing to ask)
         const int cols_resident = persistent_grid((const void *)cols, ct, (int)sc, every);

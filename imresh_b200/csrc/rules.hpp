@@ -28,8 +28,13 @@ inline bool fft_rows_start_early(int cols, int cols_resident, int rows, int rows
 // where the wide tiles leave half of the SMs without one.  Whole transform, wide ->
 // narrow: 256 x 256 6.2 -> 5.2 us (16 wide tiles), 512 x 1024 10.5 -> 8.9 (64); beyond
 // that narrow tiles only make the strides shorter: 2048 x 512 13.0 -> 13.9 (128),
-// 2048 x 1024 23.8 -> 25.0 (256), 4096 x 64 7.7 -> 8.0.
-inline bool fft_narrow_columns(int wide_tiles) { return 2 * wide_tiles < kSms; }
+// 2048 x 1024 23.8 -> 25.0 (256), 4096 x 64 7.7 -> 8.0 -- unless the wide ones
+// (`wide_resident` of them run at the same time) just begin a second wave:
+// 1536 x 1024 (192 on 148) 26.1 -> 24.8, 3072 x 512 26.2 -> 25.0, 1920 x 1024 (240) 25.6 -> 27.2.
+inline bool fft_narrow_columns(int wide_tiles, int wide_resident = 1 << 30)
+{
+    return 2 * wide_tiles < kSms || (wide_tiles > wide_resident && 2 * wide_tiles <= 3 * wide_resident);
+}
 
 // Whether the passes of an iteration are launched dependently (launch_pass):
 // `tiles` work items on at most `resident` CTAs for each of the two passes.

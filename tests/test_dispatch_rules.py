@@ -74,6 +74,19 @@ def test_narrow_columns_where_wide_tiles_leave_sms_idle(rule, w, h, tile, narrow
     assert rule("fft_narrow_columns(%d)" % ((w + tile - 1) // tile)) == narrow
 
 
+# wide tiles, as many at the same time: 1536 x 1024 26.1 us wide, 24.8 narrow; 1920 x 1024 25.6, 27.2
+@pytest.mark.parametrize("tiles,resident,narrow", [(148, 148, 0), (149, 148, 1), (192, 148, 1), (222, 148, 1), (223, 148, 0), (192, 740, 0)])
+def test_narrow_columns_where_wide_tiles_begin_a_second_wave(rule, tiles, resident, narrow):
+    assert rule("fft_narrow_columns(%d, %d)" % (tiles, resident)) == narrow
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,w", [(1024, 1185), (1024, 1778), (512, 3072)])
+@pytest.mark.parametrize("sign", [-1, 1])
+def test_transforms_in_the_second_wave(cuda, h, w, sign):
+    _check_fft(h, w, sign)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("h,w", [(64, 33), (128, 3), (128, 1165), (128, 1169), (512, 1168), (512, 1171), (1024, 583), (1024, 585)])
 @pytest.mark.parametrize("sign", [-1, 1])
