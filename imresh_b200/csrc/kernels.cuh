@@ -737,10 +737,17 @@ static __global__ void __launch_bounds__(kRowThreads) k_hblur(const float *src, 
 #pragma unroll 4
             for (int r = threadIdx.x >> lgx; r < rows; r += T >> lgx)
                 if (x < pw) f(r, x * PC);
-        } else {
+        } else if (VEC || rows == 1) {
             for (int r = 0; r < rows; ++r)
 #pragma unroll 4
                 for (int e = e0 + threadIdx.x * PC; e < e1; e += T * PC) f(r, e);
+        } else {   // (two rows at a time: more loads in flight)
+            for (int r = 0; r < rows; r += 2)
+#pragma unroll 2
+                for (int e = threadIdx.x; e < W; e += T) {
+                    f(r, e);
+                    if (r + 1 < rows) f(r + 1, e);
+                }
         }
     };
     pieces(0, W, [&](int r, int e) {

@@ -72,8 +72,8 @@ inline bool small_plan_columns_early(int blocks, int threads) { return threads <
 inline bool hblur_rolling(int W, int H, int K, bool vec)
 {
     const double turns = (W + 255) / 256, mpx = 1e-6 * W * H;
-    return 0.16 * turns + 0.006 * turns * K + 0.56e-3 * H + (0.1 * K - 0.41) * mpx >
-           0.94 + 0.015 * K + (vec ? 0.0 : 1.0 + 0.8 * mpx);
+    return 0.14 * turns + 0.007 * turns * K + 0.54e-3 * H + (0.126 * K - 0.5) * mpx >
+           1.05 + 0.02 * K + (vec ? 0.0 : 1.0 + 0.4 * mpx);
 }
 
 // Whether grouped-pass columns of n > 1024 values run in tiles of two columns instead

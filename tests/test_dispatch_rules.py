@@ -105,7 +105,8 @@ def test_long_pipelined_rows_do_not_start_early(rule, w, dependent):
     (64, 64, 19, 1, 0),          # 4.2, 2.2
     (256, 256, 19, 1, 0),        # 4.5, 2.5
     (16, 1024, 59, 1, 0),        # 5.9, 3.2
-    (331, 2649, 5, 0, 0),        # 10.4, 6.8
+    (331, 2649, 5, 0, 0),        # 7.8, 6.8
+    (1021, 733, 19, 0, 1),       # 6.0, 8.1
     (64, 16384, 3, 1, 1),        # 7.6, 16.6
     (1000, 800, 19, 1, 1),       # 5.6, 9.0
     (2048, 1536, 19, 1, 1),      # 14, 26
@@ -115,8 +116,8 @@ def test_rolling_row_blur_where_its_long_code_pays(rule, w, h, taps, vec, rollin
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("h,w", [(16384, 64), (5003, 61), (4000, 30), (600, 256), (297, 1000), (593, 331), (7, 4100), (2, 9002),
-                                 (2, 53952), (2, 53956), (1, 58048)])
+@pytest.mark.parametrize("h,w", [(16384, 64), (5003, 61), (4000, 30), (600, 256), (297, 1000), (593, 331), (3479, 463),
+                                 (2003, 1023), (7, 4100), (2, 9002), (2, 53952), (2, 53956), (1, 58048)])
 @pytest.mark.parametrize("sigma", [0.4, 3.0])
 def test_rows_of_a_blur_bitexact(cuda, h, w, sigma):
     """Many narrow rows per block, rows with and without a stage for their sums."""
